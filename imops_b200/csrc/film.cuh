@@ -29,14 +29,15 @@ struct ExposeSpec {
     float hal_threshold;
 };
 
-// Spectral scan: d(l) = sum_e Dimg_e*eps_e(l) + Dmask_e*meps_e(l);
+// Spectral scan: d(l) = sum_e Dimg_e*eps_e(l) + meps(l) sum_e Dmask_e (the
+// mask curve is the stock's, the same for each of its masked layers);
 // T = 2^(-d) * illum(l) (eps pre-scaled by log2(10));
 // rgb_c = sum_l C[l][c] * T(l)  (C folds trapezoid weights, CMFs, XYZ->AP1 and
 // the 1/peak(Dmin) normalisation; densitometry.rs:13-73).
 struct ScanSpec16 {
     int E;
     float eps[MAXE][NB16];
-    float meps[MAXE][NB16];
+    float meps[NB16];
     float C[NB16][3];
 };
 

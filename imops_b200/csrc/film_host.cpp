@@ -463,7 +463,7 @@ int build_reference(const StockDef& sd, int W, float shutter, Stock* st, float* 
         const Layer& L = sd.layers[em[e]];
         for (int i = 0; i < NB16; i++) {
             C.eps[e][i] = (float)(L.eps[i] * LOG2_10);
-            C.meps[e][i] = L.mask_eps.empty() ? 0.0f : (float)(L.mask_eps[i] * LOG2_10);
+            if (!L.mask_eps.empty()) C.meps[i] = (float)(L.mask_eps[i] * LOG2_10);  // the same for every layer
         }
     }
     double dmin[3];
