@@ -15,6 +15,7 @@
 #include <cstring>
 #include <mutex>
 #include <type_traits>
+#include <utility>
 #include <vector>
 
 #include "film.cuh"
@@ -407,6 +408,14 @@ int blur(const float* in, float* tmp, int W, int H, const Taps& tp, Epi epi, cud
     IMOPS_CUDA_TRY(cudaGetLastError(), "film blur launch");
     return IMOPS_OK;
 }
+
+}  // namespace film
+}  // namespace imops
+
+#include "film_tiles.cuh"
+
+namespace imops {
+namespace film {
 
 // ---------------------------------------------------------------------------
 // capture LUT + reduce (capture.rs:61-88, reduction.rs:16-68)
@@ -1487,12 +1496,29 @@ int stage_halation(float* planes, int W, int H, const Stock& st, float* tmp, flo
     return IMOPS_OK;
 }
 
+int launch_dir(const float* in, float* out, int W, int H, const Taps& tp, const RefSpec& R, cudaStream_t s) {
+    return with_layers(R.E, [&](auto e) {
+        constexpr int E = decltype(e)::value;
+        DirMix<E> mix;
+        for (int i = 0; i < E; i++)
+            for (int j = 0; j < E; j++) mix.m[i][j] = R.dir[i][j];
+        const size_t smem = (size_t)(2 * ft_tile_floats(tp.R) + ft_row_floats(tp.R)) * sizeof(float);
+        IMOPS_CUDA_TRY(cudaFuncSetAttribute(dir_kernel<E>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+                       "cudaFuncSetAttribute(DIR)");
+        const dim3 g((W + FT_W - 1) / FT_W, (H + FT_H - 1) / FT_H);
+        dir_kernel<E><<<g, FT_THREADS, smem, s>>>(in, out, W, H, tp, mix);
+        note_launch();
+        return IMOPS_OK;
+    });
+}
+
 //   develop: capture LUT + reciprocity + reduction to image-dye and mask
 //     densities, DIR inhibition, adjacency (capture.rs:61-88,
-//     reduction.rs:16-68, diffusion.rs:11-84); inh: E planes, tmp: one
-//     sum: `mask` is the one plane of the layers' mask sum
+//     reduction.rs:16-68, diffusion.rs:11-84); inh: E planes, tmp: one.
+//     sum: `mask` is the one plane of the layers' mask sum.  The densities
+//     end up in *result (planes or inh), or in planes when result is NULL.
 int stage_develop(float* planes, float* mask, bool sum, int W, int H, const Stock& st, const RefSpec* dR, float* inh,
-                  float* tmp, cudaStream_t s) {
+                  float* tmp, float** result, cudaStream_t s) {
     const RefSpec& R = st.ref;
     const int E = R.E;
     const size_t n = (size_t)W * H;
@@ -1502,12 +1528,27 @@ int stage_develop(float* planes, float* mask, bool sum, int W, int H, const Stoc
     if (sum) lut_reduce_kernel<true><<<g, 256, 0, s>>>(planes, mask, n, E, dR);
     else lut_reduce_kernel<false><<<g, 256, 0, s>>>(planes, mask, n, E, dR);
     note_launch();
+    if (result) *result = planes;
     if (R.dir_any && R.sigma_dir >= 1e-3f) {
         if ((rc = taps_for(R.sigma_dir, &tp))) return rc;
-        for (int i = 0; i < E; i++)
-            if ((rc = blur(planes + i * n, tmp, W, H, tp, EpiStore{inh + i * n}, s))) return rc;
-        dir_apply_kernel<<<g, 256, 0, s>>>(planes, inh, n, E, dR);
-        note_launch();
+        if (tp.R <= FT_MAXR) {
+            float *in = planes, *out = inh;
+            if (result) {
+                *result = inh;
+            } else {
+                std::swap(in, out);
+                IMOPS_CUDA_TRY(cudaMemcpyAsync(in, out, E * n * 4, cudaMemcpyDeviceToDevice, s), "copy");
+            }
+            if ((rc = launch_dir(in, out, W, H, tp, R, s))) return rc;
+            planes = out;
+        } else {
+            // a blur wider than the tiles' halo: 35 mm images above 12000 pixels, which only the
+            // sub-stage takes (their wide bounce is above 64 px)
+            for (int i = 0; i < E; i++)
+                if ((rc = blur(planes + i * n, tmp, W, H, tp, EpiStore{inh + i * n}, s))) return rc;
+            dir_apply_kernel<<<g, 256, 0, s>>>(planes, inh, n, E, dR);
+            note_launch();
+        }
     }
     if (!(fabsf(R.beta) < 1e-8f || R.sigma_adj < 1e-3f)) {
         if ((rc = taps_for(R.sigma_adj, &tp))) return rc;
@@ -1566,11 +1607,12 @@ int run_reference(float* rgb, int W, int H, const Stock& st, uint64_t seed, int 
     int rc;
     if ((rc = stage_expose(rgb, W, H, st, planes, s))) return rc;
     if ((rc = stage_halation(planes, W, H, st, tmp, noise, s))) return rc;
-    if ((rc = stage_develop(planes, mask, true, W, H, st, dR, inh, tmp, s))) return rc;
-    // the inhibition planes are free after develop: they hold the grain's block sums
-    if (grain && (rc = stage_grain(planes, W, H, st, seed, noise, reinterpret_cast<double*>(inh), sums, s)))
-        return rc;
-    if ((rc = stage_scan(planes, mask, true, W, H, st.scan16, rgb, s))) return rc;
+    float* dens = nullptr;
+    if ((rc = stage_develop(planes, mask, true, W, H, st, dR, inh, tmp, &dens, s))) return rc;
+    // the other set of planes is free after develop: it holds the grain's block sums
+    float* spare = dens == planes ? inh : planes;
+    if (grain && (rc = stage_grain(dens, W, H, st, seed, noise, reinterpret_cast<double*>(spare), sums, s))) return rc;
+    if ((rc = stage_scan(dens, mask, true, W, H, st.scan16, rgb, s))) return rc;
     IMOPS_CUDA_TRY(cudaGetLastError(), "film kernels");
     return IMOPS_OK;
 }
@@ -1829,7 +1871,7 @@ extern "C" int imops_film_develop(float* planes, float* mask, int w, int h, cons
     if (!planes || !mask) return fail(IMOPS_ERR_INVALID_ARGUMENT, "film_develop: NULL buffer");
     float* inh = c.A.take<float>((size_t)c.st.ref.E * n);
     float* tmp = c.A.take<float>(n);
-    if ((rc = film::stage_develop(planes, mask, false, w, h, c.st, c.dR, inh, tmp, s))) return rc;
+    if ((rc = film::stage_develop(planes, mask, false, w, h, c.st, c.dR, inh, tmp, nullptr, s))) return rc;
     IMOPS_CUDA_TRY(cudaGetLastError(), "film_develop");
     return IMOPS_OK;
 }

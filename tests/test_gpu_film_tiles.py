@@ -42,3 +42,21 @@ def test_sub_stages_equal_the_whole_on_ragged_frames(gpu, stock, H, W):
     ref = im.film_process(x.clone(), stock=stock, seed=5, output=1, grain=True)
     got = im.FilmStages(stock=stock, seed=5, output=1, grain=True).run(x.clone())
     assert torch.equal(got, ref)
+
+
+@pytest.mark.parametrize("stock", [1, 2])
+def test_develop_agrees_across_the_tile_radius_line(gpu, stock):
+    """Flat planes develop to the same densities on both sides of the width
+    above which the DIR blur no longer fits the tiles' halo (a flat plane's
+    blur is the plane; f32 rounding of 33 taps and the exponential, 1e-5)."""
+    import torch
+
+    import imops_b200 as im
+    st = im.FilmStages(stock=stock, grain=False)
+    res = []
+    for w in (11000, 13500):
+        planes = torch.full((st.layers, 3, w), 0.37, device=gpu) * torch.arange(1, st.layers + 1, device=gpu)[:, None, None]
+        dens, mask = st.develop(planes)
+        assert float((dens - dens[:, :1, :1]).abs().max()) < 1e-5
+        res.append(torch.cat([dens[:, 0, 0], mask[:, 0, 0]]))
+    assert float((res[0] - res[1]).abs().max()) < 1e-5
