@@ -100,43 +100,94 @@ __global__ void expose_kernel(const float* __restrict__ rgb, size_t n, ExposeSpe
 // ---------------------------------------------------------------------------
 // separable Gaussian blur with mirror reflection (blur.rs:10-89)
 
-constexpr int ROW_TILE = 256;
+// One kernel pair for any radius up to 64 (the reference model's wide bounce,
+// the adjoint with another radius than 64).  A thread slides a window over
+// several outputs (4 along a row, 16 down a column), so a staged sample is
+// read once for all of them instead of once per tap and output; the head and
+// tail of the window test the tap range, the middle does not.  Each output
+// sums its taps in ascending order.
+constexpr int ROW_OUT = 4, ROW_THREADS = 256, ROW_TILE = ROW_OUT * ROW_THREADS;
 
-__global__ void blur_rows_kernel(const float* __restrict__ in, float* __restrict__ out, int W, int H, Taps tp) {
-    __shared__ float s[ROW_TILE + 2 * MAXR];
-    int y = blockIdx.y;
-    int x0 = blockIdx.x * ROW_TILE;
+__global__ void __launch_bounds__(ROW_THREADS) blur_rows_kernel(const float* __restrict__ in, float* __restrict__ out,
+                                                                int W, int H, const __grid_constant__ Taps tp) {
+    __shared__ __align__(16) float s[ROW_TILE + 2 * MAXR + ROW_OUT];
+    const int y = blockIdx.y, x0 = blockIdx.x * ROW_TILE, R2 = 2 * tp.R;
     const float* row = in + (size_t)y * W;
-    int span = ROW_TILE + 2 * tp.R;
-    for (int j = threadIdx.x; j < span; j += blockDim.x) s[j] = __ldg(row + reflect(x0 - tp.R + j, W));
+    // only the samples that outputs inside the image read
+    const int span = min(ROW_TILE, W - x0) + R2;
+    for (int j = threadIdx.x; j < span; j += ROW_THREADS) s[j] = __ldg(row + reflect(x0 - tp.R + j, W));
     __syncthreads();
-    int x = x0 + threadIdx.x;
-    if (x >= W) return;
-    float acc = 0.0f;
-    for (int k = 0; k <= 2 * tp.R; k++) acc = fmaf(s[threadIdx.x + k], tp.t[k], acc);
-    out[(size_t)y * W + x] = acc;
+    const int xb = ROW_OUT * threadIdx.x;
+    if (x0 + xb >= W) return;
+    float a[ROW_OUT] = {0.0f, 0.0f, 0.0f, 0.0f};
+    // samples 4q .. 4q+3 of the window: sample 4q+u is tap 4q+u-j of output j
+    auto step = [&](int q, bool lo, bool hi) {
+        const float4 v4 = *reinterpret_cast<const float4*>(s + xb + 4 * q);
+        const float v[4] = {v4.x, v4.y, v4.z, v4.w};
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+#pragma unroll
+            for (int j = 0; j < ROW_OUT; j++) {
+                const int k = 4 * q + u - j;
+                if ((!lo || k >= 0) && (!hi || k <= R2)) a[j] = fmaf(v[u], tp.t[k], a[j]);
+            }
+    };
+    step(0, true, true);
+    int q = 1;
+#pragma unroll 2
+    for (; 4 * q + 3 <= R2; q++) step(q, false, false);
+    for (; 4 * q - 3 <= R2; q++) step(q, false, true);
+    float* o = out + (size_t)y * W + x0 + xb;
+#pragma unroll
+    for (int j = 0; j < ROW_OUT; j++)
+        if (x0 + xb + j < W) o[j] = a[j];
 }
 
-constexpr int COL_TW = 32, COL_TH = 64, COL_RPT = 8;  // 32x8 threads, 8 rows each
+constexpr int COL_TW = 32, COL_GROUPS = 8, COL_OUT = 16, COL_TH = COL_GROUPS * COL_OUT;  // 32x8 threads, 16 rows each
 
 // Column pass; epi(index, blurred) writes the result.
 template <class Epi>
-__global__ void blur_cols_kernel(const float* __restrict__ in, int W, int H, Taps tp, Epi epi) {
+__global__ void __launch_bounds__(COL_TW * COL_GROUPS) blur_cols_kernel(const float* __restrict__ in, int W, int H,
+                                                                        const __grid_constant__ Taps tp, Epi epi) {
     __shared__ float s[(COL_TH + 2 * MAXR) * COL_TW];
-    int x0 = blockIdx.x * COL_TW, y0 = blockIdx.y * COL_TH;
-    int tx = threadIdx.x, ty = threadIdx.y;
-    int x = x0 + tx;
-    int span = COL_TH + 2 * tp.R;
-    if (x < W)
-        for (int j = ty; j < span; j += blockDim.y) s[j * COL_TW + tx] = __ldg(in + (size_t)reflect(y0 - tp.R + j, H) * W + x);
+    const int tx = threadIdx.x, ty = threadIdx.y, x = blockIdx.x * COL_TW + tx, y0 = blockIdx.y * COL_TH;
+    const int R2 = 2 * tp.R, rb = ty * COL_OUT;
+    if (x < W) {
+        const int span = min(COL_TH, H - y0) + R2;
+        if (y0 - tp.R >= 0 && y0 - tp.R + span <= H) {
+            const float* src = in + (size_t)(y0 - tp.R) * W + x;
+#pragma unroll 8
+            for (int j = ty; j < span; j += COL_GROUPS) s[j * COL_TW + tx] = __ldg(src + (size_t)j * W);
+        } else {
+            for (int j = ty; j < span; j += COL_GROUPS)
+                s[j * COL_TW + tx] = __ldg(in + (size_t)reflect(y0 - tp.R + j, H) * W + x);
+        }
+    }
     __syncthreads();
-    if (x >= W) return;
-    for (int r = 0; r < COL_RPT; r++) {
-        int ly = ty * COL_RPT + r, y = y0 + ly;
-        if (y >= H) break;
-        float acc = 0.0f;
-        for (int k = 0; k <= 2 * tp.R; k++) acc = fmaf(s[(ly + k) * COL_TW + tx], tp.t[k], acc);
-        epi((size_t)y * W + x, acc);
+    if (x >= W || y0 + rb >= H) return;
+    float a[COL_OUT];
+#pragma unroll
+    for (int j = 0; j < COL_OUT; j++) a[j] = 0.0f;
+    // rows m0 .. m0+15 of the window: row m is tap m-j of output j
+    auto step = [&](int m0, bool lo, bool hi) {
+#pragma unroll
+        for (int u = 0; u < COL_OUT; u++) {
+            const int m = m0 + u;
+            if (hi && m > R2 + COL_OUT - 1) break;
+            const float v = s[(rb + m) * COL_TW + tx];
+#pragma unroll
+            for (int j = 0; j < COL_OUT; j++)
+                if ((!lo || u - j >= 0) && (!hi || m - j <= R2)) a[j] = fmaf(v, tp.t[m - j], a[j]);
+        }
+    };
+    step(0, true, true);
+    int m0 = COL_OUT;
+    for (; m0 + COL_OUT - 1 <= R2; m0 += COL_OUT) step(m0, false, false);
+    for (; m0 <= R2 + COL_OUT - 1; m0 += COL_OUT) step(m0, false, true);
+#pragma unroll
+    for (int j = 0; j < COL_OUT; j++) {
+        const int y = y0 + rb + j;
+        if (y < H) epi((size_t)y * W + x, a[j]);
     }
 }
 
@@ -311,17 +362,6 @@ struct EpiMix {
     float keep, mix;
     __device__ __forceinline__ void operator()(size_t i, float v) const { plane[i] = keep * plane[i] + mix * v; }
 };
-// support bounce: plane_e += gain_e * blur(deep) (halation.rs:80-92)
-struct EpiBounce {
-    float* planes;
-    size_t n;
-    int E;
-    float gain[MAXE];
-    __device__ __forceinline__ void operator()(size_t i, float v) const {
-        for (int e = 0; e < E; e++)
-            if (gain[e] > 0.0f) planes[e * n + i] += gain[e] * v;
-    }
-};
 // adjacency: d += beta * (d - blur(d)) (diffusion.rs:11-28)
 struct EpiAdjacency {
     float* plane;
@@ -347,7 +387,7 @@ int blur_rows(const float* in, float* out, int W, int H, const float* taps, int 
         blur_rows_r64_kernel<<<rg, R64_ROW_THREADS, 0, s>>>(PlaneSource{in}, out, W, H, pair_taps(tp));
     } else {
         dim3 rg((W + ROW_TILE - 1) / ROW_TILE, H);
-        blur_rows_kernel<<<rg, ROW_TILE, 0, s>>>(in, out, W, H, tp);
+        blur_rows_kernel<<<rg, ROW_THREADS, 0, s>>>(in, out, W, H, tp);
     }
     note_launch();
     IMOPS_CUDA_TRY(cudaGetLastError(), "blur rows");
@@ -381,7 +421,7 @@ int blur_cols(const float* in, float* out, int W, int H, const float* taps, int 
         if (add) blur_cols_r64_stream_kernel<<<cg, cb, 0, s>>>(in, W, H, t2, EpiAdd{out});
         else blur_cols_r64_stream_kernel<<<cg, cb, 0, s>>>(in, W, H, t2, EpiStore{out});
     } else {
-        dim3 cb(COL_TW, COL_TH / COL_RPT), cg((W + COL_TW - 1) / COL_TW, (H + COL_TH - 1) / COL_TH);
+        dim3 cb(COL_TW, COL_GROUPS), cg((W + COL_TW - 1) / COL_TW, (H + COL_TH - 1) / COL_TH);
         if (add) blur_cols_kernel<<<cg, cb, 0, s>>>(in, W, H, tp, EpiAdd{out});
         else blur_cols_kernel<<<cg, cb, 0, s>>>(in, W, H, tp, EpiStore{out});
     }
@@ -400,9 +440,9 @@ int taps_for(float sigma, Taps* tp) {
 template <class Epi>
 int blur(const float* in, float* tmp, int W, int H, const Taps& tp, Epi epi, cudaStream_t s) {
     dim3 rg((W + ROW_TILE - 1) / ROW_TILE, H);
-    blur_rows_kernel<<<rg, ROW_TILE, 0, s>>>(in, tmp, W, H, tp);
+    blur_rows_kernel<<<rg, ROW_THREADS, 0, s>>>(in, tmp, W, H, tp);
     note_launch();
-    dim3 cb(COL_TW, COL_TH / COL_RPT), cg((W + COL_TW - 1) / COL_TW, (H + COL_TH - 1) / COL_TH);
+    dim3 cb(COL_TW, COL_GROUPS), cg((W + COL_TW - 1) / COL_TW, (H + COL_TH - 1) / COL_TH);
     blur_cols_kernel<<<cg, cb, 0, s>>>(tmp, W, H, tp, epi);
     note_launch();
     IMOPS_CUDA_TRY(cudaGetLastError(), "film blur launch");
@@ -418,45 +458,110 @@ namespace imops {
 namespace film {
 
 // ---------------------------------------------------------------------------
-// capture LUT + reduce (capture.rs:61-88, reduction.rs:16-68)
+// support bounce, capture LUT, reduce (halation.rs:80-92, capture.rs:61-88,
+// reduction.rs:16-68)
 
-__device__ __forceinline__ float lut_sample(const float* logs, const float* fr, float phi) {
-    if (!(phi > 0.0f)) return fr[0];
-    float lp = log10f(phi);
-    if (lp <= logs[0]) return fr[0];
-    if (lp >= logs[LUTN - 1]) return fr[LUTN - 1];
-    int lo = 0, hi = LUTN - 1;
-    while (hi - lo > 1) {
-        int mid = (lo + hi) >> 1;
-        if (logs[mid] <= lp) lo = mid; else hi = mid;
+// support bounce: plane_e += gain_e * blur(deep)
+struct Bounce {
+    float gain[MAXE];
+};
+__device__ __forceinline__ float bounce_px(float p, float gain, float v) { return gain > 0.0f ? fmaf(gain, v, p) : p; }
+
+__global__ void bounce_kernel(float* __restrict__ planes, const float* __restrict__ deep, size_t n, int E,
+                              const __grid_constant__ Bounce bn) {
+    for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < n; p += (size_t)gridDim.x * blockDim.x) {
+        const float v = deep[p];
+        for (int e = 0; e < E; e++)
+            if (bn.gain[e] > 0.0f) planes[e * n + p] = bounce_px(planes[e * n + p], bn.gain[e], v);
     }
-    float t = (lp - logs[lo]) / (logs[hi] - logs[lo]);
-    return fr[lo] * (1.0f - t) + fr[hi] * t;
 }
 
-// SUM: `mask` is one plane, the sum of the layers' mask densities (layer
-// order); otherwise E planes.
-template <bool SUM>
-__global__ void lut_reduce_kernel(float* __restrict__ planes, float* __restrict__ mask, size_t n, int E,
-                                  const RefSpec* __restrict__ R) {
-    __shared__ float logs[MAXE][LUTN], fr[MAXE][LUTN];
+// Layer constants of the capture LUT and the reduction.
+template <int E>
+struct Reduce {
+    float eta[E], dmax[E], inv_gamma[E], mask_scale[E];  // mask_scale 0: no mask
+    int reversal[E];
+};
+
+// Developable fraction of a layer's fluence phi: linear interpolation in
+// log10 phi over LUTN entries at -4 .. 8 in equal steps, so the cell is found
+// by arithmetic (a search over the knots before).  With phi = 2^k m, m in
+// [1, 2), the place in cells is SCALE k + SCALE log2 m + ZERO; the first
+// term is exact but for the low part of SCALE (k times its upper 12 bits),
+// so the offset in the cell is good to about 4e-7 (the hardware logarithm of
+// m), where a logarithm of phi itself, up to 27, rounds at 1e-6.
+// lut[i] = (entry i, entry i+1 - entry i).
+__device__ __forceinline__ float lut_sample(const float2* lut, float phi) {
+    constexpr double SCALE = (LUTN - 1) / 12.0 * 0.30102999566398119521;  // cells an octave
+    constexpr float HI = (float)((int)(SCALE * 2048.0)) / 2048.0f, LO = (float)(SCALE - (double)HI);
+    constexpr float ZERO = (float)((LUTN - 1) / 3);  // cell of phi = 1
+    static_assert((LUTN - 1) % 3 == 0, "phi = 1 is a knot");
+    if (!(phi > 1.0e-5f)) return lut[0].x;  // below the first knot at 1e-4 (and NaN)
+    if (phi > 1.0e9f) return lut[LUTN - 1].x;
+    const uint32_t b = __float_as_uint(phi);
+    const float k = (float)((int)(b >> 23) - 127);
+    float lm;
+    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(lm) : "f"(__uint_as_float((b & 0x007FFFFFu) | 0x3F800000u)));
+    const float frac = fmaf(lm, (float)SCALE, k * LO);
+    const float pos = fminf(fmaxf(fmaf(k, HI, ZERO) + frac, 0.0f), (float)(LUTN - 1));
+    const int i = min((int)pos, LUTN - 2);
+    const float t = fminf(fmaxf(fmaf(k, HI, ZERO - (float)i) + frac, 0.0f), 1.0f);
+    const float2 c = lut[i];
+    return fmaf(t, c.y, c.x);
+}
+
+// f^g for f in [0, 1], g > 0, to about an ulp: the product g log2 f is split
+// into its nearest integer and a remainder rounded once, and 2^remainder is a
+// polynomial of degree 6 fitted here for least relative error on
+// [-1/2, 1/2] (2e-9).  (The hardware exponential's 2 ulp near f = 1, where a
+// positive print's highlights lie, were the largest error of the reduction.)
+__device__ __forceinline__ float pow_unit(float f, float g) {
+    const float l = log2f(f);
+    const float n = rintf(g * l);
+    if (!(n > -126.0f)) return f != f ? f : 0.0f;
+    const float r = fmaf(g, l, -n);
+    float q = 0.0001535336923552677f;
+    q = fmaf(q, r, 0.0013398876180872321f);
+    q = fmaf(q, r, 0.00961843691766262f);
+    q = fmaf(q, r, 0.055503323674201965f);
+    q = fmaf(q, r, 0.24022647738456726f);
+    q = fmaf(q, r, 0.6931471824645996f);
+    q = fmaf(q, r, 1.0f);
+    return __uint_as_float(__float_as_uint(q) + ((uint32_t)(int)n << 23));
+}
+
+// Image-dye densities over the fluences in place, and the mask densities
+// (SUM: `mask` is one plane, their sum in layer order; otherwise E planes);
+// BOUNCE: the support bounce `deep` is added to the fluences first.  Bound by
+// the issue of the interpolation and the power of each layer and pixel.  24 MP, six layers, with the bounce: 0.44 ms against 1.86
+// (reduction and bounce epilogue apart, a binary search and powf a value).
+template <int E, bool SUM, bool BOUNCE>
+__global__ void __launch_bounds__(256) lut_reduce_kernel(float* __restrict__ planes, float* __restrict__ mask,
+                                                         const float* __restrict__ deep, size_t n,
+                                                         const RefSpec* __restrict__ R,
+                                                         const __grid_constant__ Reduce<E> c,
+                                                         const __grid_constant__ Bounce bn) {
+    __shared__ float2 lut[E][LUTN];
     for (int k = threadIdx.x; k < E * LUTN; k += blockDim.x) {
-        logs[k / LUTN][k % LUTN] = R->lut_log[k / LUTN][k % LUTN];
-        fr[k / LUTN][k % LUTN] = R->lut_frac[k / LUTN][k % LUTN];
+        const int e = k / LUTN, i = k % LUTN;
+        const float a = R->lut_frac[e][i], b = i + 1 < LUTN ? R->lut_frac[e][i + 1] : a;
+        lut[e][i] = make_float2(a, b - a);
     }
     __syncthreads();
     for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < n; p += (size_t)gridDim.x * blockDim.x) {
-        float M = 0.0f;
+        float x[E], v = 0.0f, M = 0.0f;
+#pragma unroll
+        for (int e = 0; e < E; e++) x[e] = planes[e * n + p];
+        if (BOUNCE) v = __ldg(deep + p);
+#pragma unroll
         for (int e = 0; e < E; e++) {
-            float phi = planes[e * n + p] * R->eta[e];
-            float f = lut_sample(logs[e], fr[e], phi);
+            if (BOUNCE) x[e] = bounce_px(x[e], bn.gain[e], v);
+            float f = lut_sample(lut[e], __fmul_rn(x[e], c.eta[e]));
             f = fminf(fmaxf(f, 0.0f), 1.0f);
-            float ef = R->reversal[e] ? 1.0f - f : f;
-            float dmax = R->dmax[e];
-            float d = dmax * powf(ef, R->inv_gamma[e]);
-            planes[e * n + p] = d;
-            const float m =
-                R->has_mask[e] ? R->mask_scale[e] * (1.0f - fminf(fmaxf(d / dmax, 0.0f), 1.0f)) : 0.0f;
+            if (c.reversal[e]) f = 1.0f - f;
+            const float q = pow_unit(f, c.inv_gamma[e]);
+            planes[e * n + p] = __fmul_rn(c.dmax[e], q);
+            const float m = __fmul_rn(c.mask_scale[e], 1.0f - fminf(q, 1.0f));
             if (SUM) M = __fadd_rn(M, m);
             else mask[e * n + p] = m;
         }
@@ -1468,14 +1573,18 @@ int stage_expose(const float* rgb, int W, int H, const Stock& st, float* planes,
     return IMOPS_OK;
 }
 
-//   halation: local scatter and the wide bounce of the deepest layer
-//     (halation.rs:24-93); tmp, bounce: one plane each
-int stage_halation(float* planes, int W, int H, const Stock& st, float* tmp, float* bounce, cudaStream_t s) {
+//   halation: local scatter in place, and the wide bounce of the deepest
+//     layer (halation.rs:24-93): its blur in *deep (NULL when the stock has
+//     none), added to the layers by bounce_kernel or by the reduction; tmp,
+//     bounce: one plane each
+int stage_halation(float* planes, int W, int H, const Stock& st, float* tmp, float* bounce, float** deep,
+                   cudaStream_t s) {
     const RefSpec& R = st.ref;
     const int E = R.E;
     const size_t n = (size_t)W * H;
     Taps tp;
     int rc;
+    *deep = nullptr;
     if (R.sigma_local >= 1e-3f && R.local_mix > 0.0f) {
         if ((rc = taps_for(R.sigma_local, &tp))) return rc;
         for (int e = 0; e < E; e++)
@@ -1484,16 +1593,39 @@ int stage_halation(float* planes, int W, int H, const Stock& st, float* tmp, flo
     }
     if (R.sigma_wide >= 1e-3f) {
         if ((rc = taps_for(R.sigma_wide, &tp))) return rc;
-        EpiBounce eb;
-        eb.planes = planes;
-        eb.n = n;
-        eb.E = E;
-        for (int e = 0; e < MAXE; e++) eb.gain[e] = R.hal_gain[e];
-        // the bounce source is the deepest plane before the bounce is added
-        IMOPS_CUDA_TRY(cudaMemcpyAsync(bounce, planes + (E - 1) * n, n * 4, cudaMemcpyDeviceToDevice, s), "copy");
-        if ((rc = blur(bounce, tmp, W, H, tp, eb, s))) return rc;
+        if ((rc = blur(planes + (E - 1) * n, tmp, W, H, tp, EpiStore{bounce}, s))) return rc;
+        *deep = bounce;
     }
     return IMOPS_OK;
+}
+
+static Bounce bounce_gains(const RefSpec& R) {
+    Bounce b;
+    for (int e = 0; e < MAXE; e++) b.gain[e] = R.hal_gain[e];
+    return b;
+}
+
+// The bounce (deep not NULL), the capture LUT and the reduction over the layers.
+int launch_reduce(float* planes, float* mask, bool sum, const float* deep, size_t n, const RefSpec& R,
+                  const RefSpec* dR, cudaStream_t s) {
+    return with_layers(R.E, [&](auto e) {
+        constexpr int E = decltype(e)::value;
+        Reduce<E> c;
+        for (int i = 0; i < E; i++) {
+            c.eta[i] = R.eta[i];
+            c.dmax[i] = R.dmax[i];
+            c.inv_gamma[i] = R.inv_gamma[i];
+            c.mask_scale[i] = R.has_mask[i] ? R.mask_scale[i] : 0.0f;
+            c.reversal[i] = R.reversal[i];
+        }
+        const Bounce b = bounce_gains(R);
+        const int g = grid_for(n);
+        if (sum && deep) lut_reduce_kernel<E, true, true><<<g, 256, 0, s>>>(planes, mask, deep, n, dR, c, b);
+        else if (sum) lut_reduce_kernel<E, true, false><<<g, 256, 0, s>>>(planes, mask, nullptr, n, dR, c, b);
+        else lut_reduce_kernel<E, false, false><<<g, 256, 0, s>>>(planes, mask, nullptr, n, dR, c, b);
+        note_launch();
+        return IMOPS_OK;
+    });
 }
 
 int launch_dir(const float* in, float* out, int W, int H, const Taps& tp, const RefSpec& R, cudaStream_t s) {
@@ -1515,9 +1647,10 @@ int launch_dir(const float* in, float* out, int W, int H, const Taps& tp, const 
 //   develop: capture LUT + reciprocity + reduction to image-dye and mask
 //     densities, DIR inhibition, adjacency (capture.rs:61-88,
 //     reduction.rs:16-68, diffusion.rs:11-84); inh: E planes, tmp: one.
-//     sum: `mask` is the one plane of the layers' mask sum.  The densities
-//     end up in *result (planes or inh), or in planes when result is NULL.
-int stage_develop(float* planes, float* mask, bool sum, int W, int H, const Stock& st, const RefSpec* dR, float* inh,
+//     sum: `mask` is the one plane of the layers' mask sum, and the bounce
+//     `deep` (or NULL) is added first.  The densities end up in *result
+//     (planes or inh), or in planes when result is NULL.
+int stage_develop(float* planes, float* mask, bool sum, const float* deep, int W, int H, const Stock& st, const RefSpec* dR, float* inh,
                   float* tmp, float** result, cudaStream_t s) {
     const RefSpec& R = st.ref;
     const int E = R.E;
@@ -1525,9 +1658,7 @@ int stage_develop(float* planes, float* mask, bool sum, int W, int H, const Stoc
     const int g = grid_for(n);
     Taps tp;
     int rc;
-    if (sum) lut_reduce_kernel<true><<<g, 256, 0, s>>>(planes, mask, n, E, dR);
-    else lut_reduce_kernel<false><<<g, 256, 0, s>>>(planes, mask, n, E, dR);
-    note_launch();
+    if ((rc = launch_reduce(planes, mask, sum, deep, n, R, dR, s))) return rc;
     if (result) *result = planes;
     if (R.dir_any && R.sigma_dir >= 1e-3f) {
         if ((rc = taps_for(R.sigma_dir, &tp))) return rc;
@@ -1606,9 +1737,10 @@ int run_reference(float* rgb, int W, int H, const Stock& st, uint64_t seed, int 
     double* sums = A.take<double>(MAXE);
     int rc;
     if ((rc = stage_expose(rgb, W, H, st, planes, s))) return rc;
-    if ((rc = stage_halation(planes, W, H, st, tmp, noise, s))) return rc;
+    float* deep = nullptr;
+    if ((rc = stage_halation(planes, W, H, st, tmp, noise, &deep, s))) return rc;
     float* dens = nullptr;
-    if ((rc = stage_develop(planes, mask, true, W, H, st, dR, inh, tmp, &dens, s))) return rc;
+    if ((rc = stage_develop(planes, mask, true, deep, W, H, st, dR, inh, tmp, &dens, s))) return rc;
     // the other set of planes is free after develop: it holds the grain's block sums
     float* spare = dens == planes ? inh : planes;
     if (grain && (rc = stage_grain(dens, W, H, st, seed, noise, reinterpret_cast<double*>(spare), sums, s))) return rc;
@@ -1855,7 +1987,12 @@ extern "C" int imops_film_halation(float* planes, int w, int h, const ImopsFilmP
     if (!planes) return fail(IMOPS_ERR_INVALID_ARGUMENT, "film_halation: NULL buffer");
     float* tmp = c.A.take<float>(n);
     float* bounce = c.A.take<float>(n);
-    if ((rc = film::stage_halation(planes, w, h, c.st, tmp, bounce, s))) return rc;
+    float* deep = nullptr;
+    if ((rc = film::stage_halation(planes, w, h, c.st, tmp, bounce, &deep, s))) return rc;
+    if (deep) {
+        film::bounce_kernel<<<film::grid_for(n), 256, 0, s>>>(planes, deep, n, c.st.ref.E, film::bounce_gains(c.st.ref));
+        note_launch();
+    }
     IMOPS_CUDA_TRY(cudaGetLastError(), "film_halation");
     return IMOPS_OK;
 }
@@ -1871,7 +2008,7 @@ extern "C" int imops_film_develop(float* planes, float* mask, int w, int h, cons
     if (!planes || !mask) return fail(IMOPS_ERR_INVALID_ARGUMENT, "film_develop: NULL buffer");
     float* inh = c.A.take<float>((size_t)c.st.ref.E * n);
     float* tmp = c.A.take<float>(n);
-    if ((rc = film::stage_develop(planes, mask, false, w, h, c.st, c.dR, inh, tmp, nullptr, s))) return rc;
+    if ((rc = film::stage_develop(planes, mask, false, nullptr, w, h, c.st, c.dR, inh, tmp, nullptr, s))) return rc;
     IMOPS_CUDA_TRY(cudaGetLastError(), "film_develop");
     return IMOPS_OK;
 }

@@ -54,7 +54,6 @@ struct RefSpec {
     float hal_gain[MAXE];
     // capture LUT + reciprocity (capture.rs:61-88, exposure/mod.rs:97-115)
     float eta[MAXE];
-    float lut_log[MAXE][LUTN];
     float lut_frac[MAXE][LUTN];
     // reduce (reduction.rs:16-68)
     float dmax[MAXE], inv_gamma[MAXE], mask_scale[MAXE];

@@ -425,7 +425,6 @@ int build_reference(const StockDef& sd, int W, float shutter, Stock* st, float* 
             double ph = std::pow(10.0, lp);
             double f = 1.0 - expected_survival(L.mu_ln, L.sigma_ln, L.capture_k, ph);
             f = f < 0.0 ? 0.0 : (f > 1.0 ? 1.0 : f);
-            R.lut_log[e][i] = (float)lp;
             R.lut_frac[e][i] = (float)f;
         }
         R.dmax[e] = L.dmax;
