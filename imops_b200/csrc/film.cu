@@ -592,113 +592,94 @@ __global__ void dir_apply_kernel(float* __restrict__ planes, const float* __rest
 // uses draws 12x+1..12x+12 of the row stream and is generated independently.
 
 // The blurred grain fields of LAYERS consecutive RNG layers of one tile in one
-// pass: Irwin-Hall noise over the tile plus its halo (grain_noise_at),
-// mirrored at the image edge; per layer the row then column passes of blur()
-// in shared memory with the same taps and summation order (so each field
-// equals blur(noise) bit for bit); the fields written, and each layer's block
-// sum of squares (f64) stored in partial[plane][block] for the variance.
+// pass: Irwin-Hall noise over the tile plus its halo, mirrored at the image
+// edge; per layer the row then column passes of blur() in shared memory with
+// the same taps and summation order; the fields written, and each layer's
+// block sum of squares (f64) stored in partial[plane][block] for the variance.
 // Plane z holds RNG layer layer0 + z.  Radius <= GR_MAXR.
 //
-// Tiles are 128 x 39: the three layers' noise and one row-blurred layer take
-// 96 KB at radius 3, so two blocks (32 warps) share an SM.  Inside the image
-// a thread generates a run of GR_RUN consecutive pixels of a row, whose
-// layers share all but the last two draws of the next pixel
-// (grain_noise_run): 12 GR_RUN + 2 draws a run instead of 14 a pixel.  The
-// 45 rows of a tile and its halo at radius 3 are 1530 runs, three for each
-// of the 512 threads.
-constexpr int GR_TW = 128, GR_TH = 39, GR_MAXR = 16, GR_RUN = 4;
-constexpr int GR_THREADS = 512, GR_TY = GR_THREADS / 32;
+// Layer L of row y is the SplitMix64 stream seeded seed*0xD1B54A32D192ED03 +
+// L*golden + y, and pixel x takes its draws 12x+1 .. 12x+12, the sum of those
+// 12 uniforms minus 6 (grain.rs:20-45, 53-66).  Draw k of layer L has the
+// state seed*C + y + (L + 12x + k)*golden, which is draw L + k of layer 0's
+// stream: the layers of a run of RUN pixels take 12 RUN + LAYERS - 1 draws of
+// one stream, each mixed once, and every (pixel, layer) sum is a difference
+// of two prefix sums.
+//
+// A draw enters the sums as the upper 28 bits of its 64 (modulo 2^32, which
+// differences of 12 such draws cannot exceed), with the mean of what is cut
+// off added back: a uniform is then good to 2^-29 and the sum exact until its
+// one conversion to f32, where twelve f32 additions rounded at 2^-22 each.  The
+// mixer's last xor-shift by 31 reaches only bit 32 of a draw, so it is left out.
+//
+// Bound by the integer ALU (11 of the 17 instructions of a draw) at 32 warps
+// an SM.  Tiles are 128 wide and TH high, their runs a whole number of
+// rounds of the 512 threads where that fits two blocks an SM: 39 rows for up
+// to three layers (96 KB), 24 for six (113 KB).  Six layers in one block mix
+// 13.25 draws a pixel, two blocks of three 25.  Images of fewer tiles than two an
+// SM take tiles of 18 rows, so that the few blocks finish sooner (1.1 MP: 36
+// us against 44).  24 MP: three layers 0.44 ms (0.57 with f32 sums of draws
+// converted one by one), six layers 0.61 ms (2.55 one layer a launch).
+constexpr int GR_TW = 128, GR_MAXR = 16, GR_RUN = 4;
+constexpr int GR_THREADS = 512, GR_GROUPS = GR_THREADS / GR_TW;
+constexpr int GR_TH = 39, GR_TH6 = 24, GR_TH_SMALL = 18;
 static_assert(GR_TW == 128, "the blur loops index tile columns with & 127");
+// output rows a thread, and rows of the row-blurred buffer: the last group's
+// window reaches past the tile's halo where TH is not a multiple of the groups
+constexpr int gr_rows(int th) { return (th + GR_GROUPS - 1) / GR_GROUPS; }
+constexpr int gr_row_buffer(int th, int R) { return GR_GROUPS * gr_rows(th) + 2 * R; }
 
-// Noise of pixel (y, x) in LAYERS consecutive layers layer0, layer0+1, ...
-// (grain.rs:20-45, 53-66).  Layer L of row y is the SplitMix64 stream seeded
-// seed*0xD1B54A32D192ED03 + L*golden + y, and pixel x takes its draws
-// 12x+1 .. 12x+12, the sum of those 12 uniforms minus 6.  Draw k of layer L
-// has the state seed*C + y + (L + 12x + k)*golden, which is draw L + k of
-// layer 0's stream: consecutive layers share all but one of their draws.  So
-// the layers of pixel x take the LAYERS + 11 draws 12x+layer0+1 .. of one
-// stream, each draw mixed once, and layer layer0 + z sums draws z+1 .. z+12
-// of them in order (each sum in f32, in the reference's order).
-template <int LAYERS>
-__device__ __forceinline__ void grain_noise_at(uint64_t seed, int layer0, int y, int x, float (&out)[LAYERS]) {
-    const uint64_t golden = 0x9E3779B97F4A7C15ull;
-    // state of draw k is s0 + k * golden (mod 2^64): stepped, not multiplied
-    uint64_t z0 = seed * 0xD1B54A32D192ED03ull + (uint64_t)layer0 * golden + (uint64_t)y + 12 * (uint64_t)x * golden;
-    float acc[LAYERS];
-#pragma unroll
-    for (int z = 0; z < LAYERS; z++) acc[z] = 0.0f;
-#pragma unroll
-    for (int k = 1; k <= LAYERS + 11; k++) {
-        z0 += golden;
-        uint64_t v = (z0 ^ (z0 >> 30)) * 0xBF58476D1CE4E5B9ull;
-        v = (v ^ (v >> 27)) * 0x94D049BB133111EBull;
-        const float u = __ull2float_rn(v ^ (v >> 31)) / 18446744073709551616.0f;
-#pragma unroll
-        for (int z = 0; z < LAYERS; z++)
-            if (k >= z + 1 && k <= z + 12) acc[z] += u;
-    }
-#pragma unroll
-    for (int z = 0; z < LAYERS; z++) out[z] = acc[z] - 6.0f;
-}
-
-// The same for RUN consecutive pixels x .. x+RUN-1 of row y: pixel x+i takes
-// draws 12i+1 .. 12i+LAYERS+11 counted from pixel x's first, so the run
-// mixes its 12 RUN + LAYERS - 1 draws once each; every (pixel, layer) sum adds
-// its 12 draws in the order grain_noise_at does, so the values are identical.
+// The sums of RUN consecutive pixels x .. x+RUN-1 of row y in layers layer0 ..
+// layer0+LAYERS-1, as noise values (sum minus 6).
 template <int LAYERS, int RUN>
-__device__ __forceinline__ void grain_noise_run(uint64_t seed, int layer0, int y, int x, float (&out)[RUN][LAYERS]) {
+__device__ __forceinline__ void grain_noise(uint64_t seed, int layer0, int y, int x, float (&out)[RUN][LAYERS]) {
+    static_assert(LAYERS <= 12, "the prefix sums kept are those of the last pixel's start");
     const uint64_t golden = 0x9E3779B97F4A7C15ull;
+    // state of draw k is z0 + k * golden (mod 2^64): stepped, not multiplied
     uint64_t z0 = seed * 0xD1B54A32D192ED03ull + (uint64_t)layer0 * golden + (uint64_t)y + 12 * (uint64_t)x * golden;
-    float acc[RUN][LAYERS];
-#pragma unroll
-    for (int i = 0; i < RUN; i++)
-#pragma unroll
-        for (int z = 0; z < LAYERS; z++) acc[i][z] = 0.0f;
+    uint32_t sum = 0, start[LAYERS];  // prefix sum, and its value before each layer's draws of the pixel
+    start[0] = 0;
 #pragma unroll
     for (int k = 1; k <= 12 * RUN + LAYERS - 1; k++) {
         z0 += golden;
         uint64_t v = (z0 ^ (z0 >> 30)) * 0xBF58476D1CE4E5B9ull;
         v = (v ^ (v >> 27)) * 0x94D049BB133111EBull;
-        const float u = __ull2float_rn(v ^ (v >> 31)) / 18446744073709551616.0f;
-#pragma unroll
-        for (int i = 0; i < RUN; i++)
-#pragma unroll
-            for (int z = 0; z < LAYERS; z++)
-                if (k >= 12 * i + z + 1 && k <= 12 * i + z + 12) acc[i][z] += u;
+        sum += (uint32_t)(v >> 32) >> 4;
+        const int z = k % 12, i = k / 12 - 1;
+        if (z < LAYERS) {
+            // 6 for the mean, 6 half units for the bits cut off
+            if (i >= 0) out[i][z] = (float)(int)(sum - start[z] - 0x60000000u + 6u) * (1.0f / 268435456.0f);
+            start[z] = sum;
+        }
     }
-#pragma unroll
-    for (int i = 0; i < RUN; i++)
-#pragma unroll
-        for (int z = 0; z < LAYERS; z++) out[i][z] = acc[i][z] - 6.0f;
 }
 
-template <int LAYERS>
+template <int LAYERS, int TH>
 __global__ void __launch_bounds__(GR_THREADS, 2) grain_field_kernel(float* __restrict__ noise, int W, int H,
-                                                                    uint64_t seed, int layer0, Taps tp,
+                                                                    uint64_t seed, int layer0,
+                                                                    const __grid_constant__ Taps tp,
                                                                     double* __restrict__ partial) {
     extern __shared__ __align__(16) float gsm[];
-    __shared__ double red[GR_TY];
+    __shared__ double red[GR_THREADS / 32];
     const int R = tp.R;
-    const int x0 = blockIdx.x * GR_TW, y0 = blockIdx.y * GR_TH;
-    const int tid = threadIdx.y * 32 + threadIdx.x;
+    const int x0 = blockIdx.x * GR_TW, y0 = blockIdx.y * TH;
+    const int tid = threadIdx.x;
     // noise rows are NW samples; stored with a stride of NWP (a multiple of
     // the run, so runs and their float4 stores stay aligned)
-    const int NW = GR_TW + 2 * R, NH = GR_TH + 2 * R;
+    const int NW = GR_TW + 2 * R, NH = TH + 2 * R;
     const int NWP = (NW + GR_RUN - 1) / GR_RUN * GR_RUN;
     float* sn = gsm;                      // noise, tile + halo: LAYERS x NH x NWP
-    float* sr = gsm + LAYERS * NH * NWP;  // row-blurred: NH x GR_TW (one layer at a time)
-    // blocks whose tile + halo lies inside the image need no mirroring
-    const bool inner = x0 - R >= 0 && y0 - R >= 0 && x0 + GR_TW + R <= W && y0 + GR_TH + R <= H;
-    if (inner) {
-        // runs of GR_RUN pixels over the rows (the last run of a row may
-        // reach past NW: those samples are generated and never read);
-        // (row, run) of j stepped without a division
+    float* sr = gsm + LAYERS * NH * NWP;  // row-blurred: gr_row_buffer rows x GR_TW (one layer at a time)
+    if (x0 - R >= 0 && x0 + NWP - R <= W) {
+        // runs of GR_RUN pixels over the rows (rows mirrored; the last run of
+        // a row may reach past NW: those samples are generated and never
+        // read); (row, run) of j stepped without a division
         const int RPR = NWP / GR_RUN, nruns = NH * RPR;
         const int dq = GR_THREADS / RPR, dr = GR_THREADS - dq * RPR;
         int r = tid / RPR, q = tid - (tid / RPR) * RPR;
         for (int j = tid; j < nruns; j += GR_THREADS) {
             float v[GR_RUN][LAYERS];
-            grain_noise_run<LAYERS, GR_RUN>(seed, layer0, y0 - R + r, x0 - R + q * GR_RUN, v);
+            grain_noise<LAYERS, GR_RUN>(seed, layer0, reflect(y0 - R + r, H), x0 - R + q * GR_RUN, v);
 #pragma unroll
             for (int z = 0; z < LAYERS; z++) {
                 static_assert(GR_RUN == 4, "one float4 store a run and layer");
@@ -716,10 +697,10 @@ __global__ void __launch_bounds__(GR_THREADS, 2) grain_field_kernel(float* __res
         const int dq = GR_THREADS / NW, dr = GR_THREADS - dq * NW;
         int r = tid / NW, c = tid - (tid / NW) * NW;
         for (int idx = tid; idx < NH * NW; idx += GR_THREADS) {
-            float v[LAYERS];
-            grain_noise_at<LAYERS>(seed, layer0, reflect(y0 - R + r, H), reflect(x0 - R + c, W), v);
+            float v[1][LAYERS];
+            grain_noise<LAYERS, 1>(seed, layer0, reflect(y0 - R + r, H), reflect(x0 - R + c, W), v);
 #pragma unroll
-            for (int z = 0; z < LAYERS; z++) sn[(z * NH + r) * NWP + c] = v[z];
+            for (int z = 0; z < LAYERS; z++) sn[(z * NH + r) * NWP + c] = v[0][z];
             r += dq;
             c += dr;
             if (c >= NW) {
@@ -729,45 +710,77 @@ __global__ void __launch_bounds__(GR_THREADS, 2) grain_field_kernel(float* __res
         }
     }
     const size_t n = (size_t)W * H;
+    const int c = tid & (GR_TW - 1), x = x0 + c;
+#pragma unroll 1
     for (int z = 0; z < LAYERS; z++) {
         const float* snz = sn + z * NH * NWP;
-        __syncthreads();  // the noise is complete; sr is free again
-        for (int idx = tid; idx < NH * GR_TW; idx += GR_THREADS) {
-            const int r = idx >> 7, c = idx & (GR_TW - 1);
-            const float* s = snz + r * NWP + c;
-            float acc = 0.0f;
-            // radius 3 (a 1 px grain blur, every stock here) unrolled
-            if (R == 3) {
-#pragma unroll
-                for (int k = 0; k <= 6; k++) acc = fmaf(s[k], tp.t[k], acc);
-            } else {
-                for (int k = 0; k <= 2 * R; k++) acc = fmaf(s[k], tp.t[k], acc);
-            }
-            sr[idx] = acc;
-        }
-        __syncthreads();
+        float* out = noise + z * n + x;
         double sq = 0.0;
-        for (int idx = tid; idx < GR_TH * GR_TW; idx += GR_THREADS) {
-            const int r = idx >> 7, c = idx & (GR_TW - 1);
-            const int y = y0 + r, x = x0 + c;
-            if (y >= H || x >= W) continue;
-            const float* s = sr + idx;
-            float acc = 0.0f;
-            if (R == 3) {
+        __syncthreads();  // the noise is complete; sr is free again
+        if (R == 3) {
+            // radius 3 (a 1 px grain blur, every stock here): four outputs of
+            // a row a thread, then a column of ROWS outputs, each from a
+            // register window
+            constexpr int ROWS = gr_rows(TH);
+            for (int idx = tid; idx < NH * (GR_TW / 4); idx += GR_THREADS) {
+                const int r = idx / (GR_TW / 4), g = idx % (GR_TW / 4);
+                float w[12], a[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
-                for (int k = 0; k <= 6; k++) acc = fmaf(s[k * GR_TW], tp.t[k], acc);
-            } else {
-                for (int k = 0; k <= 2 * R; k++) acc = fmaf(s[k * GR_TW], tp.t[k], acc);
+                for (int t = 0; t < 3; t++) {
+                    const float4 v = *reinterpret_cast<const float4*>(snz + r * NWP + 4 * g + 4 * t);
+                    w[4 * t] = v.x;
+                    w[4 * t + 1] = v.y;
+                    w[4 * t + 2] = v.z;
+                    w[4 * t + 3] = v.w;
+                }
+#pragma unroll
+                for (int k = 0; k <= 6; k++)
+#pragma unroll
+                    for (int j = 0; j < 4; j++) a[j] = fmaf(w[j + k], tp.t[k], a[j]);
+                *reinterpret_cast<float4*>(sr + r * GR_TW + 4 * g) = make_float4(a[0], a[1], a[2], a[3]);
             }
-            noise[z * n + (size_t)y * W + x] = acc;
-            sq += (double)acc * (double)acc;
+            __syncthreads();
+            const int rb = tid / GR_TW * ROWS;
+            float a[ROWS];
+#pragma unroll
+            for (int j = 0; j < ROWS; j++) a[j] = 0.0f;
+#pragma unroll
+            for (int m = 0; m < ROWS + 6; m++) {
+                const float v = sr[(rb + m) * GR_TW + c];
+#pragma unroll
+                for (int j = 0; j < ROWS; j++)
+                    if (m - j >= 0 && m - j <= 6) a[j] = fmaf(v, tp.t[m - j], a[j]);
+            }
+#pragma unroll
+            for (int j = 0; j < ROWS; j++) {
+                const int r = rb + j;
+                if (r < TH && y0 + r < H && x < W) {
+                    out[(size_t)(y0 + r) * W] = a[j];
+                    sq += (double)a[j] * (double)a[j];
+                }
+            }
+        } else {
+            for (int idx = tid; idx < NH * GR_TW; idx += GR_THREADS) {
+                const float* s = snz + (idx >> 7) * NWP + c;
+                float acc = 0.0f;
+                for (int k = 0; k <= 2 * R; k++) acc = fmaf(s[k], tp.t[k], acc);
+                sr[idx] = acc;
+            }
+            __syncthreads();
+            for (int r = tid >> 7; r < TH; r += GR_GROUPS) {
+                if (y0 + r >= H || x >= W) continue;
+                float acc = 0.0f;
+                for (int k = 0; k <= 2 * R; k++) acc = fmaf(sr[(r + k) * GR_TW + c], tp.t[k], acc);
+                out[(size_t)(y0 + r) * W] = acc;
+                sq += (double)acc * (double)acc;
+            }
         }
         for (int o = 16; o > 0; o >>= 1) sq += __shfl_down_sync(0xffffffffu, sq, o);
-        if (threadIdx.x == 0) red[threadIdx.y] = sq;
+        if ((tid & 31) == 0) red[tid >> 5] = sq;
         __syncthreads();
         if (tid == 0) {
             double t = 0.0;
-            for (int w = 0; w < GR_TY; w++) t += red[w];
+            for (int w = 0; w < GR_THREADS / 32; w++) t += red[w];
             partial[(size_t)z * gridDim.x * gridDim.y + blockIdx.y * gridDim.x + blockIdx.x] = t;
         }
     }
@@ -790,45 +803,61 @@ __global__ void __launch_bounds__(1024) sum_partials_kernel(const double* __rest
     if (threadIdx.x == 0) sums[blockIdx.x] = red[0];
 }
 
+// Fewer tiles of full height than two an SM: the low tiles.
+static bool grain_small(int W, int H) {
+    return (size_t)((W + GR_TW - 1) / GR_TW) * ((H + GR_TH - 1) / GR_TH) < (size_t)sm_count() * 2;
+}
+
+// Doubles of scratch that grain_fields needs for its block sums.
+size_t grain_partials(int W, int H, int layers) {
+    const int th = grain_small(W, H) ? GR_TH_SMALL : (layers >= 6 ? GR_TH6 : GR_TH);
+    return (size_t)((W + GR_TW - 1) / GR_TW) * ((H + th - 1) / th) * layers;
+}
+
+template <int LAYERS, int TH>
+static int grain_launch(float* noise, int W, int H, uint64_t seed, int layer0, const Taps& tp, double* partial,
+                        double* sums, cudaStream_t s) {
+    const int NH = TH + 2 * tp.R, NWP = (GR_TW + 2 * tp.R + GR_RUN - 1) / GR_RUN * GR_RUN;
+    const size_t smem = (size_t)(LAYERS * NH * NWP + gr_row_buffer(TH, tp.R) * GR_TW) * sizeof(float);
+    IMOPS_CUDA_TRY(cudaFuncSetAttribute(grain_field_kernel<LAYERS, TH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)smem),
+                   "cudaFuncSetAttribute(grain)");
+    const dim3 g((W + GR_TW - 1) / GR_TW, (H + TH - 1) / TH);
+    grain_field_kernel<LAYERS, TH><<<g, GR_THREADS, smem, s>>>(noise, W, H, seed, layer0, tp, partial);
+    sum_partials_kernel<<<LAYERS, 1024, 0, s>>>(partial, (int)(g.x * g.y), sums);
+    note_launch(2);
+    return IMOPS_OK;
+}
+
 // Blurred grain fields of RNG layers layer0 .. layer0+layers-1 (planes
 // noise[z * n]) and their sums of squares sums[z].  partial: scratch of
 // grain_partials(W, H, layers) doubles.
-size_t grain_partials(int W, int H, int layers) {
-    return (size_t)((W + GR_TW - 1) / GR_TW) * ((H + GR_TH - 1) / GR_TH) * layers;
-}
-
 int grain_fields(float* noise, int W, int H, uint64_t seed, int layer0, int layers, const Taps& tp, double* partial,
                  double* sums, cudaStream_t s) {
     if (tp.R > GR_MAXR) return fail(IMOPS_ERR_UNSUPPORTED_SIZE, "film: grain blur radius above 16 px");
-    dim3 b(32, GR_TY), g((W + GR_TW - 1) / GR_TW, (H + GR_TH - 1) / GR_TH);
-    const int NW = GR_TW + 2 * tp.R, NH = GR_TH + 2 * tp.R;
-    const int NWP = (NW + GR_RUN - 1) / GR_RUN * GR_RUN;
-    // three layers per block (their draws shared) while their noise fits in
-    // shared memory; otherwise one block per (tile, layer)
-    const size_t smem3 = (size_t)NH * (3 * NWP + GR_TW) * sizeof(float);
-    const size_t n = (size_t)W * H, nb = (size_t)g.x * g.y;
-    int z = 0;
-    if (layers >= 3 && smem3 <= 200 * 1024) {
-        IMOPS_CUDA_TRY(cudaFuncSetAttribute(grain_field_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            (int)smem3),
-                       "cudaFuncSetAttribute(grain)");
-        for (; z + 3 <= layers; z += 3) {
-            grain_field_kernel<3><<<g, b, smem3, s>>>(noise + z * n, W, H, seed, layer0 + z, tp, partial + z * nb);
-            note_launch();
+    const size_t n = (size_t)W * H;
+    const bool small = grain_small(W, H);
+    for (int z = 0; z < layers;) {
+        int rc, take;
+        float* nz = noise + z * n;
+        const int left = layers - z, l0 = layer0 + z;
+        if (left >= 6 && tp.R <= 3 && !small) {  // six layers and a wider halo outgrow the shared memory
+            take = 6;
+            rc = grain_launch<6, GR_TH6>(nz, W, H, seed, l0, tp, partial, sums + z, s);
+        } else if (left >= 3) {
+            take = 3;
+            rc = small ? grain_launch<3, GR_TH_SMALL>(nz, W, H, seed, l0, tp, partial, sums + z, s)
+                       : grain_launch<3, GR_TH>(nz, W, H, seed, l0, tp, partial, sums + z, s);
+        } else if (left == 2) {
+            take = 2;
+            rc = grain_launch<2, GR_TH>(nz, W, H, seed, l0, tp, partial, sums + z, s);
+        } else {
+            take = 1;
+            rc = grain_launch<1, GR_TH>(nz, W, H, seed, l0, tp, partial, sums + z, s);
         }
+        if (rc) return rc;
+        z += take;
     }
-    if (z < layers) {
-        const size_t smem1 = (size_t)NH * (NWP + GR_TW) * sizeof(float);
-        IMOPS_CUDA_TRY(cudaFuncSetAttribute(grain_field_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            (int)smem1),
-                       "cudaFuncSetAttribute(grain)");
-        for (; z < layers; z++) {
-            grain_field_kernel<1><<<g, b, smem1, s>>>(noise + z * n, W, H, seed, layer0 + z, tp, partial + z * nb);
-            note_launch();
-        }
-    }
-    sum_partials_kernel<<<layers, 1024, 0, s>>>(partial, (int)nb, sums);
-    note_launch();
     IMOPS_CUDA_TRY(cudaGetLastError(), "grain fields");
     return IMOPS_OK;
 }
@@ -1556,9 +1585,9 @@ struct Arena {
     }
 };
 
-size_t ref_workspace_bytes(size_t n, int E) {
-    // planes(E) + inh(E) + mask sum(1) + tmp(1) + noise(1) + spec copy + sums
-    return (size_t)(2 * E + 3) * n * 4 + sizeof(RefSpec) + 64 * 1024;
+size_t ref_workspace_bytes(int W, int H, int E) {
+    // planes(E) + inh(E) + mask sum(1) + tmp(1) + bounce(1) + grain partials + spec copy + sums
+    return (size_t)(2 * E + 3) * W * H * 4 + grain_partials(W, H, E) * 8 + sizeof(RefSpec) + 64 * 1024;
 }
 
 // The reference model's stages (film/mod.rs:77-129), each on the stock's E
@@ -1690,7 +1719,7 @@ int stage_develop(float* planes, float* mask, bool sum, const float* deep, int W
 }
 
 //   grain: seeded SplitMix64 fields, normalised and scaled per layer
-//     (grain.rs:53-100); noise: one plane, partial: grain_partials(W, H, 1)
+//     (grain.rs:53-100); noise: E planes, partial: grain_partials(W, H, E)
 //     doubles, sums: MAXE doubles
 int stage_grain(float* planes, int W, int H, const Stock& st, uint64_t seed, float* noise, double* partial,
                 double* sums, cudaStream_t s) {
@@ -1699,11 +1728,11 @@ int stage_grain(float* planes, int W, int H, const Stock& st, uint64_t seed, flo
     Taps tp;
     int rc;
     if ((rc = taps_for(fmaxf(R.sigma_grain, 1.0f), &tp))) return rc;
-    IMOPS_CUDA_TRY(cudaMemsetAsync(sums, 0, MAXE * sizeof(double), s), "memset");
+    if ((rc = grain_fields(noise, W, H, seed, 0, R.E, tp, partial, sums, s))) return rc;
     for (int e = 0; e < R.E; e++) {
         if (R.kappa[e] <= 0.0f || R.dmax[e] <= 0.0f) continue;
-        if ((rc = grain_fields(noise, W, H, seed, e, 1, tp, partial, sums + e, s))) return rc;
-        grain_apply_kernel<<<grid_for(n), 256, 0, s>>>(planes + e * n, noise, n, sums + e, R.kappa[e], R.dmax[e]);
+        grain_apply_kernel<<<grid_for(n), 256, 0, s>>>(planes + e * n, noise + e * n, n, sums + e, R.kappa[e],
+                                                      R.dmax[e]);
         note_launch();
     }
     return IMOPS_OK;
@@ -1733,17 +1762,18 @@ int run_reference(float* rgb, int W, int H, const Stock& st, uint64_t seed, int 
     float* mask = A.take<float>(n);  // the layers' mask sum
     float* inh = A.take<float>(E * n);
     float* tmp = A.take<float>(n);
-    float* noise = A.take<float>(n);
+    float* bounce = A.take<float>(n);
+    double* partial = A.take<double>(grain_partials(W, H, E));
     double* sums = A.take<double>(MAXE);
     int rc;
     if ((rc = stage_expose(rgb, W, H, st, planes, s))) return rc;
     float* deep = nullptr;
-    if ((rc = stage_halation(planes, W, H, st, tmp, noise, &deep, s))) return rc;
+    if ((rc = stage_halation(planes, W, H, st, tmp, bounce, &deep, s))) return rc;
     float* dens = nullptr;
     if ((rc = stage_develop(planes, mask, true, deep, W, H, st, dR, inh, tmp, &dens, s))) return rc;
-    // the other set of planes is free after develop: it holds the grain's block sums
+    // the other set of planes is free after develop: it takes the grain fields
     float* spare = dens == planes ? inh : planes;
-    if (grain && (rc = stage_grain(dens, W, H, st, seed, noise, reinterpret_cast<double*>(spare), sums, s))) return rc;
+    if (grain && (rc = stage_grain(dens, W, H, st, seed, spare, partial, sums, s))) return rc;
     if ((rc = stage_scan(dens, mask, true, W, H, st.scan16, rgb, s))) return rc;
     IMOPS_CUDA_TRY(cudaGetLastError(), "film kernels");
     return IMOPS_OK;
@@ -1752,7 +1782,7 @@ int run_reference(float* rgb, int W, int H, const Stock& st, uint64_t seed, int 
 // PositiveLinear's reference points (film/mod.rs:136-151): the mean RGB of
 // a 32x32 mid-grey patch through the same path (seed 0) into mid_dmin[0..2]
 // and the stock's normalised Dmin into mid_dmin[3..5].  Takes
-// ref_workspace_bytes(1024, E) + 1024 * 12 bytes of A.
+// ref_workspace_bytes(32, 32, E) + 1024 * 12 bytes of A.
 int mid_gray_negative(const Stock& st, int grain, Arena& A, const RefSpec* dR, float* mid_dmin, cudaStream_t s) {
     const size_t nm = 32 * 32;
     float g = relative_to_absolute_y(0.185f, st.ref.box_iso);
@@ -1774,7 +1804,7 @@ int process_reference(float* rgb, int W, int H, const ImopsFilmParams& P, cudaSt
     if (rc) return rc;
     const size_t n = (size_t)W * H;
     const size_t nm = 32 * 32;
-    size_t bytes = ref_workspace_bytes(n, st.ref.E) + ref_workspace_bytes(nm, st.ref.E) + nm * 12 + 4096;
+    size_t bytes = ref_workspace_bytes(W, H, st.ref.E) + ref_workspace_bytes(32, 32, st.ref.E) + nm * 12 + 4096;
     void* ws = nullptr;
     if ((rc = workspace(s, bytes, &ws))) return rc;
     Arena A{static_cast<char*>(ws), 0};
@@ -2017,13 +2047,13 @@ extern "C" int imops_film_grain(float* planes, int w, int h, const ImopsFilmPara
     clear_error();
     cudaStream_t s = as_stream(stream);
     const size_t n = (size_t)(w > 0 ? w : 0) * (h > 0 ? h : 0);
-    const size_t np = w > 0 && h > 0 ? film::grain_partials(w, h, 1) : 0;
+    const size_t np = w > 0 && h > 0 ? film::grain_partials(w, h, film::MAXE) : 0;
     film::StageCtx c;
-    int rc = film::stage_ctx(params, w, h, n * 4 + np * 8 + film::MAXE * 8 + 768, s, &c);
+    int rc = film::stage_ctx(params, w, h, film::MAXE * n * 4 + np * 8 + film::MAXE * 8 + 768, s, &c);
     if (rc) return rc;
     if (!planes) return fail(IMOPS_ERR_INVALID_ARGUMENT, "film_grain: NULL buffer");
     if (!params->grain) return IMOPS_OK;
-    float* noise = c.A.take<float>(n);
+    float* noise = c.A.take<float>(c.st.ref.E * n);
     double* partial = c.A.take<double>(np);
     double* sums = c.A.take<double>(film::MAXE);
     if ((rc = film::stage_grain(planes, w, h, c.st, params->seed, noise, partial, sums, s))) return rc;
@@ -2050,7 +2080,7 @@ extern "C" int imops_film_invert(float* rgb, int w, int h, const ImopsFilmParams
     // the mid-grey patch's path and its reference points come from the same arena
     const size_t nm = 32 * 32;
     film::StageCtx c;
-    int rc = film::stage_ctx(params, w, h, film::ref_workspace_bytes(nm, film::MAXE) + nm * 12 + 1024, s, &c);
+    int rc = film::stage_ctx(params, w, h, film::ref_workspace_bytes(32, 32, film::MAXE) + nm * 12 + 1024, s, &c);
     if (rc) return rc;
     if (!rgb) return fail(IMOPS_ERR_INVALID_ARGUMENT, "film_invert: NULL buffer");
     if (!(params->output == IMOPS_FILM_POSITIVE_LINEAR && !c.st.ref.any_reversal)) return IMOPS_OK;

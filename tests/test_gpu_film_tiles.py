@@ -60,3 +60,48 @@ def test_develop_agrees_across_the_tile_radius_line(gpu, stock):
         assert float((dens - dens[:, :1, :1]).abs().max()) < 1e-5
         res.append(torch.cat([dens[:, 0, 0], mask[:, 0, 0]]))
     assert float((res[0] - res[1]).abs().max()) < 1e-5
+
+
+def _noise_rows(seed, layer, y0, y1, W):
+    """Unblurred grain of rows y0..y1-1: the sum of twelve SplitMix64 uniforms a pixel, minus 6."""
+    m = (1 << 64) - 1
+    golden = 0x9E3779B97F4A7C15
+    y = np.arange(y0, y1, dtype=np.uint64)[:, None]
+    x = np.arange(W, dtype=np.uint64)[None, :]
+    base = np.uint64((seed * 0xD1B54A32D192ED03 + layer * golden) & m) + y + x * np.uint64((12 * golden) & m)
+    acc = np.zeros(base.shape)
+    for k in range(1, 13):
+        z = base + np.uint64((k * golden) & m)
+        z = (z ^ (z >> np.uint64(30))) * np.uint64(0xBF58476D1CE4E5B9)
+        z = (z ^ (z >> np.uint64(27))) * np.uint64(0x94D049BB133111EB)
+        acc += (z ^ (z >> np.uint64(31))).astype(np.float64) / 2.0 ** 64
+    return acc - 6.0
+
+
+@pytest.mark.parametrize("stock,H,W", [(2, 1500, 2100), (4, 1500, 2100), (1, 1500, 2100), (1, 300, 517), (6, 300, 517)])
+def test_grain_fields_match_the_generator(gpu, stock, H, W):
+    """The grain added to flat planes, against the generator in 64 bits, over
+    rows that cross tile edges, for one block of six layers (2), six and one
+    (4), three (1), the low tiles of small images, and two layers (6).  Up to
+    the layer's amplitude the added densities are the blurred noise.  Error: two
+    f32 roundings of an output below 0.5 (6e-8 each), and 1e-5 of the
+    grain for the rounding of its blur and scale."""
+    import torch
+
+    import imops_b200 as im
+    seed, y0, y1 = 12345, 20, 64
+    st = im.FilmStages(stock=stock, seed=seed, grain=True)
+    planes = torch.full((st.layers, H, W), 0.25, device=gpu)  # inside every layer's range
+    out = st.grain(planes.clone()).cpu().numpy().astype(np.float64) - 0.25
+    t = np.exp(-np.arange(-3, 4) ** 2 / 2.0)
+    t /= t.sum()
+    for e in range(st.layers):
+        n = _noise_rows(seed, e, y0 - 3, y1 + 3, W)
+        n = np.pad(n, ((0, 0), (3, 3)), mode="reflect")
+        n = sum(t[k] * n[:, k:k + W] for k in range(7))
+        n = sum(t[k] * n[k:k + y1 - y0] for k in range(7))
+        got = out[e, y0:y1]
+        scale = (got * n).sum() / (n * n).sum()
+        assert scale > 0
+        assert np.abs(got - scale * n).max() < 1e-5 * np.abs(got).max() + 1.2e-7
+        assert abs(got.std() / out[e].std() - 1) < 0.05
