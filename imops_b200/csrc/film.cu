@@ -72,16 +72,20 @@ __device__ __forceinline__ int reflect(int i, int n) {
 // ---------------------------------------------------------------------------
 // exposure
 
-// The basis weights of one pixel: w = max(0, Minv * rgb).
+// The basis weights of one pixel: w = max(0, Minv * rgb).  Explicit
+// multiply-adds: a kernel of its own and a fused one give the same bits.
+__device__ __forceinline__ float dot3(float a0, float x0, float a1, float x1, float a2, float x2) {
+    return fmaf(a2, x2, fmaf(a1, x1, __fmul_rn(a0, x0)));
+}
 __device__ __forceinline__ void basis_weights(const ExposeSpec& X, float r, float g, float b, float (&w)[3]) {
-    w[0] = fmaxf(0.0f, X.minv[0] * r + X.minv[1] * g + X.minv[2] * b);
-    w[1] = fmaxf(0.0f, X.minv[3] * r + X.minv[4] * g + X.minv[5] * b);
-    w[2] = fmaxf(0.0f, X.minv[6] * r + X.minv[7] * g + X.minv[8] * b);
+    w[0] = fmaxf(0.0f, dot3(X.minv[0], r, X.minv[1], g, X.minv[2], b));
+    w[1] = fmaxf(0.0f, dot3(X.minv[3], r, X.minv[4], g, X.minv[5], b));
+    w[2] = fmaxf(0.0f, dot3(X.minv[6], r, X.minv[7], g, X.minv[8], b));
 }
 
 // Layer e's absorbed band-mean fluence from the basis weights.
 __device__ __forceinline__ float layer_exposure(const ExposeSpec& X, const float (&w)[3], int e) {
-    return w[0] * X.A[0][e] + w[1] * X.A[1][e] + w[2] * X.A[2][e];
+    return dot3(X.A[0][e], w[0], X.A[1][e], w[1], X.A[2][e], w[2]);
 }
 
 // rgb (interleaved) -> E planes of absorbed band-mean fluence, optional
@@ -357,19 +361,20 @@ struct EpiStore {
     __device__ __forceinline__ void operator()(size_t i, float v) const { out[i] = v; }
 };
 // local scatter: p = keep*p + mix*blur(p) (halation.rs:164-181)
+__device__ __forceinline__ float mix_px(float p, float v, float keep, float mix) {
+    return fmaf(mix, v, __fmul_rn(keep, p));
+}
 struct EpiMix {
     float* plane;
     float keep, mix;
-    __device__ __forceinline__ void operator()(size_t i, float v) const { plane[i] = keep * plane[i] + mix * v; }
+    __device__ __forceinline__ void operator()(size_t i, float v) const { plane[i] = mix_px(plane[i], v, keep, mix); }
 };
 // adjacency: d += beta * (d - blur(d)) (diffusion.rs:11-28)
+__device__ __forceinline__ float adjacency_px(float d, float v, float beta) { return fmaf(beta, __fsub_rn(d, v), d); }
 struct EpiAdjacency {
     float* plane;
     float beta;
-    __device__ __forceinline__ void operator()(size_t i, float v) const {
-        float d = plane[i];
-        plane[i] = d + beta * (d - v);
-    }
+    __device__ __forceinline__ void operator()(size_t i, float v) const { plane[i] = adjacency_px(plane[i], v, beta); }
 };
 
 struct EpiAdd {
@@ -487,9 +492,10 @@ struct Reduce {
 // log10 phi over LUTN entries at -4 .. 8 in equal steps, so the cell is found
 // by arithmetic (a search over the knots before).  With phi = 2^k m, m in
 // [1, 2), the place in cells is SCALE k + SCALE log2 m + ZERO; the first
-// term is exact but for the low part of SCALE (k times its upper 12 bits),
-// so the offset in the cell is good to about 4e-7 (the hardware logarithm of
-// m), where a logarithm of phi itself, up to 27, rounds at 1e-6.
+// term is exact but for the low part of SCALE (k times its upper 12 bits), and
+// log2 m is at most 1, where a logarithm of phi itself, up to 27, rounds at
+// 1e-6.  (The hardware logarithm for log2 m: 0.44 ms instead of 0.55 for the
+// reduction, but Portra400's error against 64 bits rose from 1.2e-7 to 1.3e-7.)
 // lut[i] = (entry i, entry i+1 - entry i).
 __device__ __forceinline__ float lut_sample(const float2* lut, float phi) {
     constexpr double SCALE = (LUTN - 1) / 12.0 * 0.30102999566398119521;  // cells an octave
@@ -500,8 +506,7 @@ __device__ __forceinline__ float lut_sample(const float2* lut, float phi) {
     if (phi > 1.0e9f) return lut[LUTN - 1].x;
     const uint32_t b = __float_as_uint(phi);
     const float k = (float)((int)(b >> 23) - 127);
-    float lm;
-    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(lm) : "f"(__uint_as_float((b & 0x007FFFFFu) | 0x3F800000u)));
+    const float lm = log2f(__uint_as_float((b & 0x007FFFFFu) | 0x3F800000u));
     const float frac = fmaf(lm, (float)SCALE, k * LO);
     const float pos = fminf(fmaxf(fmaf(k, HI, ZERO) + frac, 0.0f), (float)(LUTN - 1));
     const int i = min((int)pos, LUTN - 2);
@@ -533,7 +538,7 @@ __device__ __forceinline__ float pow_unit(float f, float g) {
 // Image-dye densities over the fluences in place, and the mask densities
 // (SUM: `mask` is one plane, their sum in layer order; otherwise E planes);
 // BOUNCE: the support bounce `deep` is added to the fluences first.  Bound by
-// the issue of the interpolation and the power of each layer and pixel.  24 MP, six layers, with the bounce: 0.44 ms against 1.86
+// the issue of the interpolation and the power of each layer and pixel.  24 MP, six layers, with the bounce: 0.55 ms against 1.86
 // (reduction and bounce epilogue apart, a binary search and powf a value).
 template <int E, bool SUM, bool BOUNCE>
 __global__ void __launch_bounds__(256) lut_reduce_kernel(float* __restrict__ planes, float* __restrict__ mask,
@@ -862,20 +867,26 @@ int grain_fields(float* noise, int W, int H, uint64_t seed, int layer0, int laye
     return IMOPS_OK;
 }
 
+// 1 / the RMS of a grain field from its sum of squares
+__device__ __forceinline__ float grain_norm(double sumsq, size_t n) {
+    const double var = sumsq / (double)n;
+    return var > 1e-12 ? (float)(1.0 / sqrt(var)) : 1.0f;
+}
+
 // D <- clamp(D + kappa*taper*sqrt(D(Dmax-D))*n*norm, 0, 1.05 Dmax)
+__device__ __forceinline__ float grain_px(float d, float noise, float norm, float kappa, float dmax) {
+    const float dens = fminf(fmaxf(d, 0.0f), dmax);
+    const float taper = fminf(__fdiv_rn(dens, fmaf(0.02f, dmax, dens)), 1.0f);
+    const float sd = __fmul_rn(taper, sqrtf(fmaxf(__fmul_rn(dens, __fsub_rn(dmax, dens)), 0.0f)));
+    d = fmaf(__fmul_rn(__fmul_rn(kappa, sd), noise), norm, dens);
+    return fminf(fmaxf(d, 0.0f), __fmul_rn(dmax, 1.05f));
+}
+
 __global__ void grain_apply_kernel(float* __restrict__ plane, const float* __restrict__ noise, size_t n,
                                    const double* __restrict__ sumsq, float kappa, float dmax) {
-    double var = *sumsq / (double)n;
-    float norm = var > 1e-12 ? (float)(1.0 / sqrt(var)) : 1.0f;
-    for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < n; p += (size_t)gridDim.x * blockDim.x) {
-        float d = plane[p];
-        float dens = fminf(fmaxf(d, 0.0f), dmax);
-        float toe = 0.02f * dmax;
-        float taper = fminf(dens / (dens + toe), 1.0f);
-        float sd = taper * sqrtf(fmaxf(dens * (dmax - dens), 0.0f));
-        d = dens + kappa * sd * noise[p] * norm;
-        plane[p] = fminf(fmaxf(d, 0.0f), dmax * 1.05f);
-    }
+    const float norm = grain_norm(*sumsq, n);
+    for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < n; p += (size_t)gridDim.x * blockDim.x)
+        plane[p] = grain_px(plane[p], noise[p], norm, kappa, dmax);
 }
 
 // ---------------------------------------------------------------------------
@@ -964,31 +975,203 @@ int with_layers(int E, F f) {
     return fail(IMOPS_ERR_INVALID_STOCK, "film: stocks have 1, 2, 3, 6 or 7 emulsion layers");
 }
 
-// invert_negative (invert.rs:36-108); mid/dmin read from device memory.
-__global__ void invert_kernel(float* __restrict__ rgb, size_t n, const float* __restrict__ mid_dmin) {
-    const float eps = 1e-6f, HEAD = 8.0f, KEEP = 0.55f, FADE = 0.02f, MG = 0.185f;
-    const float LR = 0.2722287168f, LG = 0.6740817658f, LB = 0.0536895174f;
+// invert_negative (invert.rs:36-108): the per-channel constants from the
+// mid-grey negative and Dmin (mid_dmin, device memory), and one pixel.
+struct Invert {
     float dmin[3], sh[3], g[3];
+};
+__device__ __forceinline__ float invert_curve(float inv, float sh) { return __fdiv_rn(inv, 1.0f + __fdiv_rn(inv, sh)); }
+__device__ __forceinline__ Invert invert_constants(const float* __restrict__ mid_dmin) {
+    const float eps = 1e-6f, HEAD = 8.0f, MG = 0.185f;
+    Invert v;
+#pragma unroll
     for (int c = 0; c < 3; c++) {
-        dmin[c] = fmaxf(mid_dmin[3 + c], eps);
-        float mt = fminf(fmaxf(mid_dmin[c] / dmin[c], eps), 1.0f - eps);
-        float im = fmaxf(1.0f / mt - 1.0f, 0.0f);
-        sh[c] = fmaxf(im * HEAD, eps);
-        float i2 = fmaxf(im, 0.0f), s2 = fmaxf(sh[c], 1e-6f);
-        float sm = fmaxf(i2 / (1.0f + i2 / s2), eps);
-        g[c] = MG / sm;
+        v.dmin[c] = fmaxf(mid_dmin[3 + c], eps);
+        const float mt = fminf(fmaxf(__fdiv_rn(mid_dmin[c], v.dmin[c]), eps), 1.0f - eps);
+        const float im = fmaxf(__fsub_rn(__fdiv_rn(1.0f, mt), 1.0f), 0.0f);
+        v.sh[c] = fmaxf(__fmul_rn(im, HEAD), eps);
+        v.g[c] = __fdiv_rn(MG, fmaxf(invert_curve(im, v.sh[c]), eps));
     }
+    return v;
+}
+__device__ __forceinline__ void invert_px(const Invert& v, float (&o)[3]) {
+    const float eps = 1e-6f, KEEP = 0.55f, FADE = 0.02f;
+    float raw[3];
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+        const float t = fminf(fmaxf(__fdiv_rn(o[c], v.dmin[c]), eps), 1.0f);
+        const float inv = fmaxf(__fsub_rn(__fdiv_rn(1.0f, t), 1.0f), 0.0f);
+        raw[c] = fmaxf(__fmul_rn(v.g[c], invert_curve(inv, v.sh[c])), 0.0f);
+    }
+    const float y = fmaxf(dot3(0.2722287168f, raw[0], 0.6740817658f, raw[1], 0.0536895174f, raw[2]), 0.0f);
+    const float k = y <= 0.0f ? 0.0f : (y >= FADE ? KEEP : __fmul_rn(KEEP, __fdiv_rn(y, FADE)));
+#pragma unroll
+    for (int c = 0; c < 3; c++) o[c] = fmaxf(fmaf(k, __fsub_rn(raw[c], y), y), 0.0f);
+}
+
+__global__ void invert_kernel(float* __restrict__ rgb, size_t n, const float* __restrict__ mid_dmin) {
+    const Invert v = invert_constants(mid_dmin);
     for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < n; p += (size_t)gridDim.x * blockDim.x) {
-        float raw[3];
-        for (int c = 0; c < 3; c++) {
-            float t = fminf(fmaxf(rgb[3 * p + c] / dmin[c], eps), 1.0f);
-            float inv = fmaxf(1.0f / t - 1.0f, 0.0f);
-            float i2 = fmaxf(inv, 0.0f), s2 = fmaxf(sh[c], 1e-6f);
-            raw[c] = fmaxf(g[c] * (i2 / (1.0f + i2 / s2)), 0.0f);
+        float o[3] = {rgb[3 * p], rgb[3 * p + 1], rgb[3 * p + 2]};
+        invert_px(v, o);
+        for (int c = 0; c < 3; c++) rgb[3 * p + c] = o[c];
+    }
+}
+
+// ---- adjacency, grain, scan and inversion in one pass ------------------------
+// The last four steps of the model on a 64 x 32 tile: each layer's tile comes
+// in with cp.async while the layer before is blurred (adjacency), its grain
+// is added, and its densities stay in shared memory (a thread's own four
+// pixels); when all layers are through, the thread scans its pixels and
+// inverts them.  RC: the blur radius class (taps beyond the radius are zero:
+// densities are finite, so they add nothing), 0 where the densities are
+// final.  Same arithmetic as the steps one by one.  24 MP, six layers, grain:
+// 0.71 ms against 2.1 (12 blur launches, 6 of the grain, the scan).
+constexpr int PR_THREADS = 512, PR_ROWS = ft_rpt(PR_THREADS);
+template <int E>
+struct Print {
+    Scan16<E> scan;
+    float kappa[E], dmax[E];
+    float beta;
+    float taps[2 * 8 + 1];  // centred in the radius class
+};
+template <int RC>
+constexpr int print_smem_floats(int E) {
+    return (RC ? 2 * ft_tile_floats(RC) + ft_row_floats(RC) : 0) + E * FT_W * FT_H;
+}
+
+template <int E, int RC>
+__global__ void __launch_bounds__(PR_THREADS, 2) print_kernel(const float* __restrict__ dens,
+                                                              const float* __restrict__ mask,
+                                                              const float* __restrict__ noise,
+                                                              const double* __restrict__ sums,
+                                                              const float* __restrict__ mid_dmin, int W, int H,
+                                                              const __grid_constant__ Print<E> c,
+                                                              float* __restrict__ rgb) {
+    extern __shared__ __align__(16) float ftsm[];
+    __shared__ float norm[E];
+    __shared__ Invert inv;
+    constexpr int TILE = RC ? ft_tile_floats(RC) : 0;
+    float* rows = ftsm + 2 * TILE;
+    const int x0 = blockIdx.x * FT_W, y0 = blockIdx.y * FT_H;
+    const int tx = threadIdx.x % FT_W, rb = (int)threadIdx.x / FT_W * PR_ROWS;
+    float* own = ftsm + (RC ? 2 * TILE + ft_row_floats(RC) : 0) + threadIdx.x;  // [layer][row][thread]
+    const size_t n = (size_t)W * H;
+    const int x = x0 + tx;
+    // this thread's pixels, clamped into the image (their results are not stored)
+    size_t px[PR_ROWS];
+#pragma unroll
+    for (int r = 0; r < PR_ROWS; r++) px[r] = (size_t)min(y0 + rb + r, H - 1) * W + min(x, W - 1);
+    if (noise && threadIdx.x < E) norm[threadIdx.x] = grain_norm(sums[threadIdx.x], n);
+    if (mid_dmin && threadIdx.x == 32) inv = invert_constants(mid_dmin);
+    FtCopy copy;
+    if constexpr (RC > 0) {
+        copy = ft_copy(dens, x0, y0, RC, W, H);
+        ft_load<PR_THREADS>(ftsm, dens, copy, y0, RC, W, H);
+        ft_commit();
+    } else {
+        __syncthreads();  // norm, inv
+    }
+#pragma unroll 1
+    for (int e = 0; e < E; e++) {
+        float nz[PR_ROWS], d[PR_ROWS];
+#pragma unroll
+        for (int r = 0; r < PR_ROWS; r++) nz[r] = noise ? __ldg(noise + e * n + px[r]) : 0.0f;
+        if constexpr (RC > 0) {
+            ft_wait<0>();
+            __syncthreads();  // this layer's tile is complete; the row buffer and the other tile are free
+            if (e + 1 < E) {
+                ft_load<PR_THREADS>(ftsm + ((e + 1) & 1) * TILE, dens + (e + 1) * n, copy, y0, RC, W, H);
+                ft_commit();
+            }
+            const float* tile = ftsm + (e & 1) * TILE;
+            float v[PR_ROWS];
+            ft_rows<PR_THREADS, RC>(tile, rows, c.taps);
+            __syncthreads();
+            ft_cols<RC>(rows, tx, rb, c.taps, v);
+#pragma unroll
+            for (int r = 0; r < PR_ROWS; r++)
+                d[r] = adjacency_px(tile[(RC + rb + r) * ft_stride(RC) + ft_pad(RC) + RC + tx], v[r], c.beta);
+        } else {
+#pragma unroll
+            for (int r = 0; r < PR_ROWS; r++) d[r] = __ldg(dens + e * n + px[r]);
         }
-        float y = fmaxf(LR * raw[0] + LG * raw[1] + LB * raw[2], 0.0f);
-        float k = y <= 0.0f ? 0.0f : (y >= FADE ? KEEP : KEEP * (y / FADE));
-        for (int c = 0; c < 3; c++) rgb[3 * p + c] = fmaxf(y + k * (raw[c] - y), 0.0f);
+        if (noise && c.kappa[e] > 0.0f && c.dmax[e] > 0.0f) {
+#pragma unroll
+            for (int r = 0; r < PR_ROWS; r++) d[r] = grain_px(d[r], nz[r], norm[e], c.kappa[e], c.dmax[e]);
+        }
+#pragma unroll
+        for (int r = 0; r < PR_ROWS; r++) own[(e * PR_ROWS + r) * PR_THREADS] = d[r];
+    }
+    if (x >= W) return;
+#pragma unroll 1
+    for (int r = 0; r < PR_ROWS; r++) {
+        if (y0 + rb + r >= H) break;
+        const size_t p = (size_t)(y0 + rb + r) * W + x;
+        float D[E], o[3];
+#pragma unroll
+        for (int e = 0; e < E; e++) D[e] = own[(e * PR_ROWS + r) * PR_THREADS];
+        scan16_px<E>(c.scan, D, __ldg(mask + p), o);
+        if (mid_dmin) invert_px(inv, o);
+        rgb[3 * p] = o[0];
+        rgb[3 * p + 1] = o[1];
+        rgb[3 * p + 2] = o[2];
+    }
+}
+
+// Exposure of the layers and their local scatter on a 64 x 32 tile: the basis
+// weights of the tile and its halo once, then each layer formed from them,
+// blurred and mixed, so the layers reach memory once, scattered.  24 MP, six
+// layers, radius 2: 0.56 ms against 1.5 (an exposure pass and 12 blur launches).
+constexpr int EX_THREADS = 512, EX_ROWS = ft_rpt(EX_THREADS), EX_MAXR = 8;
+__host__ __device__ constexpr int expose_smem_floats(int R) { return 5 * ft_tile_floats(R) + ft_row_floats(R); }
+
+__global__ void __launch_bounds__(EX_THREADS, 2) expose_scatter_kernel(const float* __restrict__ rgb, int W, int H,
+                                                                       const __grid_constant__ ExposeSpec X,
+                                                                       const __grid_constant__ Taps tp, float keep,
+                                                                       float mix, float* __restrict__ planes) {
+    extern __shared__ __align__(16) float ftsm[];
+    const int R = tp.R, tile = ft_tile_floats(R), SW = ft_stride(R), NH = FT_H + 2 * R;
+    float* rows = ftsm + 5 * tile;
+    const int x0 = blockIdx.x * FT_W, y0 = blockIdx.y * FT_H;
+    const int tx = threadIdx.x % FT_W, rb = (int)threadIdx.x / FT_W * EX_ROWS, lane = threadIdx.x & 31;
+    const size_t n = (size_t)W * H;
+    int xs[FT_COLS];
+#pragma unroll
+    for (int t = 0; t < FT_COLS; t++) xs[t] = 3 * reflect(x0 - R - ft_pad(R) + lane + 32 * t, W);
+    for (int r = (int)threadIdx.x >> 5; r < NH; r += EX_THREADS / 32) {
+        const float* src = rgb + (size_t)reflect(y0 - R + r, H) * W * 3;
+#pragma unroll
+        for (int t = 0; t < FT_COLS; t++) {
+            const int q = 32 * t + lane;
+            if (q < SW) {
+                const float* s = src + xs[t];
+                float w[3];
+                basis_weights(X, __ldg(s), __ldg(s + 1), __ldg(s + 2), w);
+#pragma unroll
+                for (int k = 0; k < 3; k++) ftsm[(2 + k) * tile + r * SW + q] = w[k];
+            }
+        }
+    }
+    __syncthreads();
+    const int x = x0 + tx;
+#pragma unroll 1
+    for (int e = 0; e < X.E; e++) {
+        float* s = ftsm + (e & 1) * tile;  // free: its readers passed the barrier in the layer between
+        for (int i = threadIdx.x; i < tile; i += EX_THREADS) {
+            const float w[3] = {ftsm[2 * tile + i], ftsm[3 * tile + i], ftsm[4 * tile + i]};
+            s[i] = layer_exposure(X, w, e);
+        }
+        __syncthreads();
+        float v[EX_ROWS];
+        ft_blur<EX_THREADS, EX_MAXR>(s, rows, tx, rb, tp, v);
+#pragma unroll
+        for (int r = 0; r < EX_ROWS; r++) {
+            const int y = y0 + rb + r;
+            if (x < W && y < H)
+                planes[e * n + (size_t)y * W + x] =
+                    mix_px(s[(R + rb + r) * SW + ft_pad(R) + R + tx], v[r], keep, mix);
+        }
     }
 }
 
@@ -1602,29 +1785,51 @@ int stage_expose(const float* rgb, int W, int H, const Stock& st, float* planes,
     return IMOPS_OK;
 }
 
-//   halation: local scatter in place, and the wide bounce of the deepest
-//     layer (halation.rs:24-93): its blur in *deep (NULL when the stock has
-//     none), added to the layers by bounce_kernel or by the reduction; tmp,
-//     bounce: one plane each
-int stage_halation(float* planes, int W, int H, const Stock& st, float* tmp, float* bounce, float** deep,
-                   cudaStream_t s) {
-    const RefSpec& R = st.ref;
-    const int E = R.E;
+//   halation: local scatter in place (halation.rs:24-78); tmp: one plane
+int stage_scatter(float* planes, int W, int H, const RefSpec& R, float* tmp, cudaStream_t s) {
+    if (!(R.sigma_local >= 1e-3f && R.local_mix > 0.0f)) return IMOPS_OK;
     const size_t n = (size_t)W * H;
     Taps tp;
     int rc;
+    if ((rc = taps_for(R.sigma_local, &tp))) return rc;
+    for (int e = 0; e < R.E; e++)
+        if ((rc = blur(planes + e * n, tmp, W, H, tp, EpiMix{planes + e * n, 1.0f - R.local_mix, R.local_mix}, s)))
+            return rc;
+    return IMOPS_OK;
+}
+
+//   expose and scatter in one pass
+int expose_scatter(const float* rgb, int W, int H, const Stock& st, float* planes, float* tmp, cudaStream_t s) {
+    const RefSpec& R = st.ref;
+    Taps tp;
+    int rc;
+    const bool local = R.sigma_local >= 1e-3f && R.local_mix > 0.0f;
+    if (local && (rc = taps_for(R.sigma_local, &tp))) return rc;
+    if (!local || tp.R > EX_MAXR) {
+        if ((rc = stage_expose(rgb, W, H, st, planes, s))) return rc;
+        return stage_scatter(planes, W, H, R, tmp, s);
+    }
+    const size_t smem = (size_t)expose_smem_floats(tp.R) * sizeof(float);
+    IMOPS_CUDA_TRY(cudaFuncSetAttribute(expose_scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+                   "cudaFuncSetAttribute(exposure)");
+    const dim3 g((W + FT_W - 1) / FT_W, (H + FT_H - 1) / FT_H);
+    expose_scatter_kernel<<<g, EX_THREADS, smem, s>>>(rgb, W, H, st.expose, tp, 1.0f - R.local_mix, R.local_mix, planes);
+    note_launch();
+    return IMOPS_OK;
+}
+
+//   the wide bounce of the deepest layer (halation.rs:80-93): its blur in
+//     *deep (NULL when the stock has none), added to the layers by
+//     bounce_kernel or by the reduction; tmp, bounce: one plane each
+int stage_bounce(const float* planes, int W, int H, const RefSpec& R, float* tmp, float* bounce, float** deep,
+                 cudaStream_t s) {
     *deep = nullptr;
-    if (R.sigma_local >= 1e-3f && R.local_mix > 0.0f) {
-        if ((rc = taps_for(R.sigma_local, &tp))) return rc;
-        for (int e = 0; e < E; e++)
-            if ((rc = blur(planes + e * n, tmp, W, H, tp, EpiMix{planes + e * n, 1.0f - R.local_mix, R.local_mix}, s)))
-                return rc;
-    }
-    if (R.sigma_wide >= 1e-3f) {
-        if ((rc = taps_for(R.sigma_wide, &tp))) return rc;
-        if ((rc = blur(planes + (E - 1) * n, tmp, W, H, tp, EpiStore{bounce}, s))) return rc;
-        *deep = bounce;
-    }
+    if (!(R.sigma_wide >= 1e-3f)) return IMOPS_OK;
+    Taps tp;
+    int rc;
+    if ((rc = taps_for(R.sigma_wide, &tp))) return rc;
+    if ((rc = blur(planes + (size_t)(R.E - 1) * W * H, tmp, W, H, tp, EpiStore{bounce}, s))) return rc;
+    *deep = bounce;
     return IMOPS_OK;
 }
 
@@ -1667,18 +1872,32 @@ int launch_dir(const float* in, float* out, int W, int H, const Taps& tp, const 
         IMOPS_CUDA_TRY(cudaFuncSetAttribute(dir_kernel<E>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                        "cudaFuncSetAttribute(DIR)");
         const dim3 g((W + FT_W - 1) / FT_W, (H + FT_H - 1) / FT_H);
-        dir_kernel<E><<<g, FT_THREADS, smem, s>>>(in, out, W, H, tp, mix);
+        dir_kernel<E><<<g, DIR_THREADS, smem, s>>>(in, out, W, H, tp, mix);
         note_launch();
         return IMOPS_OK;
     });
+}
+
+static bool has_adjacency(const RefSpec& R) { return !(fabsf(R.beta) < 1e-8f || R.sigma_adj < 1e-3f); }
+
+int stage_adjacency(float* planes, int W, int H, const RefSpec& R, float* tmp, cudaStream_t s) {
+    if (!has_adjacency(R)) return IMOPS_OK;
+    const size_t n = (size_t)W * H;
+    Taps tp;
+    int rc;
+    if ((rc = taps_for(R.sigma_adj, &tp))) return rc;
+    for (int e = 0; e < R.E; e++)
+        if ((rc = blur(planes + e * n, tmp, W, H, tp, EpiAdjacency{planes + e * n, R.beta}, s))) return rc;
+    return IMOPS_OK;
 }
 
 //   develop: capture LUT + reciprocity + reduction to image-dye and mask
 //     densities, DIR inhibition, adjacency (capture.rs:61-88,
 //     reduction.rs:16-68, diffusion.rs:11-84); inh: E planes, tmp: one.
 //     sum: `mask` is the one plane of the layers' mask sum, and the bounce
-//     `deep` (or NULL) is added first.  The densities end up in *result
-//     (planes or inh), or in planes when result is NULL.
+//     `deep` (or NULL) is added first.  With result NULL the densities end
+//     up in planes; otherwise in *result (planes or inh), without the
+//     adjacency, which print_scan adds.
 int stage_develop(float* planes, float* mask, bool sum, const float* deep, int W, int H, const Stock& st, const RefSpec* dR, float* inh,
                   float* tmp, float** result, cudaStream_t s) {
     const RefSpec& R = st.ref;
@@ -1710,25 +1929,26 @@ int stage_develop(float* planes, float* mask, bool sum, const float* deep, int W
             note_launch();
         }
     }
-    if (!(fabsf(R.beta) < 1e-8f || R.sigma_adj < 1e-3f)) {
-        if ((rc = taps_for(R.sigma_adj, &tp))) return rc;
-        for (int e = 0; e < E; e++)
-            if ((rc = blur(planes + e * n, tmp, W, H, tp, EpiAdjacency{planes + e * n, R.beta}, s))) return rc;
-    }
-    return IMOPS_OK;
+    return result ? IMOPS_OK : stage_adjacency(planes, W, H, R, tmp, s);
 }
 
 //   grain: seeded SplitMix64 fields, normalised and scaled per layer
 //     (grain.rs:53-100); noise: E planes, partial: grain_partials(W, H, E)
 //     doubles, sums: MAXE doubles
+int stage_grain_fields(int W, int H, const RefSpec& R, uint64_t seed, float* noise, double* partial, double* sums,
+                       cudaStream_t s) {
+    Taps tp;
+    int rc;
+    if ((rc = taps_for(fmaxf(R.sigma_grain, 1.0f), &tp))) return rc;
+    return grain_fields(noise, W, H, seed, 0, R.E, tp, partial, sums, s);
+}
+
 int stage_grain(float* planes, int W, int H, const Stock& st, uint64_t seed, float* noise, double* partial,
                 double* sums, cudaStream_t s) {
     const RefSpec& R = st.ref;
     const size_t n = (size_t)W * H;
-    Taps tp;
     int rc;
-    if ((rc = taps_for(fmaxf(R.sigma_grain, 1.0f), &tp))) return rc;
-    if ((rc = grain_fields(noise, W, H, seed, 0, R.E, tp, partial, sums, s))) return rc;
+    if ((rc = stage_grain_fields(W, H, R, seed, noise, partial, sums, s))) return rc;
     for (int e = 0; e < R.E; e++) {
         if (R.kappa[e] <= 0.0f || R.dmax[e] <= 0.0f) continue;
         grain_apply_kernel<<<grid_for(n), 256, 0, s>>>(planes + e * n, noise + e * n, n, sums + e, R.kappa[e],
@@ -1752,10 +1972,57 @@ int stage_scan(const float* planes, const float* mask, bool sum, int W, int H, c
     });
 }
 
-// expose -> halation -> develop -> grain -> scan for the reference model;
-// rgb in, rgb out.
-int run_reference(float* rgb, int W, int H, const Stock& st, uint64_t seed, int grain, Arena& A, const RefSpec* dR,
-                  cudaStream_t s) {
+template <int E, int RC>
+int launch_print(const float* dens, const float* mask, const float* noise, const double* sums, const float* mid_dmin,
+                 int W, int H, const Print<E>& c, float* rgb, cudaStream_t s) {
+    const size_t smem = (size_t)print_smem_floats<RC>(E) * sizeof(float);
+    IMOPS_CUDA_TRY(cudaFuncSetAttribute(print_kernel<E, RC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+                   "cudaFuncSetAttribute(print)");
+    const dim3 g((W + FT_W - 1) / FT_W, (H + FT_H - 1) / FT_H);
+    print_kernel<E, RC><<<g, PR_THREADS, smem, s>>>(dens, mask, noise, sums, mid_dmin, W, H, c, rgb);
+    note_launch();
+    return IMOPS_OK;
+}
+
+// Adjacency, grain (noise not NULL), scan and inversion (mid_dmin not NULL)
+// of the densities in one pass.  The radius classes are the stocks' at 35 mm
+// up to about 25 and 50 MP; wider blurs (only where the bounce is refused)
+// run as launches of their own.
+int print_scan(float* dens, const float* mask, const float* noise, const double* sums, const float* mid_dmin, int W,
+               int H, const Stock& st, float* tmp, float* rgb, cudaStream_t s) {
+    const RefSpec& R = st.ref;
+    Taps tp;
+    tp.R = 0;
+    int rc;
+    if (has_adjacency(R) && (rc = taps_for(R.sigma_adj, &tp))) return rc;
+    if (tp.R > 8) {
+        if ((rc = stage_adjacency(dens, W, H, R, tmp, s))) return rc;
+        tp.R = 0;
+    }
+    return with_layers(R.E, [&](auto e) {
+        constexpr int E = decltype(e)::value;
+        Print<E> c;
+        c.scan = scan16_pairs<E>(st.scan16);
+        for (int i = 0; i < E; i++) {
+            c.kappa[i] = R.kappa[i];
+            c.dmax[i] = R.dmax[i];
+        }
+        c.beta = R.beta;
+        const int RC = tp.R == 0 ? 0 : (tp.R <= 4 ? 4 : 8);
+        for (int k = 0; k < 2 * 8 + 1; k++) {
+            const int j = k - RC + tp.R;
+            c.taps[k] = tp.R > 0 && j >= 0 && j <= 2 * tp.R ? tp.t[j] : 0.0f;
+        }
+        if (RC == 0) return launch_print<E, 0>(dens, mask, noise, sums, mid_dmin, W, H, c, rgb, s);
+        if (RC == 4) return launch_print<E, 4>(dens, mask, noise, sums, mid_dmin, W, H, c, rgb, s);
+        return launch_print<E, 8>(dens, mask, noise, sums, mid_dmin, W, H, c, rgb, s);
+    });
+}
+
+// The reference model's kernels on rgb in place, inverted with the reference
+// points mid_dmin unless that is NULL.
+int run_reference(float* rgb, int W, int H, const Stock& st, uint64_t seed, int grain, const float* mid_dmin, Arena& A,
+                  const RefSpec* dR, cudaStream_t s) {
     const int E = st.ref.E;
     const size_t n = (size_t)W * H;
     float* planes = A.take<float>(E * n);
@@ -1766,15 +2033,14 @@ int run_reference(float* rgb, int W, int H, const Stock& st, uint64_t seed, int 
     double* partial = A.take<double>(grain_partials(W, H, E));
     double* sums = A.take<double>(MAXE);
     int rc;
-    if ((rc = stage_expose(rgb, W, H, st, planes, s))) return rc;
-    float* deep = nullptr;
-    if ((rc = stage_halation(planes, W, H, st, tmp, bounce, &deep, s))) return rc;
-    float* dens = nullptr;
+    float *deep = nullptr, *dens = nullptr;
+    if ((rc = expose_scatter(rgb, W, H, st, planes, tmp, s))) return rc;
+    if ((rc = stage_bounce(planes, W, H, st.ref, tmp, bounce, &deep, s))) return rc;
     if ((rc = stage_develop(planes, mask, true, deep, W, H, st, dR, inh, tmp, &dens, s))) return rc;
     // the other set of planes is free after develop: it takes the grain fields
-    float* spare = dens == planes ? inh : planes;
-    if (grain && (rc = stage_grain(dens, W, H, st, seed, spare, partial, sums, s))) return rc;
-    if ((rc = stage_scan(dens, mask, true, W, H, st.scan16, rgb, s))) return rc;
+    float* noise = grain ? (dens == planes ? inh : planes) : nullptr;
+    if (grain && (rc = stage_grain_fields(W, H, st.ref, seed, noise, partial, sums, s))) return rc;
+    if ((rc = print_scan(dens, mask, noise, sums, mid_dmin, W, H, st, tmp, rgb, s))) return rc;
     IMOPS_CUDA_TRY(cudaGetLastError(), "film kernels");
     return IMOPS_OK;
 }
@@ -1790,7 +2056,7 @@ int mid_gray_negative(const Stock& st, int grain, Arena& A, const RefSpec* dR, f
     float* dpatch = A.take<float>(nm * 3);
     IMOPS_CUDA_TRY(cudaMemcpyAsync(dpatch, patch.data(), nm * 12, cudaMemcpyHostToDevice, s), "copy patch");
     int rc;
-    if ((rc = run_reference(dpatch, 32, 32, st, 0, grain, A, dR, s))) return rc;
+    if ((rc = run_reference(dpatch, 32, 32, st, 0, grain, nullptr, A, dR, s))) return rc;
     mean_rgb_kernel<<<1, 256, 0, s>>>(dpatch, (int)nm, mid_dmin);
     note_launch();
     IMOPS_CUDA_TRY(cudaMemcpyAsync(mid_dmin + 3, st.ref.dmin_norm, 12, cudaMemcpyHostToDevice, s), "copy dmin");
@@ -1813,13 +2079,7 @@ int process_reference(float* rgb, int W, int H, const ImopsFilmParams& P, cudaSt
     IMOPS_CUDA_TRY(cudaMemcpyAsync(dR, &st.ref, sizeof(RefSpec), cudaMemcpyHostToDevice, s), "copy spec");
     bool positive = P.output == IMOPS_FILM_POSITIVE_LINEAR && !st.ref.any_reversal;
     if (positive && (rc = mid_gray_negative(st, P.grain, A, dR, mid_dmin, s))) return rc;
-    if ((rc = run_reference(rgb, W, H, st, P.seed, P.grain, A, dR, s))) return rc;
-    if (positive) {
-        invert_kernel<<<grid_for(n), 256, 0, s>>>(rgb, n, mid_dmin);
-        note_launch();
-    }
-    IMOPS_CUDA_TRY(cudaGetLastError(), "film invert");
-    return IMOPS_OK;
+    return run_reference(rgb, W, H, st, P.seed, P.grain, positive ? mid_dmin : nullptr, A, dR, s);
 }
 
 // One sub-stage call: the stock (reference model only), device copies of its
@@ -2018,7 +2278,8 @@ extern "C" int imops_film_halation(float* planes, int w, int h, const ImopsFilmP
     float* tmp = c.A.take<float>(n);
     float* bounce = c.A.take<float>(n);
     float* deep = nullptr;
-    if ((rc = film::stage_halation(planes, w, h, c.st, tmp, bounce, &deep, s))) return rc;
+    if ((rc = film::stage_scatter(planes, w, h, c.st.ref, tmp, s))) return rc;
+    if ((rc = film::stage_bounce(planes, w, h, c.st.ref, tmp, bounce, &deep, s))) return rc;
     if (deep) {
         film::bounce_kernel<<<film::grid_for(n), 256, 0, s>>>(planes, deep, n, c.st.ref.E, film::bounce_gains(c.st.ref));
         note_launch();

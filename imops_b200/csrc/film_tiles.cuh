@@ -17,9 +17,9 @@
 namespace imops {
 namespace film {
 
-constexpr int FT_W = 64, FT_H = 32, FT_THREADS = 256, FT_ROWS = 8;
-constexpr int FT_MAXR = 16;
-static_assert(FT_THREADS / FT_W * FT_ROWS == FT_H, "a thread's rows cover the tile");
+constexpr int FT_W = 64, FT_H = 32, FT_MAXR = 16;
+// rows a thread of a block of T threads
+constexpr int ft_rpt(int T) { return FT_W * FT_H / T; }
 
 // A staged row starts ft_pad(R) samples left of the halo, at a column that is
 // a multiple of 4 (x0 is), and its stride is a multiple of 4: the copies and
@@ -68,6 +68,7 @@ __device__ __forceinline__ FtCopy ft_copy(const float* plane, int x0, int y0, in
 }
 
 // Starts the copy of one plane's tile and halo.
+template <int T>
 __device__ __forceinline__ void ft_load(float* s, const float* __restrict__ plane, const FtCopy& c, int y0, int R,
                                         int W, int H) {
     const int SW = ft_stride(R), NH = FT_H + 2 * R, lane = threadIdx.x & 31, warp = (int)threadIdx.x >> 5;
@@ -75,15 +76,15 @@ __device__ __forceinline__ void ft_load(float* s, const float* __restrict__ plan
         if (4 * lane < SW) {
             const float* src = plane + (size_t)(y0 - R + warp) * W + c.x[0];
             float* dst = s + warp * SW + 4 * lane;
-            for (int r = warp; r < NH; r += FT_THREADS / 32) {
+            for (int r = warp; r < NH; r += T / 32) {
                 ft_cp16(dst, src);
-                src += (size_t)(FT_THREADS / 32) * W;
-                dst += FT_THREADS / 32 * SW;
+                src += (size_t)(T / 32) * W;
+                dst += T / 32 * SW;
             }
         }
         return;
     }
-    for (int r = warp; r < NH; r += FT_THREADS / 32) {
+    for (int r = warp; r < NH; r += T / 32) {
         const float* src = plane + (size_t)reflect(y0 - R + r, H) * W;
         float* dst = s + r * SW + lane;
 #pragma unroll
@@ -93,10 +94,10 @@ __device__ __forceinline__ void ft_load(float* s, const float* __restrict__ plan
 }
 
 // Row pass over the tile and its row halo: s (stride ft_stride(R)) -> rows (stride FT_W).
-template <int R>
-__device__ __forceinline__ void ft_rows(const float* s, float* rows, const Taps& tp) {
+template <int T, int R>
+__device__ __forceinline__ void ft_rows(const float* s, float* rows, const float* taps) {
     constexpr int SW = ft_stride(R), A = ft_pad(R), NH = FT_H + 2 * R, NQ = (A + 4 + 2 * R + 3) / 4;
-    for (int i = threadIdx.x; i < NH * (FT_W / 4); i += FT_THREADS) {
+    for (int i = threadIdx.x; i < NH * (FT_W / 4); i += T) {
         const int r = i / (FT_W / 4), g = i % (FT_W / 4);
         const float* p = s + r * SW + 4 * g;
         float a[4] = {0.0f, 0.0f, 0.0f, 0.0f};
@@ -109,40 +110,39 @@ __device__ __forceinline__ void ft_rows(const float* s, float* rows, const Taps&
 #pragma unroll
                 for (int j = 0; j < 4; j++) {
                     const int k = 4 * q + u - A - j;
-                    if (k >= 0 && k <= 2 * R) a[j] = fmaf(v[u], tp.t[k], a[j]);
+                    if (k >= 0 && k <= 2 * R) a[j] = fmaf(v[u], taps[k], a[j]);
                 }
         }
         *reinterpret_cast<float4*>(rows + r * FT_W + 4 * g) = make_float4(a[0], a[1], a[2], a[3]);
     }
 }
 
-// Column pass: the FT_ROWS outputs of this thread (column tx, rows rb ..).
-template <int R>
-__device__ __forceinline__ void ft_cols(const float* rows, int tx, int rb, const Taps& tp, float (&out)[FT_ROWS]) {
+// Column pass: the N outputs of this thread (column tx, rows rb ..).
+template <int R, int N>
+__device__ __forceinline__ void ft_cols(const float* rows, int tx, int rb, const float* taps, float (&out)[N]) {
 #pragma unroll
-    for (int j = 0; j < FT_ROWS; j++) out[j] = 0.0f;
+    for (int j = 0; j < N; j++) out[j] = 0.0f;
 #pragma unroll
-    for (int m = 0; m < FT_ROWS + 2 * R; m++) {
+    for (int m = 0; m < N + 2 * R; m++) {
         const float v = rows[(rb + m) * FT_W + tx];
 #pragma unroll
-        for (int j = 0; j < FT_ROWS; j++) {
+        for (int j = 0; j < N; j++) {
             const int k = m - j;
-            if (k >= 0 && k <= 2 * R) out[j] = fmaf(v, tp.t[k], out[j]);
+            if (k >= 0 && k <= 2 * R) out[j] = fmaf(v, taps[k], out[j]);
         }
     }
 }
 
 // Row pass, barrier, column pass with the radius as a template argument.
-template <int R = 1, int RMAX>
-__device__ __forceinline__ void ft_blur(std::integral_constant<int, RMAX>, const float* s, float* rows, int tx, int rb,
-                                        const Taps& tp, float (&out)[FT_ROWS]) {
+template <int T, int RMAX, int R = 1, int N>
+__device__ __forceinline__ void ft_blur(const float* s, float* rows, int tx, int rb, const Taps& tp, float (&out)[N]) {
     if constexpr (R <= RMAX) {
         if (tp.R == R) {
-            ft_rows<R>(s, rows, tp);
+            ft_rows<T, R>(s, rows, tp.t);
             __syncthreads();
-            ft_cols<R>(rows, tx, rb, tp, out);
+            ft_cols<R>(rows, tx, rb, tp.t, out);
         } else {
-            ft_blur<R + 1>(std::integral_constant<int, RMAX>{}, s, rows, tx, rb, tp, out);
+            ft_blur<T, RMAX, R + 1>(s, rows, tx, rb, tp, out);
         }
     }
 }
@@ -160,46 +160,48 @@ struct DirMix {
     float m[E][E];
 };
 
+constexpr int DIR_THREADS = 256, DIR_ROWS = ft_rpt(DIR_THREADS);
+
 template <int E>
-__global__ void __launch_bounds__(FT_THREADS, 2) dir_kernel(const float* __restrict__ in, float* __restrict__ out,
+__global__ void __launch_bounds__(DIR_THREADS, E <= 3 ? 3 : 2) dir_kernel(const float* __restrict__ in, float* __restrict__ out,
                                                             int W, int H, const __grid_constant__ Taps tp,
                                                             const __grid_constant__ DirMix<E> mix) {
     extern __shared__ __align__(16) float ftsm[];
     const int R = tp.R, tile = ft_tile_floats(R);
     float* rows = ftsm + 2 * tile;
     const int x0 = blockIdx.x * FT_W, y0 = blockIdx.y * FT_H;
-    const int tx = threadIdx.x % FT_W, rb = (int)threadIdx.x / FT_W * FT_ROWS;
+    const int tx = threadIdx.x % FT_W, rb = (int)threadIdx.x / FT_W * DIR_ROWS;
     const size_t n = (size_t)W * H;
-    float tot[E][FT_ROWS];
+    float tot[E][DIR_ROWS];
 #pragma unroll
     for (int j = 0; j < E; j++)
 #pragma unroll
-        for (int r = 0; r < FT_ROWS; r++) tot[j][r] = 0.0f;
+        for (int r = 0; r < DIR_ROWS; r++) tot[j][r] = 0.0f;
     const FtCopy cols = ft_copy(in, x0, y0, R, W, H);
-    ft_load(ftsm, in, cols, y0, R, W, H);
+    ft_load<DIR_THREADS>(ftsm, in, cols, y0, R, W, H);
     ft_commit();
 #pragma unroll 1
     for (int i = 0; i < E; i++) {
         ft_wait<0>();
         __syncthreads();  // this layer's tile is complete; the row buffer and the other tile are free
         if (i + 1 < E) {
-            ft_load(ftsm + ((i + 1) & 1) * tile, in + (i + 1) * n, cols, y0, R, W, H);
+            ft_load<DIR_THREADS>(ftsm + ((i + 1) & 1) * tile, in + (i + 1) * n, cols, y0, R, W, H);
             ft_commit();
         }
-        float v[FT_ROWS];
-        ft_blur(std::integral_constant<int, FT_MAXR>{}, ftsm + (i & 1) * tile, rows, tx, rb, tp, v);
+        float v[DIR_ROWS];
+        ft_blur<DIR_THREADS, FT_MAXR>(ftsm + (i & 1) * tile, rows, tx, rb, tp, v);
 #pragma unroll
         for (int j = 0; j < E; j++) {
             const float w = mix.m[i][j];
             if (w != 0.0f)
 #pragma unroll
-                for (int r = 0; r < FT_ROWS; r++) tot[j][r] = fmaf(w, v[r], tot[j][r]);
+                for (int r = 0; r < DIR_ROWS; r++) tot[j][r] = fmaf(w, v[r], tot[j][r]);
         }
     }
     const int x = x0 + tx;
     if (x >= W) return;
 #pragma unroll
-    for (int r = 0; r < FT_ROWS; r++) {
+    for (int r = 0; r < DIR_ROWS; r++) {
         const int y = y0 + rb + r;
         if (y >= H) break;
         const size_t p = (size_t)y * W + x;
