@@ -12,7 +12,7 @@
 // first, as the separate passes do.
 #pragma once
 
-#include "film.cuh"
+#include "blur.cuh"
 
 namespace imops {
 namespace film {
