@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(BLK) pixel_forward_kernel(const float* __restr
 // The scan takes 15 multiply-adds a bin, two bins a packed FMA, and 4.8 KB of
 // tables a pixel: warps that read them at different places evict one another's
 // constants, so one block of 20 warps an SM steps through the pixels together
-// (24 MP, the barrier kept: 1.20 ms; two blocks of 8 warps 1.30, four of 4
+// (24 MP, the barrier kept: 1.26 ms; two blocks of 8 warps 1.30, four of 4
 // 1.43).  Bound by the FMA pipe (0.97 ms with the curves).  One bin an FMA,
 // bound by issue: 1.42 ms.  18 multiply-adds from the six forward tables alone
 // (1.9 KB): 1.30 ms.

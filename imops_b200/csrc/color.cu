@@ -2,10 +2,7 @@
 // white balance, exposure, BaselineExposureCompensation and camera CST.
 //
 // All are HBM-bound streams over interleaved RGB (12 B in + 12 B out per
-// pixel, or 2 B in + 4 B out for the scaling); kernels use a grid-stride
-// loop sized to a few waves of the SM count and read/write the RGB triple
-// as three floats per thread (consecutive threads touch consecutive 12-byte
-// records, so each warp instruction is a contiguous 384-byte span).
+// pixel, see map_pixels, or 2 B in + 4 B out for the scaling).
 // Built with --fmad=false: each step is the reference's own f32 arithmetic.
 #include "color.cuh"
 
@@ -151,15 +148,10 @@ __global__ void scale_u16_kernel(const uint16_t* __restrict__ raw, int raw_w, in
     }
 }
 
-__global__ void epilogue_kernel(float* __restrict__ rgb, size_t n, Epilogue e) {
-    for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x) {
-        float* p = rgb + 3 * k;
-        float r = p[0], g = p[1], b = p[2];
-        e.apply(r, g, b);
-        p[0] = r;
-        p[1] = g;
-        p[2] = b;
-    }
+template <bool VEC>
+__global__ void __launch_bounds__(PIX_THREADS) epilogue_kernel(float* __restrict__ rgb, size_t n,
+                                                               const __grid_constant__ Epilogue e) {
+    map_pixels<VEC, 4>(rgb, n, [&](float& r, float& g, float& b) { e.apply(r, g, b); });
 }
 
 int stream_grid(size_t n, int block) {
@@ -174,7 +166,8 @@ int run_epilogue(float* rgb, size_t n, const Epilogue& e, cudaStream_t s, const 
     if (!rgb && n) return fail(IMOPS_ERR_INVALID_ARGUMENT, std::string(what) + ": NULL buffer");
     if (n == 0) return IMOPS_OK;
     if (fault_injected("launch")) return fail(IMOPS_ERR_CUDA, std::string("injected launch failure (") + what + ")");
-    epilogue_kernel<<<stream_grid(n, 256), 256, 0, s>>>(rgb, n, e);
+    if (aligned16(rgb)) epilogue_kernel<true><<<pixel_grid(n), PIX_THREADS, 0, s>>>(rgb, n, e);
+    else epilogue_kernel<false><<<pixel_grid(n), PIX_THREADS, 0, s>>>(rgb, n, e);
     note_launch();
     IMOPS_CUDA_TRY(cudaGetLastError(), what);
     return IMOPS_OK;

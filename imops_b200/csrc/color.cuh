@@ -92,5 +92,59 @@ int run_epilogue(float* rgb, size_t n, const Epilogue& e, cudaStream_t s, const 
 // Grid size for a grid-stride loop over n items.
 int stream_grid(size_t n, int block);
 
+// Per-pixel passes over interleaved RGB in place: a warp takes PIX_WARP
+// consecutive pixels through its part of shared memory, so that global memory
+// sees whole float4 rows of 512 bytes a warp instruction instead of 4-byte
+// accesses 12 bytes apart (whose stores reach the L2 as three partial writes
+// of every sector), and a lane's pixels lie 3 floats apart in shared memory (no
+// bank conflicts).  f(r, g, b) maps a pixel.  rgb must be 16-byte aligned (VEC)
+// or is accessed by 4 bytes.  Launch with pixel_grid(n) blocks of
+// PIX_THREADS.  24 MP exposure gain: 86 us against 115 (89 at the copy rate).
+constexpr int PIX_THREADS = 256, PIX_WARP = 128;
+constexpr int PIX_BLOCK = PIX_THREADS / 32 * PIX_WARP;
+
+inline int pixel_grid(size_t n) { return (int)((n + PIX_BLOCK - 1) / PIX_BLOCK); }
+
+template <bool VEC, int UNROLL, class F>
+__device__ __forceinline__ void map_pixels(float* __restrict__ rgb, size_t n, F f) {
+    __shared__ __align__(16) float stage[PIX_THREADS / 32][3 * PIX_WARP];
+    const int lane = threadIdx.x & 31;
+    float* s = stage[threadIdx.x >> 5];
+    const size_t p0 = blockIdx.x * (size_t)PIX_BLOCK + (threadIdx.x >> 5) * PIX_WARP;
+    if (p0 >= n) return;  // whole warp: only warp-level synchronisation below
+    float* g = rgb + 3 * p0;
+    const int px = n - p0 < PIX_WARP ? (int)(n - p0) : PIX_WARP;
+    const bool whole = VEC && px == PIX_WARP;
+    if (whole) {
+#pragma unroll
+        for (int q = 0; q < 3; q++)
+            reinterpret_cast<float4*>(s)[lane + 32 * q] = reinterpret_cast<const float4*>(g)[lane + 32 * q];
+    } else {
+        for (int i = lane; i < 3 * px; i += 32) s[i] = g[i];
+    }
+    __syncwarp();
+#pragma unroll UNROLL
+    for (int k = 0; k < PIX_WARP / 32; k++) {
+        const int i = lane + 32 * k;
+        if (i < px) {
+            float r = s[3 * i], gr = s[3 * i + 1], b = s[3 * i + 2];
+            f(r, gr, b);
+            s[3 * i] = r;
+            s[3 * i + 1] = gr;
+            s[3 * i + 2] = b;
+        }
+    }
+    __syncwarp();
+    if (whole) {
+#pragma unroll
+        for (int q = 0; q < 3; q++)
+            reinterpret_cast<float4*>(g)[lane + 32 * q] = reinterpret_cast<const float4*>(s)[lane + 32 * q];
+    } else {
+        for (int i = lane; i < 3 * px; i += 32) g[i] = s[i];
+    }
+}
+
+inline bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
+
 }  // namespace color
 }  // namespace imops
