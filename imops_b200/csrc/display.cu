@@ -75,6 +75,28 @@ __device__ __forceinline__ float cbrt_fast(float x) {
     return copysignf((ax * r) * r, x);
 }
 
+// Three cube roots, the special cases of cbrt_fast tested once for all three.
+__device__ __forceinline__ void cbrt3_fast(float& a, float& b, float& c) {
+    const float x[3] = {fabsf(a), fabsf(b), fabsf(c)};
+    if (!(fminf(fminf(x[0], x[1]), x[2]) >= 1.17549435e-38f) || !(x[0] + x[1] + x[2] < INFINITY)) {
+        a = cbrt_fast(a);
+        b = cbrt_fast(b);
+        c = cbrt_fast(c);
+        return;
+    }
+    float y[3];
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        float r = ex2_hw(lg2_hw(x[k]) * (-1.0f / 3.0f));
+        const float r3 = (r * r) * r;
+        r = (r * fmaf(-x[k], r3, 4.0f)) * (1.0f / 3.0f);
+        y[k] = (x[k] * r) * r;
+    }
+    a = copysignf(y[0], a);
+    b = copysignf(y[1], b);
+    c = copysignf(y[2], c);
+}
+
 // atan2(y, x) in radians.  The ratio a = min/max of |x|, |y| is in [0, 1],
 // where atan(a) = a P(a^2) with P of degree 8, fitted here for least maximum
 // relative error (1.5e-7 in f32); the octant puts it in (-pi, pi].
@@ -133,9 +155,7 @@ __device__ __forceinline__ void mv_fma(const float* m, float& r, float& g, float
 
 __device__ __forceinline__ void lin_to_oklch(float& r, float& g, float& b) {
     mv_fma(OK_M1, r, g, b);
-    r = cbrt_fast(r);
-    g = cbrt_fast(g);
-    b = cbrt_fast(b);
+    cbrt3_fast(r, g, b);
     mv_fma(OK_M2, r, g, b);
     float c = sqrtf(g * g + b * b);
     float h = atan2_fast(b, g) * 57.29577951308232f;
@@ -178,13 +198,14 @@ __device__ __forceinline__ void cst(const Op& o, float& r, float& g, float& b) {
 
 // compress_value (tone_map.rs:71-125) in the forward direction with the
 // default parameters: power 1.2; s_pre = the y = 1 intersect scale, or a
-// negative value when the reference returns dist unchanged.
+// negative value when the reference returns dist unchanged.  The bases of both
+// powers are not negative (dist >= thr, s > 0).
 __device__ __forceinline__ float compress(float dist, float thr, float s) {
     if (dist < thr) return dist;
     if (!(s > 0.0f)) return dist;
     const float power = 1.2f, inv_power = 1.0f / 1.2f;
-    float dn = __fdividef(dist - thr, s);
-    float den = pow_fast(1.0f + pow_fast(dn, power), inv_power);
+    const float dn = __fdividef(dist - thr, s);
+    const float den = ex2_hw(inv_power * lg2_hw(1.0f + ex2_hw(power * lg2_hw(dn))));
     return thr + s * __fdividef(dn, den);
 }
 
@@ -212,16 +233,21 @@ __device__ __forceinline__ void sigmoid(const Op& o, float& r, float& g, float& 
     } else {
         float aa = fabsf(ach);
         const float ia = __fdividef(1.0f, aa);
-        gc0 = ach - compress((ach - r) * ia, 0.815f, o.s[0]) * aa;
-        gc1 = ach - compress((ach - g) * ia, 0.803f, o.s[1]) * aa;
-        gc2 = ach - compress((ach - b) * ia, 0.88f, o.s[2]) * aa;
+        float d0 = (ach - r) * ia, d1 = (ach - g) * ia, d2 = (ach - b) * ia;
+        // most pixels lie inside the thresholds: one branch for the three channels
+        if (!(d0 < 0.815f && d1 < 0.803f && d2 < 0.88f)) {
+            d0 = compress(d0, 0.815f, o.s[0]);
+            d1 = compress(d1, 0.803f, o.s[1]);
+            d2 = compress(d2, 0.88f, o.s[2]);
+        }
+        gc0 = ach - d0 * aa;
+        gc1 = ach - d1 * aa;
+        gc2 = ach - d2 * aa;
     }
     // hue of the compressed pixel: Oklab a, b -> atan2
     float l0 = gc0, l1 = gc1, l2 = gc2;
     mv_fma(o.m[0], l0, l1, l2);
-    l0 = cbrt_fast(l0);
-    l1 = cbrt_fast(l1);
-    l2 = cbrt_fast(l2);
+    cbrt3_fast(l0, l1, l2);
     const float ha = fmaf(OK_M2[5], l2, fmaf(OK_M2[4], l1, OK_M2[3] * l0));
     const float hb = fmaf(OK_M2[8], l2, fmaf(OK_M2[7], l1, OK_M2[6] * l0));
     // the hue enters only through its cosine and sine: (a, b) / |(a, b)|.
@@ -244,9 +270,7 @@ __device__ __forceinline__ void sigmoid(const Op& o, float& r, float& g, float& 
     float m = 1.0f - (s2 * s2) * s;
     // lightness and chroma of the sigmoid
     mv_fma(o.m[0], p0, p1, p2);
-    p0 = cbrt_fast(p0);
-    p1 = cbrt_fast(p1);
-    p2 = cbrt_fast(p2);
+    cbrt3_fast(p0, p1, p2);
     mv_fma(OK_M2, p0, p1, p2);
     const float cm = sqrtf(p1 * p1 + p2 * p2) * m;
     // (L, C m, h) -> Oklab -> LMS -> ACEScg
