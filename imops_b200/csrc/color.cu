@@ -107,8 +107,28 @@ struct Levels {
 // One thread per column, SCALE_ROWS rows: the CFA site's column is found
 // once and its row stepped, the levels are read from shared memory.  A full
 // group of rows issues all its loads before the first division, so a thread
-// keeps SCALE_ROWS loads in flight.
+// keeps SCALE_ROWS loads in flight.  Frames whose cells share one level pair
+// (most) divide by it with LevelRange: 24 MP 30 us against 34.
 constexpr int SCALE_ROWS = 16;
+
+__global__ void __launch_bounds__(256) scale_u16_equal_kernel(const uint16_t* __restrict__ raw, int raw_w, int cw,
+                                                              int ch, const __grid_constant__ LevelRange lv,
+                                                              float* __restrict__ out) {
+    const int x = blockIdx.x * blockDim.x + threadIdx.x, y0 = blockIdx.y * SCALE_ROWS;
+    if (x >= cw) return;
+    const uint16_t* src = raw + (size_t)y0 * raw_w + x;
+    float* dst = out + (size_t)y0 * cw + x;
+    const int rows = ch - y0 < SCALE_ROWS ? ch - y0 : SCALE_ROWS;
+    if (rows == SCALE_ROWS) {
+        uint16_t v[SCALE_ROWS];
+#pragma unroll
+        for (int r = 0; r < SCALE_ROWS; r++) v[r] = __ldg(src + (size_t)r * raw_w);
+#pragma unroll
+        for (int r = 0; r < SCALE_ROWS; r++) dst[(size_t)r * cw] = lv.scale((float)v[r]);
+        return;
+    }
+    for (int r = 0; r < rows; r++) dst[(size_t)r * cw] = lv.scale((float)__ldg(src + (size_t)r * raw_w));
+}
 
 __global__ void scale_u16_kernel(const uint16_t* __restrict__ raw, int raw_w, int cx, int cy, int cw, int ch, int pw,
                                  int ph, const __grid_constant__ Levels lv, float* __restrict__ out) {
@@ -162,6 +182,16 @@ int stream_grid(size_t n, int block) {
     return (int)want;
 }
 
+int check_scale(const uint16_t* raw, int raw_w, int raw_h, int crop_x, int crop_y, int crop_w, int crop_h,
+                const float* black, const float* white, int period_w, int period_h, const float* out) {
+    if (!raw || !out || !black || !white) return fail(IMOPS_ERR_INVALID_ARGUMENT, "scale_u16: NULL buffer");
+    if (period_w <= 0 || period_h <= 0 || period_w * period_h > 144)
+        return fail(IMOPS_ERR_INVALID_ARGUMENT, "scale_u16: CFA period must be 1..144 cells");
+    if (crop_x < 0 || crop_y < 0 || crop_w <= 0 || crop_h <= 0 || crop_x + crop_w > raw_w || crop_y + crop_h > raw_h)
+        return fail(IMOPS_ERR_INVALID_ARGUMENT, "scale_u16: crop rectangle outside the frame");
+    return IMOPS_OK;
+}
+
 int run_epilogue(float* rgb, size_t n, const Epilogue& e, cudaStream_t s, const char* what) {
     if (!rgb && n) return fail(IMOPS_ERR_INVALID_ARGUMENT, std::string(what) + ": NULL buffer");
     if (n == 0) return IMOPS_OK;
@@ -182,19 +212,23 @@ extern "C" int imops_scale_u16(const uint16_t* raw, int raw_w, int raw_h, int cr
                                int crop_h, const float* black, const float* white, int period_w, int period_h,
                                float* out, imops_stream_t stream) {
     clear_error();
-    if (!raw || !out || !black || !white) return fail(IMOPS_ERR_INVALID_ARGUMENT, "scale_u16: NULL buffer");
-    if (period_w <= 0 || period_h <= 0 || period_w * period_h > 144)
-        return fail(IMOPS_ERR_INVALID_ARGUMENT, "scale_u16: CFA period must be 1..144 cells");
-    if (crop_x < 0 || crop_y < 0 || crop_w <= 0 || crop_h <= 0 || crop_x + crop_w > raw_w || crop_y + crop_h > raw_h)
-        return fail(IMOPS_ERR_INVALID_ARGUMENT, "scale_u16: crop rectangle outside the frame");
-    color::Levels lv;
-    for (int i = 0; i < period_w * period_h; i++) {
-        lv.v[i] = black[i];
-        lv.v[144 + i] = white[i];
-    }
+    if (int rc = color::check_scale(raw, raw_w, raw_h, crop_x, crop_y, crop_w, crop_h, black, white, period_w, period_h,
+                                    out))
+        return rc;
     dim3 grid((crop_w + 255) / 256, (crop_h + color::SCALE_ROWS - 1) / color::SCALE_ROWS);
-    color::scale_u16_kernel<<<grid, 256, 0, as_stream(stream)>>>(raw, raw_w, crop_x, crop_y, crop_w, crop_h,
-                                                                  period_w, period_h, lv, out);
+    color::LevelRange one;
+    if (one.usable(black, white, period_w * period_h)) {
+        color::scale_u16_equal_kernel<<<grid, 256, 0, as_stream(stream)>>>(raw + (size_t)crop_y * raw_w + crop_x, raw_w,
+                                                                            crop_w, crop_h, one, out);
+    } else {
+        color::Levels lv;
+        for (int i = 0; i < period_w * period_h; i++) {
+            lv.v[i] = black[i];
+            lv.v[144 + i] = white[i];
+        }
+        color::scale_u16_kernel<<<grid, 256, 0, as_stream(stream)>>>(raw, raw_w, crop_x, crop_y, crop_w, crop_h,
+                                                                      period_w, period_h, lv, out);
+    }
     note_launch();
     IMOPS_CUDA_TRY(cudaGetLastError(), "scale_u16 launch");
     return IMOPS_OK;

@@ -83,6 +83,35 @@ struct Epilogue {
 // decoding),ACESCG}; false otherwise.
 bool to_xyz(int space, float m[9]);
 
+// Division by one level range d for many samples: with y = 1/d correctly
+// rounded, q = n y corrected once by the exact remainder, q + (n - q d) y, is
+// the correctly rounded n / d (P. Markstein, "Computation of elementary
+// functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990),
+// three operations for the ten of a division.  Exact remainders need room
+// below n: `usable` where the black level is 0 or at least 2^-20 in magnitude
+// (so v - black is 0 or at least 2^-44) and the range lies in 2^-20 .. 2^20.
+struct LevelRange {
+    float black, range, inv;
+    __device__ __forceinline__ float scale(float v) const {
+        const float n = v - black, q = n * inv;
+        return __fmaf_rn(__fmaf_rn(-range, q, n), inv, q);
+    }
+    // the n levels all the same and usable
+    bool usable(const float* blacks, const float* whites, int n) {
+        for (int i = 1; i < n; i++)
+            if (blacks[i] != blacks[0] || whites[i] != whites[0]) return false;
+        black = blacks[0];
+        range = whites[0] - black;
+        inv = 1.0f / range;
+        const float lo = 1.0f / 1048576.0f, hi = 1048576.0f, b = black < 0.0f ? -black : black;
+        return (b == 0.0f || (b >= lo && b <= hi)) && range >= lo && range <= hi;
+    }
+};
+
+// The argument checks of imops_scale_u16.
+int check_scale(const uint16_t* raw, int raw_w, int raw_h, int crop_x, int crop_y, int crop_w, int crop_h,
+                const float* black, const float* white, int period_w, int period_h, const float* out);
+
 // Builds an identity epilogue (no-op).
 Epilogue identity_epilogue();
 

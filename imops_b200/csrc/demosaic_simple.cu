@@ -2,14 +2,16 @@
 // pichromatic/src/demosaic.rs:108-186) and the quad-sampling previews
 // (Fast / SuperFast / SuperSuperFast, demosaic.rs:189-356).
 //
-// The mean is HBM-bound (4 B in, 12 B out per pixel).  Every Bayer CFA is a
-// shift of RGGB and every X-Trans sensor's CFA a shift of one 6x6 pattern, so
+// The mean reads a mosaic (4 B a pixel, or 2 B of the sensor frame, scaled
+// while it is staged) and writes 12 B.  Every Bayer CFA is a shift of RGGB and every X-Trans sensor's CFA a shift of one 6x6 pattern, so
 // for those the kernel aligns each thread's run of pixels with the pattern:
 // the colour of every site in a run's window is then a compile-time constant
 // (per row phase, and a warp handles one row), the per-colour sums are plain
 // adds and the counts constants.  Other CFAs take the per-pixel kernel.  Both
 // sum each colour's sites in row-major order and divide once, as the
 // reference's f32 code does; built with --fmad=false.
+#include <type_traits>
+
 #include "color.cuh"
 #include "common.cuh"
 #include "demosaic_simple.cuh"
@@ -21,14 +23,13 @@ namespace simple {
 // (the window clamped at the image edges), the centre's own colour keeping
 // the centre sample.  Cfa: CfaFixed<2, 2> / CfaFixed<6, 6> for Bayer and
 // X-Trans, CfaDev for other periods; coordinates here are never negative.
-template <class Cfa>
-__device__ __forceinline__ void mean_px(const float* __restrict__ in, int W, int H, const Cfa& cfa, int row,
-                                        int col, float* o) {
+// in(y, x): the mosaic.
+template <class In, class Cfa>
+__device__ __forceinline__ void mean_px(const In& in, int W, int H, const Cfa& cfa, int row, int col, float* o) {
     const int centre = cfa.at(row, col);
     if (row >= 1 && row + 1 < H && col >= 1 && col + 1 < W) {
         // interior: the whole 3x3 window, unrolled and branch-free; each
         // colour's sum takes its sites in row-major order (predicated adds)
-        const float* p = in + (size_t)(row - 1) * W + (col - 1);
         float s0 = 0.0f, s1 = 0.0f, s2 = 0.0f, n0 = 0.0f, n1 = 0.0f, n2 = 0.0f;
 #pragma unroll
         for (int a = 0; a < 3; a++)
@@ -36,7 +37,7 @@ __device__ __forceinline__ void mean_px(const float* __restrict__ in, int W, int
             for (int b = 0; b < 3; b++) {
                 if (a == 1 && b == 1) continue;
                 const int k = cfa.at(row + a - 1, col + b - 1);
-                const float v = __ldg(p + (size_t)a * W + b);
+                const float v = in(row + a - 1, col + b - 1);
                 s0 = k == 0 ? s0 + v : s0;
                 n0 = k == 0 ? n0 + 1.0f : n0;
                 s1 = k == 1 ? s1 + v : s1;
@@ -44,7 +45,7 @@ __device__ __forceinline__ void mean_px(const float* __restrict__ in, int W, int
                 s2 = k == 2 ? s2 + v : s2;
                 n2 = k == 2 ? n2 + 1.0f : n2;
             }
-        const float self = __ldg(in + (size_t)row * W + col);
+        const float self = in(row, col);
         o[0] = centre == 0 ? self : (n0 > 0.0f ? s0 / n0 : 0.0f);
         o[1] = centre == 1 ? self : (n1 > 0.0f ? s1 / n1 : 0.0f);
         o[2] = centre == 2 ? self : (n2 > 0.0f ? s2 / n2 : 0.0f);
@@ -59,7 +60,7 @@ __device__ __forceinline__ void mean_px(const float* __restrict__ in, int W, int
         for (int nx = x0; nx <= x1; nx++) {
             if (ny == row && nx == col) continue;
             const int k = cfa.at(ny, nx);
-            const float v = __ldg(in + (size_t)ny * W + nx);
+            const float v = in(ny, nx);
             if (k == 0) {
                 s0 += v;
                 n0 += 1.0f;
@@ -71,11 +72,19 @@ __device__ __forceinline__ void mean_px(const float* __restrict__ in, int W, int
                 n2 += 1.0f;
             }
         }
-    const float self = __ldg(in + (size_t)row * W + col);
+    const float self = in(row, col);
     o[0] = centre == 0 ? self : (n0 > 0.0f ? s0 / n0 : 0.0f);
     o[1] = centre == 1 ? self : (n1 > 0.0f ? s1 / n1 : 0.0f);
     o[2] = centre == 2 ? self : (n2 > 0.0f ? s2 / n2 : 0.0f);
 }
+
+// An f32 mosaic.
+struct SrcF32 {
+    const float* __restrict__ p;
+    int W;
+    using Raw = float;
+    __device__ __forceinline__ float operator()(int y, int x) const { return __ldg(p + (size_t)y * W + x); }
+};
 
 // The mean alone.
 struct NoEpilogue {
@@ -92,7 +101,7 @@ __global__ void mean3x3_kernel(const float* __restrict__ in, int W, int H, const
     int row = blockIdx.y * blockDim.y + threadIdx.y;
     if (col >= W || row >= H) return;
     float v[3];
-    mean_px(in, W, H, cfa, row, col, v);
+    mean_px(SrcF32{in, W}, W, H, cfa, row, col, v);
     epi.apply(v[0], v[1], v[2]);
     float* o = out + ((size_t)row * W + col) * 3;
     o[0] = v[0];
@@ -125,7 +134,8 @@ struct XTransCanon {  // the X-Trans sensors' 6x6 period
 };
 
 // Phase-aligned kernel geometry: a warp handles one image row, RUN pixels a
-// lane, 32 * RUN pixels a warp; RUN is a multiple of both periods.
+// lane, 32 * RUN pixels a warp; RUN is a multiple of both periods.  A block's
+// eight rows share ten staged ones.
 constexpr int RUN = 6;
 constexpr int WARP_PX = 32 * RUN;              // 192
 constexpr int IN_STRIDE = WARP_PX + 4;         // 194 staged columns, padded to a 16-byte multiple
@@ -175,58 +185,107 @@ __device__ __forceinline__ void run_phase(int rp, const float (&v)[3][RUN + 2], 
     }
 }
 
+// What the aligned kernel stages: an f32 mosaic as it is, or a u16 sensor
+// frame's crop scaled as color::scale_u16_kernel does, (v - black) / (white -
+// black) per cell of the level period, each sample once a block (1.29 times a
+// pixel with the halo).
+struct StageF32 {
+    SrcF32 src;
+    using Raw = float;
+    __device__ __forceinline__ void init(float*) const {}
+    __device__ __forceinline__ Raw fetch(int y, int x) const { return src(y, x); }
+    __device__ __forceinline__ float value(Raw v, const float*, int, int) const { return v; }
+    __device__ __forceinline__ int column(int) const { return 0; }
+    __device__ __forceinline__ int next(int c) const { return c; }
+    __device__ __forceinline__ int row(int) const { return 0; }
+};
+struct StageU16 {  // one level pair for all cells
+    const uint16_t* __restrict__ raw;  // at the crop's origin
+    int raw_w;
+    color::LevelRange lv;
+    using Raw = uint16_t;
+    __device__ __forceinline__ void init(float*) const {}
+    __device__ __forceinline__ Raw fetch(int y, int x) const { return __ldg(raw + (size_t)y * raw_w + x); }
+    __device__ __forceinline__ float value(Raw v, const float*, int, int) const { return lv.scale((float)v); }
+    __device__ __forceinline__ int column(int) const { return 0; }
+    __device__ __forceinline__ int next(int c) const { return c; }
+    __device__ __forceinline__ int row(int) const { return 0; }
+};
+struct StageU16Cells {
+    const uint16_t* __restrict__ raw;  // at the crop's origin
+    int raw_w, cx, cy, pw, ph, step;   // step = 32 % pw
+    float black[144], range[144];
+    using Raw = uint16_t;
+    __device__ __forceinline__ void init(float* levels) const {
+        for (int i = threadIdx.y * 32 + threadIdx.x; i < pw * ph; i += 32 * MEAN_WARPS) {
+            levels[i] = black[i];
+            levels[144 + i] = range[i];
+        }
+        __syncthreads();
+    }
+    __device__ __forceinline__ Raw fetch(int y, int x) const { return __ldg(raw + (size_t)y * raw_w + x); }
+    __device__ __forceinline__ float value(Raw v, const float* levels, int row, int col) const {
+        const int i = row * pw + col;
+        return ((float)v - levels[i]) / levels[144 + i];
+    }
+    // a column's and a row's place in the level period
+    __device__ __forceinline__ int column(int x) const { return (cx + x + 144 * pw) % pw; }
+    __device__ __forceinline__ int next(int c) const { return c + step >= pw ? c + step - pw : c + step; }
+    __device__ __forceinline__ int row(int y) const { return (cy + y + ph) % ph; }
+};
+
 // The CFA is P shifted: colour(y, x) = P::at((y - oy) mod PH, (x - ox) mod PW)
 // with 0 <= ox < PW, 0 <= oy < PH.  Warp w of block (bx, by) develops row
 // y = 8 by + w, pixels x_start + 192 bx .. + 191 with x_start = 0 when
 // ox == 0 else ox - PW, so every lane's run starts at canonical column 0.
-// The warp stages its three rows in shared memory (coalesced loads), each
+// The block stages its ten rows in shared memory (coalesced loads), each
 // lane computes its run from there -- or, when the run or its window touches
 // the image edge, each pixel with mean_px -- into a shared output row that
 // the warp then stores coalesced.
-template <class P, class Epi>
-__global__ void __launch_bounds__(32 * MEAN_WARPS) mean3x3_aligned_kernel(
-    const float* __restrict__ in, int W, int H, int ox, int oy, const __grid_constant__ CfaFixed<P::PW, P::PH> cfa,
+//
+// Bound by instruction issue with a colour epilogue, by HBM latency without.
+// 24 MP: X-Trans u16 frame to ACEScg in one pass 166 us, where scaling it to an
+// f32 mosaic (34) and three rows staged a warp (177) took 211; f32 mosaic to
+// camera RGB 98 us (100).
+template <class P, class Epi, class Stage>
+__global__ void __launch_bounds__(32 * MEAN_WARPS, std::is_same<Stage, StageF32>::value ? 5 : 4) mean3x3_aligned_kernel(
+    const __grid_constant__ Stage st, int W, int H, int ox, int oy, const __grid_constant__ CfaFixed<P::PW, P::PH> cfa,
     const __grid_constant__ Epi epi, float* __restrict__ out) {
-    __shared__ __align__(16) float sin_[MEAN_WARPS][3][IN_STRIDE];
+    __shared__ __align__(16) float sin_[MEAN_WARPS + 2][IN_STRIDE];
     __shared__ __align__(16) float sout[MEAN_WARPS][OUT_STRIDE];
+    __shared__ float levels[std::is_same<Stage, StageU16Cells>::value ? 288 : 1];
+    st.init(levels);
     const int lane = threadIdx.x, w = threadIdx.y;
-    const int y = blockIdx.y * MEAN_WARPS + w;
-    if (y >= H) return;  // whole warp: only warp-level synchronisation below
+    const int y0 = blockIdx.y * MEAN_WARPS, y = y0 + w;
     const int xs = ox == 0 ? 0 : ox - P::PW;
     const int xw = xs + blockIdx.x * WARP_PX;  // first pixel of the warp
-    // stage rows y-1..y+1, columns xw-1 .. xw+192 (zeros outside the image;
-    // only runs whose window lies inside read them).  All 21 loads of a lane
-    // are issued before the first store, so a warp keeps them in flight
-    // together; warps whose rows lie inside the image skip the per-element
-    // tests.
+    // stage rows y0-1 .. y0+8, columns xw-1 .. xw+192 (zeros outside the image,
+    // read by nothing that is stored): warp w row w, warps 0 and 1 also rows
+    // 8 and 9.  A row's seven loads a lane are issued before its first store.
     constexpr int NQ = (WARP_PX + 2 + 31) / 32;
-    float t[3][NQ];
-    if (y >= 1 && y + 1 < H && xw >= 1 && xw + WARP_PX + 1 <= W) {
-        const float* src = in + (size_t)(y - 1) * W + (xw - 1) + lane;
+    const bool inner = xw >= 1 && xw + WARP_PX + 1 <= W;
+    int col[NQ];
+    col[0] = st.column(xw - 1 + lane);
 #pragma unroll
-        for (int a = 0; a < 3; a++)
+    for (int q = 1; q < NQ; q++) col[q] = st.next(col[q - 1]);
+#pragma unroll 1
+    for (int a = 0; a < 2; a++) {
+        const int r = w + MEAN_WARPS * a, yy = y0 - 1 + r;
+        if (r >= MEAN_WARPS + 2) break;
+        const bool yin = yy >= 0 && yy < H;
+        typename Stage::Raw t[NQ];
 #pragma unroll
-            for (int q = 0; q < NQ; q++)
-                t[a][q] = lane + 32 * q < WARP_PX + 2 ? __ldg(src + (size_t)a * W + 32 * q) : 0.0f;
-    } else {
-#pragma unroll
-        for (int a = 0; a < 3; a++) {
-            const int yy = y + a - 1;
-            const bool yin = yy >= 0 && yy < H;
-            const float* src = in + (size_t)(yin ? yy : 0) * W;
-#pragma unroll
-            for (int q = 0; q < NQ; q++) {
-                const int i = lane + 32 * q, x = xw - 1 + i;
-                t[a][q] = yin && i < WARP_PX + 2 && x >= 0 && x < W ? __ldg(src + x) : 0.0f;
-            }
+        for (int q = 0; q < NQ; q++) {
+            const int i = lane + 32 * q, x = xw - 1 + i;
+            t[q] = yin && i < WARP_PX + 2 && (inner || (x >= 0 && x < W)) ? st.fetch(yy, x) : typename Stage::Raw(0);
         }
-    }
-#pragma unroll
-    for (int a = 0; a < 3; a++)
+        const int rp = st.row(yy);
 #pragma unroll
         for (int q = 0; q < NQ; q++)
-            if (lane + 32 * q < WARP_PX + 2) sin_[w][a][lane + 32 * q] = t[a][q];
-    __syncwarp();
+            if (lane + 32 * q < WARP_PX + 2) sin_[r][lane + 32 * q] = st.value(t[q], levels, rp, col[q]);
+    }
+    __syncthreads();
+    if (y >= H) return;  // whole warp: only warp-level synchronisation below
     // the warp's pixels inside the image, and the shared output row's offset
     // m: float k of the row goes to address dst0 + (k - K0), and m makes
     // shared and global 16-byte boundaries coincide
@@ -241,15 +300,13 @@ __global__ void __launch_bounds__(32 * MEAN_WARPS) mean3x3_aligned_kernel(
         for (int a = 0; a < 3; a++)
 #pragma unroll
             for (int c = 0; c < RUN + 2; c += 2) {
-                const float2 t2 = *reinterpret_cast<const float2*>(&sin_[w][a][RUN * lane + c]);
+                const float2 t2 = *reinterpret_cast<const float2*>(&sin_[w + a][RUN * lane + c]);
                 v[a][c] = t2.x;
                 v[a][c + 1] = t2.y;
             }
         const int rp = (y + P::PH - oy) % P::PH;
         float r[3 * RUN];
         run_phase<P, 0>(rp, v, r);
-#pragma unroll
-        for (int j = 0; j < RUN; j++) epi.apply(r[3 * j], r[3 * j + 1], r[3 * j + 2]);
         if (m & 1) {
 #pragma unroll
             for (int c = 0; c < 3 * RUN; c++) o[c] = r[c];
@@ -262,8 +319,7 @@ __global__ void __launch_bounds__(32 * MEAN_WARPS) mean3x3_aligned_kernel(
             const int x = x0 + j;
             if (x >= 0 && x < W) {
                 float q[3];
-                mean_px(in, W, H, cfa, y, x, q);
-                epi.apply(q[0], q[1], q[2]);
+                mean_px([&](int yy, int xx) { return sin_[yy - y0 + 1][xx - xw + 1]; }, W, H, cfa, y, x, q);
                 o[3 * j] = q[0];
                 o[3 * j + 1] = q[1];
                 o[3 * j + 2] = q[2];
@@ -272,6 +328,21 @@ __global__ void __launch_bounds__(32 * MEAN_WARPS) mean3x3_aligned_kernel(
     }
     __syncwarp();
     if (p1 <= p0) return;
+    if constexpr (!std::is_same<Epi, NoEpilogue>::value) {
+        // the colour epilogue in a loop of its own, a pixel a lane: inlined for
+        // each of a run's pixels its code outgrew the instruction cache, as the
+        // warps are in different row phases already
+#pragma unroll 2
+        for (int x = p0 + lane; x < p1; x += 32) {
+            float* q = &sout[w][m + 3 * (x - xw)];
+            float r = q[0], g = q[1], b = q[2];
+            epi.apply(r, g, b);
+            q[0] = r;
+            q[1] = g;
+            q[2] = b;
+        }
+        __syncwarp();
+    }
     // shared floats K0..K1-1 -> dst0: a scalar head up to a 16-byte boundary,
     // float4 chunks, a scalar tail
     const int K0 = m + 3 * (p0 - xw), K1 = m + 3 * (p1 - xw);
@@ -307,24 +378,30 @@ bool canonical_offset(const CfaDev& c, int* ox, int* oy) {
     return false;
 }
 
-template <class P, class Epi>
-void launch_aligned(const float* mosaic, int w, int h, const CfaDev& c, int ox, int oy, const Epi& epi, float* rgb,
+template <class P, class Epi, class Stage>
+void launch_aligned(const Stage& st, int w, int h, const CfaDev& c, int ox, int oy, const Epi& epi, float* rgb,
                     cudaStream_t s) {
     const int xs = ox == 0 ? 0 : ox - P::PW;
     dim3 block(32, MEAN_WARPS), grid((w - xs + WARP_PX - 1) / WARP_PX, (h + MEAN_WARPS - 1) / MEAN_WARPS);
-    mean3x3_aligned_kernel<P, Epi><<<grid, block, 0, s>>>(mosaic, w, h, ox, oy, CfaFixed<P::PW, P::PH>::from(c), epi,
-                                                          rgb);
+    mean3x3_aligned_kernel<P, Epi, Stage><<<grid, block, 0, s>>>(st, w, h, ox, oy, CfaFixed<P::PW, P::PH>::from(c),
+                                                                 epi, rgb);
+}
+
+// The aligned kernel where the CFA is a shift of a canonical pattern.
+template <class Epi, class Stage>
+bool launch_canonical(const Stage& st, int w, int h, const CfaDev& c, const Epi& epi, float* rgb, cudaStream_t s) {
+    int ox, oy;
+    if (canonical_offset<BayerCanon>(c, &ox, &oy)) launch_aligned<BayerCanon>(st, w, h, c, ox, oy, epi, rgb, s);
+    else if (canonical_offset<XTransCanon>(c, &ox, &oy)) launch_aligned<XTransCanon>(st, w, h, c, ox, oy, epi, rgb, s);
+    else return false;
+    return true;
 }
 
 template <class Epi>
 void launch_mean(const float* mosaic, int w, int h, const CfaDev& c, const Epi& epi, float* rgb, cudaStream_t s) {
     dim3 block(32, 8), grid((w + 31) / 32, (h + 7) / 8);
-    int ox, oy;
-    if (canonical_offset<BayerCanon>(c, &ox, &oy))
-        launch_aligned<BayerCanon>(mosaic, w, h, c, ox, oy, epi, rgb, s);
-    else if (canonical_offset<XTransCanon>(c, &ox, &oy))
-        launch_aligned<XTransCanon>(mosaic, w, h, c, ox, oy, epi, rgb, s);
-    else if (c.pw == 2 && c.ph == 2)
+    if (launch_canonical(StageF32{{mosaic, w}}, w, h, c, epi, rgb, s)) return;
+    if (c.pw == 2 && c.ph == 2)
         mean3x3_kernel<<<grid, block, 0, s>>>(mosaic, w, h, CfaFixed<2, 2>::from(c), epi, rgb);
     else if (c.pw == 6 && c.ph == 6)
         mean3x3_kernel<<<grid, block, 0, s>>>(mosaic, w, h, CfaFixed<6, 6>::from(c), epi, rgb);
@@ -343,6 +420,35 @@ int mean3x3(const float* mosaic, int w, int h, const CfaDev& c, const color::Epi
     else launch_mean(mosaic, w, h, c, NoEpilogue{}, rgb, s);
     note_launch();
     IMOPS_CUDA_TRY(cudaGetLastError(), "markesteijn launch");
+    return IMOPS_OK;
+}
+
+int mean3x3_u16(const uint16_t* raw, int raw_w, int raw_h, int cx, int cy, int w, int h, const float* black,
+                const float* white, int pw, int ph, const CfaDev& c, const color::Epilogue& epi, float* rgb,
+                bool* done, cudaStream_t s) {
+    *done = false;
+    int ox, oy;
+    if (!canonical_offset<BayerCanon>(c, &ox, &oy) && !canonical_offset<XTransCanon>(c, &ox, &oy)) return IMOPS_OK;
+    int rc = color::check_scale(raw, raw_w, raw_h, cx, cy, w, h, black, white, pw, ph, rgb);
+    if (rc) return rc;
+    if ((uintptr_t)rgb & 3)
+        return fail(IMOPS_ERR_INVALID_ARGUMENT, "markesteijn: buffers must be 4-byte aligned float arrays");
+    if (fault_injected("launch")) return fail(IMOPS_ERR_CUDA, "injected launch failure (markesteijn)");
+    const uint16_t* origin = raw + (size_t)cy * raw_w + cx;
+    color::LevelRange one;
+    if (one.usable(black, white, pw * ph)) {
+        launch_canonical(StageU16{origin, raw_w, one}, w, h, c, epi, rgb, s);
+    } else {
+        StageU16Cells st{origin, raw_w, cx, cy, pw, ph, 32 % pw, {}, {}};
+        for (int i = 0; i < pw * ph; i++) {
+            st.black[i] = black[i];
+            st.range[i] = white[i] - black[i];
+        }
+        launch_canonical(st, w, h, c, epi, rgb, s);
+    }
+    note_launch();
+    IMOPS_CUDA_TRY(cudaGetLastError(), "markesteijn launch");
+    *done = true;
     return IMOPS_OK;
 }
 

@@ -15,5 +15,12 @@ namespace simple {
 int mean3x3(const float* mosaic, int w, int h, const CfaDev& c, const color::Epilogue* epi, float* rgb,
             cudaStream_t s);
 
+// The same straight from a u16 sensor frame's crop, scaled as imops_scale_u16
+// does (with its checks): one pass, no f32 mosaic.  Only for shifts of the
+// Bayer and X-Trans patterns (*done tells); other CFAs scale first.
+int mean3x3_u16(const uint16_t* raw, int raw_w, int raw_h, int cx, int cy, int w, int h, const float* black,
+                const float* white, int pw, int ph, const CfaDev& c, const color::Epilogue& epi, float* rgb,
+                bool* done, cudaStream_t s);
+
 }  // namespace simple
 }  // namespace imops

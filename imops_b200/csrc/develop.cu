@@ -66,13 +66,20 @@ extern "C" int imops_develop_u16(const uint16_t* raw, int raw_w, int raw_h, int 
         rc = amaze::demosaic_color_u16(raw, raw_w, raw_h, crop_x, crop_y, crop_w, crop_h, black, white, period_w,
                                        period_h, cfa, P.clip_pt, e, rgb, s);
     } else if (P.demosaic == IMOPS_DEMOSAIC_MARKESTEIJN) {
-        float* m = nullptr;
-        if ((rc = develop::mosaic_buffer(s, (size_t)crop_w * crop_h * 4, &m))) return rc;
-        if ((rc = imops_scale_u16(raw, raw_w, raw_h, crop_x, crop_y, crop_w, crop_h, black, white, period_w,
-                                  period_h, m, stream)))
+        // the 3x3 mean with the colour epilogue applied before its store; the
+        // usual CFAs are scaled as the frame is staged
+        bool done = false;
+        if ((rc = simple::mean3x3_u16(raw, raw_w, raw_h, crop_x, crop_y, crop_w, crop_h, black, white, period_w,
+                                      period_h, cfa, e, rgb, &done, s)))
             return rc;
-        // the 3x3 mean with the colour epilogue applied before its store
-        if ((rc = simple::mean3x3(m, crop_w, crop_h, cfa, &e, rgb, s))) return rc;
+        if (!done) {
+            float* m = nullptr;
+            if ((rc = develop::mosaic_buffer(s, (size_t)crop_w * crop_h * 4, &m))) return rc;
+            if ((rc = imops_scale_u16(raw, raw_w, raw_h, crop_x, crop_y, crop_w, crop_h, black, white, period_w,
+                                      period_h, m, stream)))
+                return rc;
+            if ((rc = simple::mean3x3(m, crop_w, crop_h, cfa, &e, rgb, s))) return rc;
+        }
     } else {
         return fail(IMOPS_ERR_INVALID_ARGUMENT, "develop: demosaic must be AMaZE or Markesteijn");
     }
