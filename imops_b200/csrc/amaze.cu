@@ -35,7 +35,12 @@ namespace amaze {
 
 constexpr int TS = 128, TSH = 64, NF = TS * TS, NH = TS * TSH;
 constexpr int V1 = 128, V2 = 256, V3 = 384, P1 = 127, P2 = 254, P3 = 381, M1 = 129, M2 = 258, M3 = 387;
-constexpr int NTHREADS = 512;
+// 24 warps: 80 registers a thread (a few spill in the column pass) against 128
+// at 16 warps, and shorter column segments (their windows' run-in is 4 rows in
+// 24 instead of 4 in 34) still come out ahead, 1-6% over frames of little and
+// much texture: more warps hide the IEEE divisions' latency (0.70 of the
+// issue rate against 0.64).  6 MP: 0.66-1.11 ms against 0.67-1.18.
+constexpr int NTHREADS = 768;
 static_assert(NTHREADS % TS == 0 && NTHREADS % TSH == 0, "row mapping of the stage loops");
 
 constexpr size_t SMEM_BYTES = (3 * (size_t)NF + (size_t)NH) * 4 + 64;
@@ -170,13 +175,15 @@ __device__ void fill(const P& p, const Geo& g, float* mos) {
     if (g.rrmin == 0 && g.ccmin == 0 && g.rrmax == g.rr1 && g.ccmax == g.cc1) {
         // a whole 128 x 128 tile inside the image: every load in flight
         // before the first store
-        constexpr int RPT = TS / (NTHREADS / TS);
+        constexpr int RG = NTHREADS / TS, RPT = (TS + RG - 1) / RG;
         const int cc = (int)(threadIdx.x & (TS - 1)), r0 = (int)(threadIdx.x / TS);
         float v[RPT];
 #pragma unroll
-        for (int i = 0; i < RPT; i++) v[i] = p.in(top + r0 + i * (NTHREADS / TS), left + cc);
+        for (int i = 0; i < RPT; i++)
+            if (TS % RG == 0 || r0 + i * RG < TS) v[i] = p.in(top + r0 + i * RG, left + cc);
 #pragma unroll
-        for (int i = 0; i < RPT; i++) mos[(r0 + i * (NTHREADS / TS)) * TS + cc] = v[i];
+        for (int i = 0; i < RPT; i++)
+            if (TS % RG == 0 || r0 + i * RG < TS) mos[(r0 + i * RG) * TS + cc] = v[i];
         return;
     }
     if (g.rrmin > 0)
@@ -525,7 +532,7 @@ __device__ __forceinline__ int chain_map(float hav, float prevA, float prevB, fl
 }
 
 constexpr int VSEG = NTHREADS / TS;  // row segments of the column pass
-constexpr int VSEGLEN = 30;          // chain rows per segment
+constexpr int VSEGLEN = (TS - 8 + VSEG - 1) / VSEG;  // chain rows per segment
 static_assert(VSEG * VSEGLEN >= TS - 8, "column-pass segments must cover the band");
 
 // Column pass: demosaic.rs:612-698 (vertical half), the vcd chains of
@@ -807,7 +814,7 @@ __device__ NyqBox st_nyq_test(const P& p, const Geo& g, const Bufs& b, int* sh) 
         b.nyq2w[threadIdx.x] = 0ull;
     }
     __syncthreads();
-    constexpr int PER = 15;  // R/B rows per segment: 4 x 15 >= 58
+    constexpr int PER = ((TS - 12) / 2 + VSEG - 1) / VSEG;  // R/B rows per segment
     static_assert(VSEG * PER * 2 >= TS - 12, "Nyquist segments must cover the rows");
     const int c = threadIdx.x & (TS - 1), sg = threadIdx.x / TS;
     int lr0 = 1 << 30, lr1 = -1, lc0 = TS + 1, lc1 = 0;
@@ -881,7 +888,13 @@ __device__ NyqBox st_nyq_test(const P& p, const Geo& g, const Bufs& b, int* sh) 
 }
 
 // demosaic.rs:873-947: majority vote inside the box, then the area-based
-// weight at voted sites.
+// weight at voted sites: sums over the voted sites of the 7 x 7 same-colour
+// window, in row-major order.  A thread takes four sites of a column (rows 2
+// apart), whose windows share most of their rows: a window sample's terms are
+// formed once and added to the sums of every site that has it in its window,
+// each site's sums still in their own order.  On frames full of such texture
+// the site-by-site form took up to a third of the kernel (6 MP, such a frame: 1.18 ms, now 1.05, with 24 warps 0.99).
+constexpr int NYQ_SITES = 4;
 template <class P>
 __device__ void st_nyquist_area(const P& p, const Geo& g, const Bufs& b, const NyqBox& box) {
     const float epssq = 1e-10f;
@@ -893,31 +906,64 @@ __device__ void st_nyquist_area(const P& p, const Geo& g, const Bufs& b, const N
         if (s > 4 || (s == 4 && rbflag(n, i))) rbflag_set(b.nyq2w, i);
     });
     __syncthreads();
-    for_rb(p, g, box.r0, box.r1, box.c0, box.c1, [&](int rr, int cc) {
-        int i = rr * TS + cc;
-        if (!rbflag(b.nyq2w, i)) return;
-        const float* m = b.mos;
-        float sumcfa = 0.f, sumh = 0.f, sumv = 0.f, sumsqh = 0.f, sumsqv = 0.f, area = 0.f;
-        for (int di = -6; di < 7; di += 2)
-            for (int dj = -6; dj < 7; dj += 2) {
-                int j = i + di * TS + dj;
-                if (rbflag(b.nyq2w, j)) {
-                    float v = m[j];
-                    sumcfa += v;
-                    sumh += m[j - 1] + m[j + 1];
-                    sumv += m[j - V1] + m[j + V1];
-                    sumsqh += sqr(v - m[j - 1]) + sqr(v - m[j + 1]);
-                    sumsqv += sqr(v - m[j - V1]) + sqr(v - m[j + V1]);
-                    area += 1.0f;
-                }
+    const int w = (box.c1 - box.c0 + 1) >> 1, rows = box.r1 - box.r0;
+    if (w <= 0 || rows <= 0) return;
+    // groups of 2 NYQ_SITES rows, the even and the odd ones apart
+    const int items = (rows + 2 * NYQ_SITES - 1) / (2 * NYQ_SITES) * 2 * w;
+    for (int t = threadIdx.x; t < items; t += NTHREADS) {
+        const int q = t / w, rr = box.r0 + (q >> 1) * 2 * NYQ_SITES + (q & 1);
+        const int cc = box.c0 + (p.cfa.at(g.top + rr, g.left + 2) & 1) + 2 * (t - q * w);
+        if (cc >= box.c1) continue;
+        unsigned voted = 0;  // bit s: site s, row rr + 2 s, is voted
+#pragma unroll
+        for (int s = 0; s < NYQ_SITES; s++)
+            if (rr + 2 * s < box.r1 && rbflag(b.nyq2w, (rr + 2 * s) * TS + cc)) voted |= 1u << s;
+        if (!voted) continue;
+        float cfa[NYQ_SITES], sh[NYQ_SITES], sv[NYQ_SITES], qh[NYQ_SITES], qv[NYQ_SITES];
+        int cnt[NYQ_SITES];
+#pragma unroll
+        for (int s = 0; s < NYQ_SITES; s++) {
+            cfa[s] = sh[s] = sv[s] = qh[s] = qv[s] = 0.0f;
+            cnt[s] = 0;
+        }
+        // window rows rr - 6 .. rr + 2 NYQ_SITES + 4; row k belongs to the
+        // sites max(0, k - 6) .. min(k, NYQ_SITES - 1)
+#pragma unroll
+        for (int k = 0; k < NYQ_SITES + 6; k++) {
+            constexpr unsigned ALL = (1u << NYQ_SITES) - 1u;
+            const unsigned sites = (k < NYQ_SITES ? (2u << k) - 1u : ALL) & (k > 6 ? ALL << (k - 6) : ALL);
+            if (!(voted & sites)) continue;
+            const int row = rr - 6 + 2 * k;
+            unsigned bits = (unsigned)(b.nyq2w[row] >> ((cc >> 1) - 3)) & 127u;
+#pragma unroll
+            for (int s = 0; s < NYQ_SITES; s++)
+                if ((sites >> s) & 1u) cnt[s] += __popc(bits);
+            const float* m = b.mos + row * TS + cc - 6;
+            for (; bits; bits >>= 1, m += 2) {
+                if (!(bits & 1u)) continue;
+                const float v = m[0], l = m[-1], r = m[1], u = m[-V1], d = m[V1];
+                const float h2 = l + r, v2 = u + d;
+                const float dh = sqr(v - l) + sqr(v - r), dv = sqr(v - u) + sqr(v - d);
+#pragma unroll
+                for (int s = 0; s < NYQ_SITES; s++)
+                    if ((sites >> s) & 1u) {
+                        cfa[s] += v;
+                        sh[s] += h2;
+                        sv[s] += v2;
+                        qh[s] += dh;
+                        qv[s] += dv;
+                    }
             }
-        sumh = sumcfa - sumh * 0.5f;
-        sumv = sumcfa - sumv * 0.5f;
-        area = area * 0.5f;
-        float hvar = epssq + fabsf(area * sumsqh - sumh * sumh);
-        float vvar = epssq + fabsf(area * sumsqv - sumv * sumv);
-        b.hvwt[i >> 1] = hvar / (vvar + hvar);
-    });
+        }
+#pragma unroll
+        for (int s = 0; s < NYQ_SITES; s++) {
+            if (!((voted >> s) & 1u)) continue;
+            const float sumh = cfa[s] - sh[s] * 0.5f, sumv = cfa[s] - sv[s] * 0.5f, area = (float)cnt[s] * 0.5f;
+            const float hvar = epssq + fabsf(area * qh[s] - sumh * sumh);
+            const float vvar = epssq + fabsf(area * qv[s] - sumv * sumv);
+            b.hvwt[((rr + 2 * s) * TS + cc) >> 1] = hvar / (vvar + hvar);
+        }
+    }
 }
 
 // demosaic.rs:949-958: hvwt smoothing (one warp).
@@ -1309,7 +1355,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) amaze_kernel(const __grid_constan
     __shared__ int box_sh[4];
     // chain segment maps of the column pass, later the Nyquist row masks
     __shared__ __align__(8) unsigned long long rowbits[2 * TS];
-    static_assert(VSEG * TS * 2 <= sizeof(unsigned long long) * TS, "segment maps fit the first mask array");
+    static_assert(VSEG * TS * 2 <= sizeof(unsigned long long) * 2 * TS, "segment maps fit the mask arrays");
     uint8_t* segmap = reinterpret_cast<uint8_t*>(rowbits);
     Bufs b;
     b.mos = smem;
