@@ -6,6 +6,8 @@
 #include <cstring>
 #include <atomic>
 #include <mutex>
+#include <system_error>
+#include <thread>
 
 namespace imops {
 
@@ -147,8 +149,125 @@ void StreamCache::release_device(int dev) {
     }
 }
 
+// ---- downloads -----------------------------------------------------------------
+
+namespace {
+
+struct Ring {
+    int dev = -1;
+    bool busy = false;
+    void* slot[DOWNLOAD_SLOTS] = {};
+    cudaEvent_t filled[DOWNLOAD_SLOTS] = {};
+};
+std::mutex g_rings_mu;
+Ring g_rings[DOWNLOAD_RINGS];
+
+void free_ring(Ring& r) {
+    for (int i = 0; i < DOWNLOAD_SLOTS; i++) {
+        if (r.slot[i]) cudaFreeHost(r.slot[i]);
+        if (r.filled[i]) cudaEventDestroy(r.filled[i]);
+    }
+    r = Ring{};
+}
+
+// A free ring of the device, made if there is room for one; nullptr otherwise
+// (the caller then copies directly).
+Ring* take_ring(int dev) {
+    std::lock_guard<std::mutex> lock(g_rings_mu);
+    Ring* empty = nullptr;
+    for (Ring& r : g_rings) {
+        if (r.dev == dev && !r.busy) {
+            r.busy = true;
+            return &r;
+        }
+        if (r.dev < 0 && !empty) empty = &r;
+    }
+    if (!empty) return nullptr;
+    empty->dev = dev;
+    for (int i = 0; i < DOWNLOAD_SLOTS; i++)
+        if (cudaHostAlloc(&empty->slot[i], DOWNLOAD_CHUNK, cudaHostAllocDefault) != cudaSuccess ||
+            cudaEventCreateWithFlags(&empty->filled[i], cudaEventDisableTiming) != cudaSuccess) {
+            cudaGetLastError();  // not this call's failure: it has another way
+            free_ring(*empty);
+            return nullptr;
+        }
+    empty->busy = true;
+    return empty;
+}
+
+void give_back(Ring* r) {
+    std::lock_guard<std::mutex> lock(g_rings_mu);
+    r->busy = false;
+}
+
+}  // namespace
+
+int download(void* dst, const void* src, size_t bytes, cudaStream_t s, const char* what) {
+    int dev = 0;
+    IMOPS_CUDA_TRY(cudaGetDevice(&dev), "cudaGetDevice");
+    Ring* ring = nullptr;
+    cudaPointerAttributes to{}, from{};
+    if (bytes > 2 * DOWNLOAD_CHUNK && cudaPointerGetAttributes(&to, dst) == cudaSuccess &&
+        to.type == cudaMemoryTypeUnregistered && cudaPointerGetAttributes(&from, src) == cudaSuccess &&
+        from.type == cudaMemoryTypeDevice && from.device == dev)
+        ring = take_ring(dev);
+    if (!ring) {
+        IMOPS_CUDA_TRY(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s), what);
+        IMOPS_CUDA_TRY(cudaStreamSynchronize(s), "cudaStreamSynchronize");
+        return IMOPS_OK;
+    }
+    const size_t chunks = (bytes + DOWNLOAD_CHUNK - 1) / DOWNLOAD_CHUNK;
+    std::atomic<int> failed{(int)cudaSuccess};
+    auto size_of = [&](size_t c) { return c + 1 < chunks ? DOWNLOAD_CHUNK : bytes - c * DOWNLOAD_CHUNK; };
+    // slot i takes the chunks i, i + DOWNLOAD_SLOTS, ...
+    auto queue = [&](int i, size_t c) {
+        cudaError_t e = cudaMemcpyAsync(ring->slot[i], static_cast<const char*>(src) + c * DOWNLOAD_CHUNK, size_of(c),
+                                        cudaMemcpyDeviceToHost, s);
+        if (e == cudaSuccess) e = cudaEventRecord(ring->filled[i], s);
+        return e;
+    };
+    auto drain = [&](int i) {
+        cudaError_t e = cudaSetDevice(dev);  // a helper's; the caller's current device already
+        for (size_t c = i; c < chunks && e == cudaSuccess && failed.load() == (int)cudaSuccess; c += DOWNLOAD_SLOTS) {
+            if ((e = cudaEventSynchronize(ring->filled[i])) != cudaSuccess) break;
+            std::memcpy(static_cast<char*>(dst) + c * DOWNLOAD_CHUNK, ring->slot[i], size_of(c));
+            if (c + DOWNLOAD_SLOTS < chunks) e = queue(i, c + DOWNLOAD_SLOTS);
+        }
+        if (e != cudaSuccess) failed.store((int)e);
+    };
+    int queued = 0;
+    for (; queued < DOWNLOAD_SLOTS && (size_t)queued < chunks; queued++) {
+        const cudaError_t e = queue(queued, queued);
+        if (e != cudaSuccess) {
+            failed.store((int)e);
+            break;
+        }
+    }
+    std::thread helpers[DOWNLOAD_SLOTS];
+    int started = 1;  // slot 0 is this thread's
+    try {
+        for (; started < queued; started++) helpers[started] = std::thread(drain, started);
+    } catch (const std::system_error&) {
+        // no more threads: this one drains the rest
+    }
+    if (queued > 0) drain(0);
+    for (int i = started; i < queued; i++) drain(i);
+    for (int i = 1; i < started; i++) helpers[i].join();
+    // nothing of this call may still be writing to the ring
+    const cudaError_t e = cudaStreamSynchronize(s);
+    give_back(ring);
+    IMOPS_CUDA_TRY((cudaError_t)failed.load(), what);
+    IMOPS_CUDA_TRY(e, "cudaStreamSynchronize");
+    return IMOPS_OK;
+}
+
 int release_working_sets(int dev) {
     IMOPS_CUDA_TRY(cudaDeviceSynchronize(), "cudaDeviceSynchronize");
+    {
+        std::lock_guard<std::mutex> lock(g_rings_mu);
+        for (Ring& r : g_rings)
+            if (r.dev == dev && !r.busy) free_ring(r);
+    }
     std::lock_guard<std::mutex> lock(g_caches_mu);
     for (StreamCache* c : caches()) c->release_device(dev);
     return IMOPS_OK;

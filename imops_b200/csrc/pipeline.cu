@@ -979,9 +979,7 @@ extern "C" int get_image_rgb_f32_c(ImopsImage* image, float* out, size_t n_float
     if (!image->has_rgb) return fail(IMOPS_ERR_INVALID_ARGUMENT, "get_image_rgb_f32_c: the image has no RGB data");
     size_t need = image->width * image->height * 3;
     if (n_floats < need) return fail(IMOPS_ERR_INVALID_ARGUMENT, "get_image_rgb_f32_c: output buffer too small");
-    IMOPS_CUDA_TRY(cudaMemcpyAsync(out, image->rgb.p, need * 4, cudaMemcpyDeviceToHost, image->stream), "download");
-    IMOPS_CUDA_TRY(cudaStreamSynchronize(image->stream), "cudaStreamSynchronize");
-    return IMOPS_OK;
+    return download(out, image->rgb.p, need * 4, image->stream, "download");
 }
 
 namespace imops {
@@ -1021,11 +1019,9 @@ extern "C" const uint8_t* get_image_rgb_data_c(ImopsImage* image, size_t* out_wi
     pipe::to_u8_kernel<<<color::stream_grid(n, 256), 256, 0, image->stream>>>(static_cast<const float*>(image->rgb.p),
                                                                                n, static_cast<uint8_t*>(tmp.p));
     note_launch();
-    cudaError_t e = cudaMemcpyAsync(host, tmp.p, n, cudaMemcpyDeviceToHost, image->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(image->stream);
+    const int rc = download(host, tmp.p, n, image->stream, "get_image_rgb_data_c");
     pipe::buf_free(tmp, image->stream);
-    if (e != cudaSuccess) {
-        cuda_status(e, "get_image_rgb_data_c");
+    if (rc) {
         std::free(host);
         return nullptr;
     }
