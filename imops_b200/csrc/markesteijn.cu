@@ -20,6 +20,7 @@
 // allocated.  Built with --fmad=false: the same IEEE f32 operations in the
 // same order as the oracle, including its cube root (t r^2 with
 // r = t^(-1/3) by a division-free Newton iteration).
+#include "cfa_canon.cuh"
 #include "common.cuh"
 
 namespace imops {
@@ -93,7 +94,365 @@ __device__ void mean3(const Img& im, int r, int c, float* o) {
     }
 }
 
-// ---- fused tiles ---------------------------------------------------------
+// ---- X-Trans tiles ---------------------------------------------------------
+// The same method for the X-Trans pattern itself (any of its shifts), whose
+// colours are compiled in.  Tiles are 36 x 36 outputs on a 54 x 54 frame, both
+// multiples of the 6 x 6 period, and the tile grid starts where a frame's
+// origin falls on the pattern's: a frame cell's colour, neighbours and lists
+// are then the same in every tile, one table for all (Tab).
+//
+// What the pattern gives:
+//  - a green cell has two red and two blue cells in its 3 x 3 window, a red
+//    (blue) cell three blue (red) ones and none of its own colour, and each
+//    red or blue cell three green orthogonal neighbours, and greens at one or
+//    two steps on both sides along every direction;
+//  - so the red / blue step only ever reads m - G at red and blue cells.  The
+//    planes dr, db hold R - G and B - G: at red (blue) cells dr (db) is m - G,
+//    written with G by the green stages, which is what the red / blue step
+//    sums; the other entries are written by the red / blue step, which is all
+//    that the refinement reads.  R and B themselves are formed only at the
+//    end, straight into Lab;
+//  - no cell lies next to one of its own colour (red, blue) in any direction,
+//    so a refinement's writes never meet another's reads, and G, dr, db are
+//    updated in place;
+//  - the bounds of the green estimates depend on the mosaic alone: min and max
+//    of the three green neighbours are formed once a tile.
+// Each stage runs over the lists' prefixes of the cells it needs (lists are
+// ordered from the inside out).  Every value is the specification's f32
+// arithmetic in its order (a sum's leading 0 + x aside).
+//
+// Bound by instruction issue; half of it is CIELab's cube roots.  24 MP: @XT_NEW@
+// ms against 4.52 (the general tiles below: 5260 instructions an output, here
+// @XT_INST@).
+namespace aligned {
+
+using canon::XTransCanon;
+
+constexpr int T = 36;              // outputs a tile side
+constexpr int S = T + 18;          // frame side (radius 9 each way)
+constexpr int N = S * S;
+constexpr int LS = T + 4;          // Lab planes: radius 2
+constexpr int DS = T + 2;          // difference planes: radius 1
+constexpr int THREADS = 448;
+constexpr int OUT = (T * T + THREADS - 1) / THREADS;  // outputs a thread
+static_assert(T % 6 == 0 && S % 6 == 0, "every tile starts at the period's origin");
+
+__host__ __device__ constexpr int colour(int y, int x) { return XTransCanon::at((y + 6) % 6, (x + 6) % 6); }
+constexpr int depth_of(int y, int x) {
+    const int a = y < x ? y : x, b = S - 1 - (y > x ? y : x);
+    return a < b ? a : b;
+}
+// cells at least `lo` from the frame's edge
+constexpr int cells(int lo, bool green) {
+    int n = 0;
+    for (int y = lo; y < S - lo; y++)
+        for (int x = lo; x < S - lo; x++) n += (colour(y, x) == 1) == green;
+    return n;
+}
+constexpr int NN2 = cells(2, false), NN3 = cells(3, false), NN4 = cells(4, false), NN5 = cells(5, false),
+              NN6 = cells(6, false), NN7 = cells(7, false);
+constexpr int NG3 = cells(3, true), NG5 = cells(5, true), NG7 = cells(7, true);
+
+constexpr uint32_t byte_of(int v, int at) { return (uint32_t)(uint8_t)(int8_t)v << (8 * at); }
+
+// Cell lists (frame cell | phase << 12, phase = 6 (y % 6) + x % 6) and the
+// phases' facts, offsets as signed bytes in frame cells.
+struct Tab {
+    uint32_t ng[NN2], gr[NG3];
+    uint32_t phase[6 * 36];
+    // phase[p]:            green cells: offsets of the two red, then the two blue window cells
+    // phase[36 + p]:       others: offsets of the three window cells of the other colour, byte 3 the cell's own
+    // phase[72 + 36 d + p]: others, direction d: offsets of the nearest green each way, byte 2 = 0 when both are
+    //                      one step away, 1 when the one behind is two, 2 when the one ahead is
+};
+constexpr Tab make_tab() {
+    Tab t{};
+    int nn = 0, ng = 0;
+    for (int key = 7; key >= 2; key--)
+        for (int y = 2; y < S - 2; y++)
+            for (int x = 2; x < S - 2; x++) {
+                const int d = depth_of(y, x) < 7 ? depth_of(y, x) : 7;
+                if (d != key) continue;
+                const uint32_t e = (uint32_t)(y * S + x) | (uint32_t)(6 * (y % 6) + x % 6) << 12;
+                if (colour(y, x) != 1) t.ng[nn++] = e;
+                else if (key >= 3) t.gr[ng++] = e;
+            }
+    const int dy[4] = {0, 1, 1, 1}, dx[4] = {1, 0, 1, -1};
+    for (int y = 0; y < 6; y++)
+        for (int x = 0; x < 6; x++) {
+            const int p = 6 * y + x, own = colour(y, x);
+            int nr = 0, nb = 0;
+            uint32_t r = 0, b = 0;
+            for (int i = -1; i <= 1; i++)
+                for (int j = -1; j <= 1; j++) {
+                    if (i == 0 && j == 0) continue;
+                    if (colour(y + i, x + j) == 0) r |= byte_of(i * S + j, nr++);
+                    if (colour(y + i, x + j) == 2) b |= byte_of(i * S + j, nb++);
+                }
+            if (own == 1) t.phase[p] = r | b << 16;
+            else t.phase[36 + p] = (own == 0 ? b : r) | (uint32_t)own << 24;
+            if (own != 1)
+                for (int d = 0; d < 4; d++) {
+                    const int kp = colour(y + dy[d], x + dx[d]) == 1 ? 1 : 2, km = colour(y - dy[d], x - dx[d]) == 1 ? 1 : 2;
+                    const int off = dy[d] * S + dx[d];
+                    // two steps of a diagonal do not fit a byte: the kernel doubles the step
+                    t.phase[72 + 36 * d + p] = byte_of(off, 0) | (uint32_t)(kp == 2 ? 2 : (km == 2 ? 1 : 0)) << 16;
+                }
+        }
+    return t;
+}
+// What the kernel takes for granted of the pattern.
+constexpr bool pattern_ok() {
+    const int dy[4] = {0, 1, 1, 1}, dx[4] = {1, 0, 1, -1};
+    for (int y = 0; y < 6; y++)
+        for (int x = 0; x < 6; x++) {
+            const int own = colour(y, x);
+            int n[3] = {0, 0, 0}, go = 0;
+            for (int i = -1; i <= 1; i++)
+                for (int j = -1; j <= 1; j++) {
+                    if (i == 0 && j == 0) continue;
+                    n[colour(y + i, x + j)]++;
+                    if ((i == 0 || j == 0) && colour(y + i, x + j) == 1) go++;
+                }
+            if (own == 1 && (n[0] != 2 || n[2] != 2)) return false;
+            if (own != 1 && (n[own] != 0 || n[2 - own] != 3 || go != 3)) return false;
+            if (own != 1)
+                for (int d = 0; d < 4; d++) {
+                    const bool p1 = colour(y + dy[d], x + dx[d]) == 1, m1 = colour(y - dy[d], x - dx[d]) == 1;
+                    const bool p2 = colour(y + 2 * dy[d] + 6, x + 2 * dx[d] + 6) == 1,
+                               m2 = colour(y - 2 * dy[d] + 6, x - 2 * dx[d] + 6) == 1;
+                    if (!(p1 || p2) || !(m1 || m2) || (!p1 && !m1)) return false;
+                }
+        }
+    return true;
+}
+static_assert(pattern_ok(), "the X-Trans pattern's counts");
+__device__ const Tab TAB = make_tab();
+static_assert(2 * (S + 1) < 128, "two diagonal steps fit a signed byte");
+
+constexpr size_t SMEM = (size_t)(4 * N + 2 * T * T + 3 * LS * LS + 4 * DS * DS + 2 * NN2 + 6 * 36) * sizeof(float);
+static_assert(2 * (SMEM + 1024) <= 228 * 1024, "two blocks an SM");
+
+__device__ __forceinline__ int off_at(uint32_t w, int k) { return (int)(w << (24 - 8 * k)) >> 24; }
+__device__ __forceinline__ float bounded(float g, float2 lh) {
+    g = g < lh.x ? lh.x : g;
+    return g > lh.y ? lh.y : g;
+}
+
+// The colour differences at a cell of the red / blue step: green cells from
+// two cells of each colour, others from three of the other one.
+__device__ __forceinline__ void green_rb(const float* dr, const float* db, uint32_t w, int f, float g, float& R,
+                                         float& B) {
+    R = g + (dr[f + off_at(w, 0)] + dr[f + off_at(w, 1)]) * 0.5f;
+    B = g + (db[f + off_at(w, 2)] + db[f + off_at(w, 3)]) * 0.5f;
+}
+__device__ __forceinline__ float other_rb(const float* dc, uint32_t w, int f, float g) {
+    const float s = (dc[f + off_at(w, 0)] + dc[f + off_at(w, 1)]) + dc[f + off_at(w, 2)];
+    return g + s * (1.0f / 3.0f);
+}
+
+__global__ void __launch_bounds__(THREADS, 2) tile_kernel(const float* __restrict__ mosaic, int W, int H, int sx,
+                                                         int sy, float* __restrict__ out) {
+    extern __shared__ __align__(16) float fsm[];
+    float *m = fsm, *G = m + N, *dr = G + N, *db = dr + N;
+    float *k1 = db + N, *k2 = k1 + T * T;                       // the kept colours of the outputs, this direction
+    float *pL = k2 + T * T, *pa = pL + LS * LS, *pb = pa + LS * LS;
+    float* D = pb + LS * LS;
+    float2* lohi = reinterpret_cast<float2*>(D + 4 * DS * DS);  // bounds of the non-green cells, by list place
+    uint32_t* ph = reinterpret_cast<uint32_t*>(lohi + NN2);
+    const int tid = threadIdx.x;
+    const int oy = sy + blockIdx.y * T, ox = sx + blockIdx.x * T;  // first output of the tile
+    for (int i = tid; i < 6 * 36; i += THREADS) ph[i] = TAB.phase[i];
+    // frame: image rows oy-9 .. oy+T+8, clamped (cells outside the image feed
+    // only outputs outside the interior); green cells keep their sample in G
+    for (int k = tid; k < N; k += THREADS) {
+        const int y = oy - 9 + k / S, x = ox - 9 + k % S;
+        const float v = __ldg(mosaic + (size_t)min(max(y, 0), H - 1) * W + min(max(x, 0), W - 1));
+        m[k] = v;
+        G[k] = v;
+    }
+    __syncthreads();
+    for (int i = tid; i < NN2; i += THREADS) {
+        const uint32_t e = TAB.ng[i];
+        const int f = e & 4095, p = e >> 12, y = p / 6, x = p - 6 * y;
+        const int nb[4] = {f + 1, f - 1, f + S, f - S};
+        const bool ok[4] = {colour(y, x + 1) == 1, colour(y, x - 1) == 1, colour(y + 1, x) == 1, colour(y - 1, x) == 1};
+        float lo = 0.0f, hi = 0.0f;
+        bool any = false;
+#pragma unroll
+        for (int t = 0; t < 4; t++)
+            if (ok[t]) {
+                const float v = m[nb[t]];
+                lo = !any ? v : (v < lo ? v : lo);
+                hi = !any ? v : (v > hi ? v : hi);
+                any = true;
+            }
+        lohi[i] = make_float2(lo, hi);
+    }
+    // a thread's own entries of lohi are read only by itself (the same stride)
+    float keep1[4][OUT], keep2[4][OUT];
+#pragma unroll
+    for (int d = 0; d < 4; d++) {
+        const int off = d == 0 ? 1 : d == 1 ? S : d == 2 ? S + 1 : S - 1;
+        const int loff = d == 0 ? 1 : d == 1 ? LS : d == 2 ? LS + 1 : LS - 1;
+        // pass 1: green from the nearest greens along d
+        for (int i = tid; i < NN2; i += THREADS) {
+            const uint32_t e = TAB.ng[i];
+            const int f = e & 4095, p = e >> 12;
+            const int kind = ph[72 + 36 * d + p] >> 16;
+            const float a = m[f + (kind == 2 ? 2 * off : off)], b = m[f - (kind == 1 ? 2 * off : off)];
+            const float wa = kind == 1 ? 2.0f : 1.0f, wb = kind == 2 ? 2.0f : 1.0f;
+            const float r = kind == 0 ? 1.0f / 2.0f : 1.0f / 3.0f;
+            const float g = bounded((a * wa + b * wb) * r, lohi[i]);
+            G[f] = g;
+            ((ph[36 + p] >> 24) ? db : dr)[f] = m[f] - g;
+        }
+        __syncthreads();
+        auto red_blue = [&](int ng, int nn) {
+            for (int i = tid; i < ng; i += THREADS) {
+                const uint32_t e = TAB.gr[i];
+                const int f = e & 4095;
+                const float g = m[f];
+                float R, B;
+                green_rb(dr, db, ph[e >> 12], f, g, R, B);
+                dr[f] = R - g;
+                db[f] = B - g;
+            }
+            for (int i = tid; i < nn; i += THREADS) {
+                const uint32_t e = TAB.ng[i];
+                const int f = e & 4095;
+                const uint32_t w = ph[36 + (e >> 12)];
+                float* dc = (w >> 24) ? dr : db;  // the other colour
+                const float g = G[f];
+                dc[f] = other_rb(dc, w, f, g) - g;
+            }
+        };
+        auto refine = [&](int nn) {
+            for (int i = tid; i < nn; i += THREADS) {
+                const uint32_t e = TAB.ng[i];
+                const int f = e & 4095;
+                float* dc = (ph[36 + (e >> 12)] >> 24) ? db : dr;  // its own colour
+                const float k = (dc[f + off] + dc[f - off]) * 0.5f;
+                const float v = m[f], g = bounded(v - k, lohi[i]);
+                G[f] = g;
+                dc[f] = v - g;
+            }
+        };
+        red_blue(NG3, NN3);
+        __syncthreads();
+        refine(NN4);
+        __syncthreads();
+        red_blue(NG5, NN5);
+        __syncthreads();
+        refine(NN6);
+        __syncthreads();
+        // red and blue of pass 3 into CIELab, and the outputs' two colours
+        // that are not the cell's own into k1 (red, or green at red cells)
+        // and k2 (blue, or green at blue cells)
+        for (int i = tid; i < NG7 + NN7; i += THREADS) {
+            const bool green = i < NG7;
+            const uint32_t e = green ? TAB.gr[i] : TAB.ng[i - NG7];
+            const int f = e & 4095;
+            const float v = m[f], g = G[f];
+            float r, b;
+            int own = 1;
+            if (green) {
+                green_rb(dr, db, ph[e >> 12], f, g, r, b);
+            } else {
+                const uint32_t w = ph[36 + (e >> 12)];
+                own = (int)(w >> 24);
+                const float c = other_rb(own ? dr : db, w, f, g);
+                r = own ? c : v;
+                b = own ? v : c;
+            }
+            const float x = 0.4338873455660398f * r + 0.3762240091374988f * g + 0.18988864529646143f * b;
+            const float y = 0.21263900587151027f * r + 0.715168678767756f * g + 0.07219231536073371f * b;
+            const float z = 0.017750040070973232f * r + 0.10944762085523847f * g + 0.8728023390737883f * b;
+            const float fx = lab_f(x), fy = lab_f(y), fz = lab_f(z);
+            const int fr = f / S, fc = f - fr * S, l = (fr - 7) * LS + fc - 7;
+            pL[l] = 116.0f * fy - 16.0f;
+            pa[l] = 500.0f * (fx - fy);
+            pb[l] = 200.0f * (fy - fz);
+            if (fr >= 9 && fr < 9 + T && fc >= 9 && fc < 9 + T) {
+                const int o = (fr - 9) * T + fc - 9;
+                k1[o] = own == 0 ? g : r;
+                k2[o] = own == 2 ? g : b;
+            }
+        }
+        __syncthreads();
+        // the next direction's stages up to its Lab touch none of the planes
+        // read here, and there are barriers between
+#pragma unroll
+        for (int q = 0; q < OUT; q++) {
+            const int o = tid + q * THREADS;
+            if (o < T * T) {
+                keep1[d][q] = k1[o];
+                keep2[d][q] = k2[o];
+            }
+        }
+        for (int k = tid; k < DS * DS; k += THREADS) {
+            const int l = (k / DS + 1) * LS + k % DS + 1;
+            float sp = 0.0f, sm = 0.0f;
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                const float* P = c == 0 ? pL : c == 1 ? pa : pb;
+                const float v = P[l], ep = v - P[l + loff], em = v - P[l - loff];
+                sp = sp + ep * ep;
+                sm = sm + em * em;
+            }
+            D[d * DS * DS + k] = sp + sm;
+        }
+    }
+    __syncthreads();
+    // vote over the 3x3 window of the four difference planes
+#pragma unroll
+    for (int q = 0; q < OUT; q++) {
+        const int o = tid + q * THREADS, ty = o / T, tx = o - ty * T;
+        const int y = oy + ty, x = ox + tx;
+        if (o >= T * T || y < BAND || x < BAND || y >= H - BAND || x >= W - BAND) continue;
+        int hm[4] = {0, 0, 0, 0};
+#pragma unroll
+        for (int a = 0; a < 3; a++)
+#pragma unroll
+            for (int b = 0; b < 3; b++) {
+                const int j = (ty + a) * DS + tx + b;
+                float v[4];
+#pragma unroll
+                for (int d = 0; d < 4; d++) v[d] = D[d * DS * DS + j];
+                float mn = v[0];
+#pragma unroll
+                for (int d = 1; d < 4; d++) mn = v[d] < mn ? v[d] : mn;
+                const float t = 8.0f * mn;
+#pragma unroll
+                for (int d = 0; d < 4; d++) hm[d] += v[d] <= t;
+            }
+        int hx = hm[0];
+#pragma unroll
+        for (int d = 1; d < 4; d++) hx = hm[d] > hx ? hm[d] : hx;
+        const int thr = hx - hx / 8;
+        int cnt = 0;
+        float s1 = 0.0f, s2 = 0.0f;
+#pragma unroll
+        for (int d = 0; d < 4; d++) {
+            if (hm[d] < thr) continue;
+            s1 = s1 + keep1[d][q];
+            s2 = s2 + keep2[d][q];
+            cnt++;
+        }
+        const float rc = cnt == 1 ? 1.0f : cnt == 2 ? 1.0f / 2.0f : cnt == 3 ? 1.0f / 3.0f : 1.0f / 4.0f;
+        const int f = (ty + 9) * S + tx + 9;
+        const int own = colour((ty + 9) % 6, (tx + 9) % 6);
+        const float v = m[f], c1 = s1 * rc, c2 = s2 * rc;
+        float* po = out + 3 * ((size_t)y * W + x);
+        po[0] = own == 0 ? v : c1;
+        po[1] = own == 1 ? v : (own == 0 ? c1 : c2);
+        po[2] = own == 2 ? v : c2;
+    }
+}
+
+}  // namespace aligned
+
+// ---- general tiles (any other 6 x 6 CFA) -----------------------------------
 // An interior output (at least BAND from every edge) depends on inputs within
 // radius 9 only, all inside the image, so a block takes a 32 x 32 tile of
 // interior outputs and runs the whole method for it in shared memory on a
@@ -563,7 +922,17 @@ extern "C" int imops_demosaic_markesteijn3(const float* mosaic, int w, int h, co
     using xtrans::BAND;
     // interior tiles, then the band (every pixel within BAND of an edge)
     const int iw = w - 2 * BAND, ih = h - 2 * BAND;
-    if (iw > 0 && ih > 0) {
+    int cx, cy;
+    if (iw > 0 && ih > 0 && canon::canonical_offset<canon::XTransCanon>(c, &cx, &cy)) {
+        namespace A = xtrans::aligned;
+        // first output of the tile grid: at or before BAND, its frame (9 earlier) on the pattern's origin
+        const int sx = BAND - (BAND - 9 - cx + 12) % 6, sy = BAND - (BAND - 9 - cy + 12) % 6;
+        const dim3 grd((w - BAND - sx + A::T - 1) / A::T, (h - BAND - sy + A::T - 1) / A::T);
+        IMOPS_CUDA_TRY(cudaFuncSetAttribute(A::tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)A::SMEM),
+                       "cudaFuncSetAttribute(markesteijn3)");
+        A::tile_kernel<<<grd, A::THREADS, A::SMEM, s>>>(mosaic, w, h, sx, sy, rgb);
+        note_launch();
+    } else if (iw > 0 && ih > 0) {
         namespace F = xtrans::fused;
         const dim3 grd((iw + F::T - 1) / F::T, (ih + F::T - 1) / F::T);
         const F::Masks mk = F::build_masks(c);
