@@ -121,9 +121,12 @@ __device__ void mean3(const Img& im, int r, int c, float* o) {
 // ordered from the inside out).  Every value is the specification's f32
 // arithmetic in its order (a sum's leading 0 + x aside).
 //
-// Bound by instruction issue; half of it is CIELab's cube roots.  24 MP: @XT_NEW@
-// ms against 4.52 (the general tiles below: 5260 instructions an output, here
-// @XT_INST@).
+// Bound by instruction issue (0.61 of its rate; a third of the instructions
+// are CIELab's cube roots) and shared-memory latency between the barriers.
+// 24 MP: 2.07 ms against 4.52 (the general tiles below: 5260 instructions an
+// output, here 1930).  512 threads: 2.07 ms, 384 2.14, 448 2.12, 576 2.13, 672
+// 2.23; list entries read from memory in every stage instead of held in
+// registers: 2.50.
 namespace aligned {
 
 using canon::XTransCanon;
@@ -133,7 +136,7 @@ constexpr int S = T + 18;          // frame side (radius 9 each way)
 constexpr int N = S * S;
 constexpr int LS = T + 4;          // Lab planes: radius 2
 constexpr int DS = T + 2;          // difference planes: radius 1
-constexpr int THREADS = 448;
+constexpr int THREADS = 512;
 constexpr int OUT = (T * T + THREADS - 1) / THREADS;  // outputs a thread
 static_assert(T % 6 == 0 && S % 6 == 0, "every tile starts at the period's origin");
 
@@ -155,50 +158,53 @@ constexpr int NG3 = cells(3, true), NG5 = cells(5, true), NG7 = cells(7, true);
 
 constexpr uint32_t byte_of(int v, int at) { return (uint32_t)(uint8_t)(int8_t)v << (8 * at); }
 
-// Cell lists (frame cell | phase << 12, phase = 6 (y % 6) + x % 6) and the
-// phases' facts, offsets as signed bytes in frame cells.
+// Cell lists: x = frame cell, y = its window (offsets as signed bytes in frame
+// cells).
+//   green cells (gr): y: the two red, then the two blue window cells
+//   others (ng):      y: the three window cells of the other colour, byte 3 the
+//                     cell's own; x also holds, from bit 12 on, two bits a
+//                     direction: 0 when the nearest greens both ways are one
+//                     step away, 1 when the one behind is two, 2 when the one
+//                     ahead is; and from bit 20 on its green orthogonal
+//                     neighbours (0,+1) (0,-1) (+1,0) (-1,0)
+// A thread takes the entries tid, tid + THREADS, ... of each list in every stage
+// and direction, so it holds them in registers.
 struct Tab {
-    uint32_t ng[NN2], gr[NG3];
-    uint32_t phase[6 * 36];
-    // phase[p]:            green cells: offsets of the two red, then the two blue window cells
-    // phase[36 + p]:       others: offsets of the three window cells of the other colour, byte 3 the cell's own
-    // phase[72 + 36 d + p]: others, direction d: offsets of the nearest green each way, byte 2 = 0 when both are
-    //                      one step away, 1 when the one behind is two, 2 when the one ahead is
+    uint2 ng[NN2], gr[NG3];
 };
+constexpr int PN = (NN2 + THREADS - 1) / THREADS, PG = (NG3 + THREADS - 1) / THREADS;
 constexpr Tab make_tab() {
     Tab t{};
     int nn = 0, ng = 0;
+    const int dy[4] = {0, 1, 1, 1}, dx[4] = {1, 0, 1, -1};
     for (int key = 7; key >= 2; key--)
         for (int y = 2; y < S - 2; y++)
             for (int x = 2; x < S - 2; x++) {
-                const int d = depth_of(y, x) < 7 ? depth_of(y, x) : 7;
-                if (d != key) continue;
-                const uint32_t e = (uint32_t)(y * S + x) | (uint32_t)(6 * (y % 6) + x % 6) << 12;
-                if (colour(y, x) != 1) t.ng[nn++] = e;
-                else if (key >= 3) t.gr[ng++] = e;
+                const int d = depth_of(y, x) < 7 ? depth_of(y, x) : 7, own = colour(y, x);
+                if (d != key || (own == 1 && key < 3)) continue;
+                int nr = 0, nb = 0;
+                uint32_t r = 0, b = 0, cell = (uint32_t)(y * S + x);
+                for (int i = -1; i <= 1; i++)
+                    for (int j = -1; j <= 1; j++) {
+                        if (i == 0 && j == 0) continue;
+                        if (colour(y + i, x + j) == 0) r |= byte_of(i * S + j, nr++);
+                        if (colour(y + i, x + j) == 2) b |= byte_of(i * S + j, nb++);
+                    }
+                if (own == 1) {
+                    t.gr[ng].x = cell;
+                    t.gr[ng++].y = r | b << 16;
+                    continue;
+                }
+                for (int q = 0; q < 4; q++) {
+                    const bool p1 = colour(y + dy[q], x + dx[q]) == 1, m1 = colour(y - dy[q], x - dx[q]) == 1;
+                    cell |= (uint32_t)(p1 ? (m1 ? 0 : 1) : 2) << (12 + 2 * q);
+                }
+                const int oy[4] = {0, 0, 1, -1}, ox[4] = {1, -1, 0, 0};
+                for (int q = 0; q < 4; q++)
+                    if (colour(y + oy[q], x + ox[q]) == 1) cell |= 1u << (20 + q);
+                t.ng[nn].x = cell;
+                t.ng[nn++].y = (own == 0 ? b : r) | (uint32_t)own << 24;
             }
-    const int dy[4] = {0, 1, 1, 1}, dx[4] = {1, 0, 1, -1};
-    for (int y = 0; y < 6; y++)
-        for (int x = 0; x < 6; x++) {
-            const int p = 6 * y + x, own = colour(y, x);
-            int nr = 0, nb = 0;
-            uint32_t r = 0, b = 0;
-            for (int i = -1; i <= 1; i++)
-                for (int j = -1; j <= 1; j++) {
-                    if (i == 0 && j == 0) continue;
-                    if (colour(y + i, x + j) == 0) r |= byte_of(i * S + j, nr++);
-                    if (colour(y + i, x + j) == 2) b |= byte_of(i * S + j, nb++);
-                }
-            if (own == 1) t.phase[p] = r | b << 16;
-            else t.phase[36 + p] = (own == 0 ? b : r) | (uint32_t)own << 24;
-            if (own != 1)
-                for (int d = 0; d < 4; d++) {
-                    const int kp = colour(y + dy[d], x + dx[d]) == 1 ? 1 : 2, km = colour(y - dy[d], x - dx[d]) == 1 ? 1 : 2;
-                    const int off = dy[d] * S + dx[d];
-                    // two steps of a diagonal do not fit a byte: the kernel doubles the step
-                    t.phase[72 + 36 * d + p] = byte_of(off, 0) | (uint32_t)(kp == 2 ? 2 : (km == 2 ? 1 : 0)) << 16;
-                }
-        }
     return t;
 }
 // What the kernel takes for granted of the pattern.
@@ -228,9 +234,9 @@ constexpr bool pattern_ok() {
 }
 static_assert(pattern_ok(), "the X-Trans pattern's counts");
 __device__ const Tab TAB = make_tab();
-static_assert(2 * (S + 1) < 128, "two diagonal steps fit a signed byte");
+static_assert(N <= 4096 && S + 1 < 128, "a cell fits 12 bits, a window offset a signed byte");
 
-constexpr size_t SMEM = (size_t)(4 * N + 2 * T * T + 3 * LS * LS + 4 * DS * DS + 2 * NN2 + 6 * 36) * sizeof(float);
+constexpr size_t SMEM = (size_t)(4 * N + 2 * T * T + 3 * LS * LS + 4 * DS * DS + 2 * NN2) * sizeof(float);
 static_assert(2 * (SMEM + 1024) <= 228 * 1024, "two blocks an SM");
 
 __device__ __forceinline__ int off_at(uint32_t w, int k) { return (int)(w << (24 - 8 * k)) >> 24; }
@@ -259,10 +265,13 @@ __global__ void __launch_bounds__(THREADS, 2) tile_kernel(const float* __restric
     float *pL = k2 + T * T, *pa = pL + LS * LS, *pb = pa + LS * LS;
     float* D = pb + LS * LS;
     float2* lohi = reinterpret_cast<float2*>(D + 4 * DS * DS);  // bounds of the non-green cells, by list place
-    uint32_t* ph = reinterpret_cast<uint32_t*>(lohi + NN2);
     const int tid = threadIdx.x;
     const int oy = sy + blockIdx.y * T, ox = sx + blockIdx.x * T;  // first output of the tile
-    for (int i = tid; i < 6 * 36; i += THREADS) ph[i] = TAB.phase[i];
+    uint2 ng[PN], gr[PG];
+#pragma unroll
+    for (int k = 0; k < PN; k++) ng[k] = tid + k * THREADS < NN2 ? TAB.ng[tid + k * THREADS] : make_uint2(0u, 0u);
+#pragma unroll
+    for (int k = 0; k < PG; k++) gr[k] = tid + k * THREADS < NG3 ? TAB.gr[tid + k * THREADS] : make_uint2(0u, 0u);
     // frame: image rows oy-9 .. oy+T+8, clamped (cells outside the image feed
     // only outputs outside the interior); green cells keep their sample in G
     for (int k = tid; k < N; k += THREADS) {
@@ -272,22 +281,22 @@ __global__ void __launch_bounds__(THREADS, 2) tile_kernel(const float* __restric
         G[k] = v;
     }
     __syncthreads();
-    for (int i = tid; i < NN2; i += THREADS) {
-        const uint32_t e = TAB.ng[i];
-        const int f = e & 4095, p = e >> 12, y = p / 6, x = p - 6 * y;
+#pragma unroll
+    for (int k = 0; k < PN; k++) {
+        if (tid + k * THREADS >= NN2) break;
+        const int f = ng[k].x & 4095;
         const int nb[4] = {f + 1, f - 1, f + S, f - S};
-        const bool ok[4] = {colour(y, x + 1) == 1, colour(y, x - 1) == 1, colour(y + 1, x) == 1, colour(y - 1, x) == 1};
         float lo = 0.0f, hi = 0.0f;
         bool any = false;
 #pragma unroll
         for (int t = 0; t < 4; t++)
-            if (ok[t]) {
+            if ((ng[k].x >> (20 + t)) & 1u) {
                 const float v = m[nb[t]];
                 lo = !any ? v : (v < lo ? v : lo);
                 hi = !any ? v : (v > hi ? v : hi);
                 any = true;
             }
-        lohi[i] = make_float2(lo, hi);
+        lohi[tid + k * THREADS] = make_float2(lo, hi);
     }
     // a thread's own entries of lohi are read only by itself (the same stride)
     float keep1[4][OUT], keep2[4][OUT];
@@ -296,44 +305,46 @@ __global__ void __launch_bounds__(THREADS, 2) tile_kernel(const float* __restric
         const int off = d == 0 ? 1 : d == 1 ? S : d == 2 ? S + 1 : S - 1;
         const int loff = d == 0 ? 1 : d == 1 ? LS : d == 2 ? LS + 1 : LS - 1;
         // pass 1: green from the nearest greens along d
-        for (int i = tid; i < NN2; i += THREADS) {
-            const uint32_t e = TAB.ng[i];
-            const int f = e & 4095, p = e >> 12;
-            const int kind = ph[72 + 36 * d + p] >> 16;
+#pragma unroll
+        for (int k = 0; k < PN; k++) {
+            if (tid + k * THREADS >= NN2) break;
+            const int f = ng[k].x & 4095, kind = (ng[k].x >> (12 + 2 * d)) & 3;
             const float a = m[f + (kind == 2 ? 2 * off : off)], b = m[f - (kind == 1 ? 2 * off : off)];
             const float wa = kind == 1 ? 2.0f : 1.0f, wb = kind == 2 ? 2.0f : 1.0f;
             const float r = kind == 0 ? 1.0f / 2.0f : 1.0f / 3.0f;
-            const float g = bounded((a * wa + b * wb) * r, lohi[i]);
+            const float g = bounded((a * wa + b * wb) * r, lohi[tid + k * THREADS]);
             G[f] = g;
-            ((ph[36 + p] >> 24) ? db : dr)[f] = m[f] - g;
+            ((ng[k].y >> 24) ? db : dr)[f] = m[f] - g;
         }
         __syncthreads();
-        auto red_blue = [&](int ng, int nn) {
-            for (int i = tid; i < ng; i += THREADS) {
-                const uint32_t e = TAB.gr[i];
-                const int f = e & 4095;
+        auto red_blue = [&](int n_green, int n_other) {
+#pragma unroll
+            for (int k = 0; k < PG; k++) {
+                if (tid + k * THREADS >= n_green) break;
+                const int f = gr[k].x;
                 const float g = m[f];
                 float R, B;
-                green_rb(dr, db, ph[e >> 12], f, g, R, B);
+                green_rb(dr, db, gr[k].y, f, g, R, B);
                 dr[f] = R - g;
                 db[f] = B - g;
             }
-            for (int i = tid; i < nn; i += THREADS) {
-                const uint32_t e = TAB.ng[i];
-                const int f = e & 4095;
-                const uint32_t w = ph[36 + (e >> 12)];
-                float* dc = (w >> 24) ? dr : db;  // the other colour
+#pragma unroll
+            for (int k = 0; k < PN; k++) {
+                if (tid + k * THREADS >= n_other) break;
+                const int f = ng[k].x & 4095;
+                float* dc = (ng[k].y >> 24) ? dr : db;  // the other colour
                 const float g = G[f];
-                dc[f] = other_rb(dc, w, f, g) - g;
+                dc[f] = other_rb(dc, ng[k].y, f, g) - g;
             }
         };
-        auto refine = [&](int nn) {
-            for (int i = tid; i < nn; i += THREADS) {
-                const uint32_t e = TAB.ng[i];
-                const int f = e & 4095;
-                float* dc = (ph[36 + (e >> 12)] >> 24) ? db : dr;  // its own colour
-                const float k = (dc[f + off] + dc[f - off]) * 0.5f;
-                const float v = m[f], g = bounded(v - k, lohi[i]);
+        auto refine = [&](int n_other) {
+#pragma unroll
+            for (int k = 0; k < PN; k++) {
+                if (tid + k * THREADS >= n_other) break;
+                const int f = ng[k].x & 4095;
+                float* dc = (ng[k].y >> 24) ? db : dr;  // its own colour
+                const float c = (dc[f + off] + dc[f - off]) * 0.5f;
+                const float v = m[f], g = bounded(v - c, lohi[tid + k * THREADS]);
                 G[f] = g;
                 dc[f] = v - g;
             }
@@ -349,22 +360,7 @@ __global__ void __launch_bounds__(THREADS, 2) tile_kernel(const float* __restric
         // red and blue of pass 3 into CIELab, and the outputs' two colours
         // that are not the cell's own into k1 (red, or green at red cells)
         // and k2 (blue, or green at blue cells)
-        for (int i = tid; i < NG7 + NN7; i += THREADS) {
-            const bool green = i < NG7;
-            const uint32_t e = green ? TAB.gr[i] : TAB.ng[i - NG7];
-            const int f = e & 4095;
-            const float v = m[f], g = G[f];
-            float r, b;
-            int own = 1;
-            if (green) {
-                green_rb(dr, db, ph[e >> 12], f, g, r, b);
-            } else {
-                const uint32_t w = ph[36 + (e >> 12)];
-                own = (int)(w >> 24);
-                const float c = other_rb(own ? dr : db, w, f, g);
-                r = own ? c : v;
-                b = own ? v : c;
-            }
+        auto to_lab = [&](int f, int own, float r, float g, float b) {
             const float x = 0.4338873455660398f * r + 0.3762240091374988f * g + 0.18988864529646143f * b;
             const float y = 0.21263900587151027f * r + 0.715168678767756f * g + 0.07219231536073371f * b;
             const float z = 0.017750040070973232f * r + 0.10944762085523847f * g + 0.8728023390737883f * b;
@@ -378,6 +374,22 @@ __global__ void __launch_bounds__(THREADS, 2) tile_kernel(const float* __restric
                 k1[o] = own == 0 ? g : r;
                 k2[o] = own == 2 ? g : b;
             }
+        };
+#pragma unroll
+        for (int k = 0; k < PG; k++) {
+            if (tid + k * THREADS >= NG7) break;
+            const int f = gr[k].x;
+            const float g = m[f];
+            float r, b;
+            green_rb(dr, db, gr[k].y, f, g, r, b);
+            to_lab(f, 1, r, g, b);
+        }
+#pragma unroll
+        for (int k = 0; k < PN; k++) {
+            if (tid + k * THREADS >= NN7) break;
+            const int f = ng[k].x & 4095, own = (int)(ng[k].y >> 24);
+            const float v = m[f], g = G[f], c = other_rb(own ? dr : db, ng[k].y, f, g);
+            to_lab(f, own, own ? c : v, g, own ? v : c);
         }
         __syncthreads();
         // the next direction's stages up to its Lab touch none of the planes
