@@ -237,6 +237,35 @@ __device__ __forceinline__ float pow_unit(float f, float g) {
     return __uint_as_float(__float_as_uint(q) + ((uint32_t)(int)n << 23));
 }
 
+// The capture LUT (capture.rs:37-58, 91-106): entry i of layer e is the
+// developable fraction 1 - E[exp(-k s^2 phi)] at log10 phi = -4 + 12 i / 63 for
+// log-normal grain sizes s, the expectation by the trapezoid rule over 65
+// points of the normal variable, in f64: frac[e * LUTN + i].  A block a layer,
+// eight lanes an entry; bound by the latency of the f64 exponentials.  3.1 us
+// for six layers, where the same 8300 exponentials a layer took a host thread
+// 0.14 ms a layer before the first launch of every call.
+struct CaptureSpec {
+    double mu[MAXE], sigma[MAXE], k[MAXE];
+};
+__global__ void __launch_bounds__(8 * LUTN) capture_lut_kernel(const __grid_constant__ CaptureSpec c,
+                                                               float* __restrict__ frac) {
+    constexpr int PTS = 65;
+    __shared__ double weight[PTS], ks2[PTS];
+    const int e = blockIdx.x, t = threadIdx.x;
+    if (t < PTS) {
+        const double z = -8.0 + 0.25 * t, s = exp(c.mu[e] + c.sigma[e] * z);
+        weight[t] = (t == 0 || t == PTS - 1 ? 0.5 : 1.0) * 0.25 * 0.39894228040143267794 * exp(-0.5 * z * z);
+        ks2[t] = c.k[e] * s * s;
+    }
+    __syncthreads();
+    const int i = t >> 3;
+    const double phi = exp10(-4.0 + 12.0 * ((double)i / (LUTN - 1)));
+    double acc = 0.0;
+    for (int j = t & 7; j < PTS; j += 8) acc += weight[j] * exp(-ks2[j] * phi);
+    for (int o = 4; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if ((t & 7) == 0) frac[e * LUTN + i] = (float)fmin(fmax(1.0 - acc, 0.0), 1.0);
+}
+
 // Image-dye densities over the fluences in place, and the mask densities
 // (SUM: `mask` is one plane, their sum in layer order; otherwise E planes);
 // BOUNCE: the support bounce `deep` is added to the fluences first.  Bound by
@@ -245,13 +274,13 @@ __device__ __forceinline__ float pow_unit(float f, float g) {
 template <int E, bool SUM, bool BOUNCE>
 __global__ void __launch_bounds__(256) lut_reduce_kernel(float* __restrict__ planes, float* __restrict__ mask,
                                                          const float* __restrict__ deep, size_t n,
-                                                         const RefSpec* __restrict__ R,
+                                                         const float* __restrict__ frac,
                                                          const __grid_constant__ Reduce<E> c,
                                                          const __grid_constant__ Bounce bn) {
     __shared__ float2 lut[E][LUTN];
     for (int k = threadIdx.x; k < E * LUTN; k += blockDim.x) {
         const int e = k / LUTN, i = k % LUTN;
-        const float a = R->lut_frac[e][i], b = i + 1 < LUTN ? R->lut_frac[e][i + 1] : a;
+        const float a = frac[k], b = i + 1 < LUTN ? frac[k + 1] : a;
         lut[e][i] = make_float2(a, b - a);
     }
     __syncthreads();
@@ -276,15 +305,19 @@ __global__ void __launch_bounds__(256) lut_reduce_kernel(float* __restrict__ pla
     }
 }
 
-// DIR inhibition: D_j *= exp(-sum_i m[i][j] * inh_i) (diffusion.rs:39-84)
+// DIR inhibition: D_j *= exp(-sum_i m[i][j] * inh_i) (diffusion.rs:39-84),
+// for blurs wider than dir_kernel's tiles
+struct DirAny {
+    float m[MAXE][MAXE];
+};
 __global__ void dir_apply_kernel(float* __restrict__ planes, const float* __restrict__ inh, size_t n, int E,
-                                 const RefSpec* __restrict__ R) {
+                                 const __grid_constant__ DirAny dir) {
     for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < n; p += (size_t)gridDim.x * blockDim.x)
         for (int j = 0; j < E; j++) {
             float tot = 0.0f;
             bool active = false;
             for (int i = 0; i < E; i++) {
-                float w = R->dir[i][j];
+                float w = dir.m[i][j];
                 if (w != 0.0f) {
                     active = true;
                     tot += w * inh[i * n + p];
@@ -1471,8 +1504,8 @@ struct Arena {
 };
 
 size_t ref_workspace_bytes(int W, int H, int E) {
-    // planes(E) + inh(E) + mask sum(1) + tmp(1) + bounce(1) + grain partials + spec copy + sums
-    return (size_t)(2 * E + 3) * W * H * 4 + grain_partials(W, H, E) * 8 + sizeof(RefSpec) + 64 * 1024;
+    // planes(E) + inh(E) + mask sum(1) + tmp(1) + bounce(1) + grain partials + LUT + sums
+    return (size_t)(2 * E + 3) * W * H * 4 + grain_partials(W, H, E) * 8 + MAXE * LUTN * 4 + 64 * 1024;
 }
 
 // The reference model's stages (film/mod.rs:77-129), each on the stock's E
@@ -1541,9 +1574,23 @@ static Bounce bounce_gains(const RefSpec& R) {
     return b;
 }
 
+// The stock's capture LUT into lut (MAXE * LUTN floats on the device).
+int launch_capture_lut(const RefSpec& R, float* lut, cudaStream_t s) {
+    CaptureSpec c;
+    for (int e = 0; e < MAXE; e++) {
+        c.mu[e] = R.mu_ln[e];
+        c.sigma[e] = R.sigma_ln[e];
+        c.k[e] = R.capture_k[e];
+    }
+    capture_lut_kernel<<<R.E, 8 * LUTN, 0, s>>>(c, lut);
+    note_launch();
+    IMOPS_CUDA_TRY(cudaGetLastError(), "capture LUT");
+    return IMOPS_OK;
+}
+
 // The bounce (deep not NULL), the capture LUT and the reduction over the layers.
 int launch_reduce(float* planes, float* mask, bool sum, const float* deep, size_t n, const RefSpec& R,
-                  const RefSpec* dR, cudaStream_t s) {
+                  const float* lut, cudaStream_t s) {
     return with_layers(R.E, [&](auto e) {
         constexpr int E = decltype(e)::value;
         Reduce<E> c;
@@ -1556,9 +1603,9 @@ int launch_reduce(float* planes, float* mask, bool sum, const float* deep, size_
         }
         const Bounce b = bounce_gains(R);
         const int g = grid_for(n);
-        if (sum && deep) lut_reduce_kernel<E, true, true><<<g, 256, 0, s>>>(planes, mask, deep, n, dR, c, b);
-        else if (sum) lut_reduce_kernel<E, true, false><<<g, 256, 0, s>>>(planes, mask, nullptr, n, dR, c, b);
-        else lut_reduce_kernel<E, false, false><<<g, 256, 0, s>>>(planes, mask, nullptr, n, dR, c, b);
+        if (sum && deep) lut_reduce_kernel<E, true, true><<<g, 256, 0, s>>>(planes, mask, deep, n, lut, c, b);
+        else if (sum) lut_reduce_kernel<E, true, false><<<g, 256, 0, s>>>(planes, mask, nullptr, n, lut, c, b);
+        else lut_reduce_kernel<E, false, false><<<g, 256, 0, s>>>(planes, mask, nullptr, n, lut, c, b);
         note_launch();
         return IMOPS_OK;
     });
@@ -1600,15 +1647,15 @@ int stage_adjacency(float* planes, int W, int H, const RefSpec& R, float* tmp, c
 //     `deep` (or NULL) is added first.  With result NULL the densities end
 //     up in planes; otherwise in *result (planes or inh), without the
 //     adjacency, which print_scan adds.
-int stage_develop(float* planes, float* mask, bool sum, const float* deep, int W, int H, const Stock& st, const RefSpec* dR, float* inh,
-                  float* tmp, float** result, cudaStream_t s) {
+int stage_develop(float* planes, float* mask, bool sum, const float* deep, int W, int H, const Stock& st,
+                  const float* lut, float* inh, float* tmp, float** result, cudaStream_t s) {
     const RefSpec& R = st.ref;
     const int E = R.E;
     const size_t n = (size_t)W * H;
     const int g = grid_for(n);
     Taps tp;
     int rc;
-    if ((rc = launch_reduce(planes, mask, sum, deep, n, R, dR, s))) return rc;
+    if ((rc = launch_reduce(planes, mask, sum, deep, n, R, lut, s))) return rc;
     if (result) *result = planes;
     if (R.dir_any && R.sigma_dir >= 1e-3f) {
         if ((rc = taps_for(R.sigma_dir, &tp))) return rc;
@@ -1627,7 +1674,10 @@ int stage_develop(float* planes, float* mask, bool sum, const float* deep, int W
             // sub-stage takes (their wide bounce is above 64 px)
             for (int i = 0; i < E; i++)
                 if ((rc = blur(planes + i * n, tmp, W, H, tp, EpiStore{inh + i * n}, s))) return rc;
-            dir_apply_kernel<<<g, 256, 0, s>>>(planes, inh, n, E, dR);
+            DirAny any;
+            for (int i = 0; i < MAXE; i++)
+                for (int j = 0; j < MAXE; j++) any.m[i][j] = R.dir[i][j];
+            dir_apply_kernel<<<g, 256, 0, s>>>(planes, inh, n, E, any);
             note_launch();
         }
     }
@@ -1724,7 +1774,7 @@ int print_scan(float* dens, const float* mask, const float* noise, const double*
 // The reference model's kernels on rgb in place, inverted with the reference
 // points mid_dmin unless that is NULL.
 int run_reference(float* rgb, int W, int H, const Stock& st, uint64_t seed, int grain, const float* mid_dmin, Arena& A,
-                  const RefSpec* dR, cudaStream_t s) {
+                  const float* lut, cudaStream_t s) {
     const int E = st.ref.E;
     const size_t n = (size_t)W * H;
     float* planes = A.take<float>(E * n);
@@ -1738,7 +1788,7 @@ int run_reference(float* rgb, int W, int H, const Stock& st, uint64_t seed, int 
     float *deep = nullptr, *dens = nullptr;
     if ((rc = expose_scatter(rgb, W, H, st, planes, tmp, s))) return rc;
     if ((rc = stage_bounce(planes, W, H, st.ref, tmp, bounce, &deep, s))) return rc;
-    if ((rc = stage_develop(planes, mask, true, deep, W, H, st, dR, inh, tmp, &dens, s))) return rc;
+    if ((rc = stage_develop(planes, mask, true, deep, W, H, st, lut, inh, tmp, &dens, s))) return rc;
     // the other set of planes is free after develop: it takes the grain fields
     float* noise = grain ? (dens == planes ? inh : planes) : nullptr;
     if (grain && (rc = stage_grain_fields(W, H, st.ref, seed, noise, partial, sums, s))) return rc;
@@ -1751,14 +1801,14 @@ int run_reference(float* rgb, int W, int H, const Stock& st, uint64_t seed, int 
 // a 32x32 mid-grey patch through the same path (seed 0) into mid_dmin[0..2]
 // and the stock's normalised Dmin into mid_dmin[3..5].  Takes
 // ref_workspace_bytes(32, 32, E) + 1024 * 12 bytes of A.
-int mid_gray_negative(const Stock& st, int grain, Arena& A, const RefSpec* dR, float* mid_dmin, cudaStream_t s) {
+int mid_gray_negative(const Stock& st, int grain, Arena& A, const float* lut, float* mid_dmin, cudaStream_t s) {
     const size_t nm = 32 * 32;
     float g = relative_to_absolute_y(0.185f, st.ref.box_iso);
     std::vector<float> patch(nm * 3, g);
     float* dpatch = A.take<float>(nm * 3);
     IMOPS_CUDA_TRY(cudaMemcpyAsync(dpatch, patch.data(), nm * 12, cudaMemcpyHostToDevice, s), "copy patch");
     int rc;
-    if ((rc = run_reference(dpatch, 32, 32, st, 0, grain, nullptr, A, dR, s))) return rc;
+    if ((rc = run_reference(dpatch, 32, 32, st, 0, grain, nullptr, A, lut, s))) return rc;
     mean_rgb_kernel<<<1, 256, 0, s>>>(dpatch, (int)nm, mid_dmin);
     note_launch();
     IMOPS_CUDA_TRY(cudaMemcpyAsync(mid_dmin + 3, st.ref.dmin_norm, 12, cudaMemcpyHostToDevice, s), "copy dmin");
@@ -1776,20 +1826,19 @@ int process_reference(float* rgb, int W, int H, const ImopsFilmParams& P, cudaSt
     void* ws = nullptr;
     if ((rc = workspace(s, bytes, &ws))) return rc;
     Arena A{static_cast<char*>(ws), 0};
-    RefSpec* dR = A.take<RefSpec>(1);
+    float* lut = A.take<float>(MAXE * LUTN);
     float* mid_dmin = A.take<float>(8);
-    IMOPS_CUDA_TRY(cudaMemcpyAsync(dR, &st.ref, sizeof(RefSpec), cudaMemcpyHostToDevice, s), "copy spec");
+    if ((rc = launch_capture_lut(st.ref, lut, s))) return rc;
     bool positive = P.output == IMOPS_FILM_POSITIVE_LINEAR && !st.ref.any_reversal;
-    if (positive && (rc = mid_gray_negative(st, P.grain, A, dR, mid_dmin, s))) return rc;
-    return run_reference(rgb, W, H, st, P.seed, P.grain, positive ? mid_dmin : nullptr, A, dR, s);
+    if (positive && (rc = mid_gray_negative(st, P.grain, A, lut, mid_dmin, s))) return rc;
+    return run_reference(rgb, W, H, st, P.seed, P.grain, positive ? mid_dmin : nullptr, A, lut, s);
 }
 
-// One sub-stage call: the stock (reference model only), device copies of its
-// specs and an arena of `extra` bytes in the film workspace.
+// One sub-stage call: the stock (reference model only) and an arena of `extra` bytes in the film workspace.
 struct StageCtx {
     Stock st;
     Arena A;
-    RefSpec* dR;
+    float* lut;  // the capture LUT's place (launch_capture_lut fills it)
 };
 
 int stage_ctx(const ImopsFilmParams* P, int W, int H, size_t extra, cudaStream_t s, StageCtx* c) {
@@ -1801,10 +1850,9 @@ int stage_ctx(const ImopsFilmParams* P, int W, int H, size_t extra, cudaStream_t
     if (c->st.model != MODEL_REFERENCE)
         return fail(IMOPS_ERR_INVALID_STOCK, "film stages: the baseline preset runs only whole (imops_film_process)");
     void* ws = nullptr;
-    if ((rc = workspace(s, sizeof(RefSpec) + extra + 4096, &ws))) return rc;
+    if ((rc = workspace(s, MAXE * LUTN * sizeof(float) + extra + 4096, &ws))) return rc;
     c->A = Arena{static_cast<char*>(ws), 0};
-    c->dR = c->A.take<RefSpec>(1);
-    IMOPS_CUDA_TRY(cudaMemcpyAsync(c->dR, &c->st.ref, sizeof(RefSpec), cudaMemcpyHostToDevice, s), "copy spec");
+    c->lut = c->A.take<float>(MAXE * LUTN);
     return IMOPS_OK;
 }
 
@@ -2001,7 +2049,8 @@ extern "C" int imops_film_develop(float* planes, float* mask, int w, int h, cons
     if (!planes || !mask) return fail(IMOPS_ERR_INVALID_ARGUMENT, "film_develop: NULL buffer");
     float* inh = c.A.take<float>((size_t)c.st.ref.E * n);
     float* tmp = c.A.take<float>(n);
-    if ((rc = film::stage_develop(planes, mask, false, nullptr, w, h, c.st, c.dR, inh, tmp, nullptr, s))) return rc;
+    if ((rc = film::launch_capture_lut(c.st.ref, c.lut, s))) return rc;
+    if ((rc = film::stage_develop(planes, mask, false, nullptr, w, h, c.st, c.lut, inh, tmp, nullptr, s))) return rc;
     IMOPS_CUDA_TRY(cudaGetLastError(), "film_develop");
     return IMOPS_OK;
 }
@@ -2048,7 +2097,8 @@ extern "C" int imops_film_invert(float* rgb, int w, int h, const ImopsFilmParams
     if (!rgb) return fail(IMOPS_ERR_INVALID_ARGUMENT, "film_invert: NULL buffer");
     if (!(params->output == IMOPS_FILM_POSITIVE_LINEAR && !c.st.ref.any_reversal)) return IMOPS_OK;
     float* mid_dmin = c.A.take<float>(8);
-    if ((rc = film::mid_gray_negative(c.st, params->grain, c.A, c.dR, mid_dmin, s))) return rc;
+    if ((rc = film::launch_capture_lut(c.st.ref, c.lut, s))) return rc;
+    if ((rc = film::mid_gray_negative(c.st, params->grain, c.A, c.lut, mid_dmin, s))) return rc;
     const size_t n = (size_t)w * h;
     film::invert_kernel<<<film::grid_for(n), 256, 0, s>>>(rgb, n, mid_dmin);
     note_launch();

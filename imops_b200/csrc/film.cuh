@@ -54,7 +54,7 @@ struct RefSpec {
     float hal_gain[MAXE];
     // capture LUT + reciprocity (capture.rs:61-88, exposure/mod.rs:97-115)
     float eta[MAXE];
-    float lut_frac[MAXE][LUTN];
+    double mu_ln[MAXE], sigma_ln[MAXE], capture_k[MAXE];  // of the grain sizes and the capture LUT
     // reduce (reduction.rs:16-68)
     float dmax[MAXE], inv_gamma[MAXE], mask_scale[MAXE];
     int reversal[MAXE], has_mask[MAXE];

@@ -3,7 +3,7 @@
 // for spectral quantities) and handed to the kernels as f32 tables.
 //
 // Stocks follow pichromatic/src/film/stock/{color_neg_200.rs, bw_stub.rs};
-// the LUT, kappa and scan constants follow stock/mod.rs:152-214,
+// the kappa and scan constants follow stock/mod.rs:152-214,
 // exposure/capture.rs:37-110, film/scan/densitometry.rs:13-117.
 #include <cmath>
 #include <cstring>
@@ -263,24 +263,6 @@ void spectrum_to_ap1_16(const double* s, double out[3]) {
     for (int i = 0; i < 3; i++) out[i] = XYZ2AP1[i][0] * xyz[0] + XYZ2AP1[i][1] * xyz[1] + XYZ2AP1[i][2] * xyz[2];
 }
 
-// E_s[exp(-k s^2 phi)] (capture.rs:91-106)
-double expected_survival(double mu, double sig, double k, double phi) {
-    const int N = 64;
-    const double ZMAX = 8.0;
-    double dz = (2.0 * ZMAX) / (double)N;
-    double isq = 1.0 / std::sqrt(2.0 * PI);
-    double acc = 0.0;
-    for (int i = 0; i <= N; i++) {
-        double z = -ZMAX + (double)i * dz;
-        double tw = (i == 0 || i == N) ? 0.5 : 1.0;
-        double pdf = isq * std::exp(-0.5 * z * z);
-        double s = std::exp(mu + sig * z);
-        double g = std::exp(-k * s * s * phi);
-        acc += tw * pdf * g * dz;
-    }
-    return acc;
-}
-
 double curve_integrate(const std::vector<double>& s) {
     double acc = 0.0;
     for (int i = 0; i < NB16 - 1; i++) acc += 0.5 * (s[i] + s[i + 1]) * 20.0;
@@ -419,14 +401,9 @@ int build_reference(const StockDef& sd, int W, float shutter, Stock* st, float* 
         double p = (double)L.recip_p, t = (double)shutter;
         double eta = (t <= 1.0 || p >= 0.9999) ? 1.0 : std::pow(t > 1.0 ? t : 1.0, p - 1.0);
         R.eta[e] = (float)eta;
-        for (int i = 0; i < LUTN; i++) {
-            double tt = (double)i / 63.0;
-            double lp = -4.0 + tt * (8.0 - -4.0);
-            double ph = std::pow(10.0, lp);
-            double f = 1.0 - expected_survival(L.mu_ln, L.sigma_ln, L.capture_k, ph);
-            f = f < 0.0 ? 0.0 : (f > 1.0 ? 1.0 : f);
-            R.lut_frac[e][i] = (float)f;
-        }
+        R.mu_ln[e] = L.mu_ln;
+        R.sigma_ln[e] = L.sigma_ln;
+        R.capture_k[e] = L.capture_k;
         R.dmax[e] = L.dmax;
         float gam = L.gamma > 1e-6f ? L.gamma : 1e-6f;
         R.inv_gamma[e] = 1.0f / gam;

@@ -105,3 +105,19 @@ def test_grain_fields_match_the_generator(gpu, stock, H, W):
         assert scale > 0
         assert np.abs(got - scale * n).max() < 1e-5 * np.abs(got).max() + 1.2e-7
         assert abs(got.std() / out[e].std() - 1) < 0.05
+
+
+@pytest.mark.parametrize("stock", STOCKS)
+@pytest.mark.parametrize("output", [0, 1])
+def test_capture_over_twelve_decades_matches_oracle(oracle_lib, gpu, stock, output):
+    """Steps of exposure from below the capture LUT's first entry to above its
+    last, so that every entry of every layer is read (and the ends clamp)."""
+    import torch
+
+    import imops_b200 as im
+    steps = np.repeat(10.0 ** np.linspace(-7, 7, 141), 4)
+    x = np.broadcast_to(steps[None, :, None], (9, steps.size, 3)).astype(np.float32).copy()
+    ref = oracle_lib.film_process(x, stock=stock, seed=3, output=output, grain=False, precision="f32")
+    out = im.film_process(torch.from_numpy(x).to(gpu), stock=stock, seed=3, output=output, grain=False).cpu().numpy()
+    assert np.isfinite(out).all()
+    assert np.abs(out - ref).max() < TOL
