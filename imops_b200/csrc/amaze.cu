@@ -222,10 +222,9 @@ __device__ void fill(const P& p, const Geo& g, float* mos) {
                   [&](int rr, int cc) { return get_in(p, H - rr - 2, 32 - cc); });
 }
 
-// Loop helpers: every site of rows [r0,r1) x cols [c0,c1), and the R/B
-// sites of those rows (first R/B column = c0 + parity of the row; c0 even).
-// Threads map to (row group, column) directly: a tile row has at most 128
-// sites and 64 R/B sites, so no integer division is needed.
+// Loop helpers: every site of rows [r0,r1) x cols [c0,c1).  Threads map to
+// (row group, column) directly: a tile row has at most 128 sites, so no
+// integer division is needed.
 template <class F>
 __device__ __forceinline__ void for_rect(int r0, int r1, int c0, int c1, F f) {
     const int cc = c0 + (int)(threadIdx.x & (TS - 1));
@@ -233,16 +232,8 @@ __device__ __forceinline__ void for_rect(int r0, int r1, int c0, int c1, F f) {
     for (int rr = r0 + (int)(threadIdx.x / TS); rr < r1; rr += NTHREADS / TS) f(rr, cc);
 }
 
-template <class F, class P>
-__device__ __forceinline__ void for_rb(const P& p, const Geo& g, int r0, int r1, int c0, int c1, F f) {
-    const int k = (int)(threadIdx.x & (TSH - 1));
-    for (int rr = r0 + (int)(threadIdx.x / TSH); rr < r1; rr += NTHREADS / TSH) {
-        int cc = c0 + (p.cfa.at(g.top + rr, g.left + 2) & 1) + 2 * k;
-        if (cc < c1) f(rr, cc);
-    }
-}
-
-// The same sites dense over the block's threads: thread t takes sites t,
+// The same sites, and the R/B sites of those rows (first R/B column = c0 +
+// parity of the row; c0 even), dense over the block's threads: thread t takes sites t,
 // t + NTHREADS, ... in row-major order, so no lane idles at a row's end (the
 // inner stages' rows are 96-112 sites of 128, or 50-56 R/B sites of 64); the
 // row and column advance without a division.  Bayer rows alternate the
@@ -889,22 +880,62 @@ __device__ NyqBox st_nyq_test(const P& p, const Geo& g, const Bufs& b, int* sh) 
 
 // demosaic.rs:873-947: majority vote inside the box, then the area-based
 // weight at voted sites: sums over the voted sites of the 7 x 7 same-colour
-// window, in row-major order.  A thread takes four sites of a column (rows 2
-// apart), whose windows share most of their rows: a window sample's terms are
-// formed once and added to the sums of every site that has it in its window,
-// each site's sums still in their own order.  On frames full of such texture
-// the site-by-site form took up to a third of the kernel (6 MP, such a frame: 1.18 ms, now 1.05, with 24 warps 0.99).
-constexpr int NYQ_SITES = 4;
+// window, in row-major order.
+//
+// The vote is a count of eight neighbours' flags, over a whole row's mask at
+// once: a thread a row adds the neighbours' masks in bit planes.  The
+// neighbours of pair k two rows away are pair k, those one row away pairs
+// k-1, k (site in the even column) or k, k+1 (odd), those of the row k +- 1.
+//
+// The sums: a thread takes NYQ_SITES sites of a column (rows 2 apart), whose
+// windows share most of their rows: a window sample's terms are formed once
+// and added to the sums of every site that has it in its window, each site's
+// sums still in their own order.  The horizontal and vertical terms go in
+// pairs (f32x2, each half rounded as by itself), and so do the plain sums of
+// two sites.  Bound by issue.  Five sites: a full box is 1344 columns of
+// sites, two a thread at most, where four sites make 1568, three for one
+// warp, which then ran its third alone.  Two columns a thread as well (5 x 2
+// sites) save 1% on such frames and cost 3% on others (spills elsewhere).
+// A 6 MP frame full of such texture: 1.11 ms with four sites' scalar sums and
+// a vote site by site, 0.89 ms now, with st_nyquist_green's share; a frame
+// with little: 0.65 ms.
+constexpr int NYQ_SITES = 5;
+
+// bits of x + y + z per position: sum and carry
+__device__ __forceinline__ void full_add(unsigned long long x, unsigned long long y, unsigned long long z,
+                                         unsigned long long& sum, unsigned long long& carry) {
+    sum = x ^ y ^ z;
+    carry = (x & y) | (z & (x ^ y));
+}
+
 template <class P>
 __device__ void st_nyquist_area(const P& p, const Geo& g, const Bufs& b, const NyqBox& box) {
     const float epssq = 1e-10f;
-    for_rb(p, g, box.r0, box.r1, box.c0, box.c1, [&](int rr, int cc) {
-        int i = rr * TS + cc;
-        const unsigned long long* n = b.nyqw;
-        unsigned s = rbflag(n, i - V2) + rbflag(n, i - M1) + rbflag(n, i - P1) + rbflag(n, i - 2) + rbflag(n, i + 2) +
-                     rbflag(n, i + P1) + rbflag(n, i + M1) + rbflag(n, i + V2);
-        if (s > 4 || (s == 4 && rbflag(n, i))) rbflag_set(b.nyq2w, i);
-    });
+    if ((int)threadIdx.x < box.r1 - box.r0 && box.c1 > box.c0) {
+        typedef unsigned long long u64;
+        const int row = box.r0 + threadIdx.x;
+        const int par = p.cfa.at(g.top + row, g.left + 2) & 1;  // the row's R/B sites: columns 2 k + par
+        const u64* n = b.nyqw + row;
+        const u64 up = n[-1], dn = n[1], self = n[0];
+        u64 s0, c0, s1, c1, s2, c2, s3, c3, c4, c5;
+        full_add(n[-2], n[2], up, s0, c0);
+        full_add(par ? up >> 1 : up << 1, dn, par ? dn >> 1 : dn << 1, s1, c1);
+        full_add(self << 1, self >> 1, s0, s2, c2);
+        s3 = s1 ^ s2;             // ones
+        c3 = s1 & s2;
+        u64 twos, fours, x, y;
+        full_add(c0, c1, c2, x, c4);
+        twos = x ^ c3;
+        c5 = x & c3;
+        fours = c4 ^ c5;          // 4 .. 7
+        y = c4 & c5;              // 8
+        // more than four, or four and flagged itself
+        u64 v = y | (fours & (twos | s3 | self));
+        // pairs whose site lies in [c0, c1)
+        const int k0 = (box.c0 - par + 1) >> 1, k1 = (box.c1 - par + 1) >> 1;
+        v &= (k1 >= 64 ? ~0ull : (1ull << k1) - 1ull) & (~0ull << k0);
+        b.nyq2w[row] = v;
+    }
     __syncthreads();
     const int w = (box.c1 - box.c0 + 1) >> 1, rows = box.r1 - box.r0;
     if (w <= 0 || rows <= 0) return;
@@ -919,11 +950,13 @@ __device__ void st_nyquist_area(const P& p, const Geo& g, const Bufs& b, const N
         for (int s = 0; s < NYQ_SITES; s++)
             if (rr + 2 * s < box.r1 && rbflag(b.nyq2w, (rr + 2 * s) * TS + cc)) voted |= 1u << s;
         if (!voted) continue;
-        float cfa[NYQ_SITES], sh[NYQ_SITES], sv[NYQ_SITES], qh[NYQ_SITES], qv[NYQ_SITES];
+        // per site: (horizontal, vertical) sums of the neighbour pairs and of
+        // the squared differences; the plain sums of sites 2j, 2j+1
+        float2 sn[NYQ_SITES], sd[NYQ_SITES], sc[(NYQ_SITES + 1) / 2];
         int cnt[NYQ_SITES];
 #pragma unroll
         for (int s = 0; s < NYQ_SITES; s++) {
-            cfa[s] = sh[s] = sv[s] = qh[s] = qv[s] = 0.0f;
+            sn[s] = sd[s] = sc[s >> 1] = make_float2(0.0f, 0.0f);
             cnt[s] = 0;
         }
         // window rows rr - 6 .. rr + 2 NYQ_SITES + 4; row k belongs to the
@@ -935,32 +968,46 @@ __device__ void st_nyquist_area(const P& p, const Geo& g, const Bufs& b, const N
             if (!(voted & sites)) continue;
             const int row = rr - 6 + 2 * k;
             unsigned bits = (unsigned)(b.nyq2w[row] >> ((cc >> 1) - 3)) & 127u;
+            const int pc = __popc(bits);
 #pragma unroll
             for (int s = 0; s < NYQ_SITES; s++)
-                if ((sites >> s) & 1u) cnt[s] += __popc(bits);
+                if ((sites >> s) & 1u) cnt[s] += pc;
             const float* m = b.mos + row * TS + cc - 6;
+            float l = m[-1];
+#pragma unroll 1
             for (; bits; bits >>= 1, m += 2) {
-                if (!(bits & 1u)) continue;
-                const float v = m[0], l = m[-1], r = m[1], u = m[-V1], d = m[V1];
-                const float h2 = l + r, v2 = u + d;
-                const float dh = sqr(v - l) + sqr(v - r), dv = sqr(v - u) + sqr(v - d);
+                const float r = m[1];
+                if (bits & 1u) {
+                    const float v = m[0];
+                    const float2 a = make_float2(l, m[-V1]), c = make_float2(r, m[V1]);
+                    const float2 nb = __fadd2_rn(a, c);
+                    const float2 nv = make_float2(-v, -v), da = __fadd2_rn(a, nv), dc = __fadd2_rn(c, nv);
+                    // scalar squares: a packed product may contract into the packed sum
+                    const float2 sq = __fadd2_rn(make_float2(sqr(da.x), sqr(da.y)), make_float2(sqr(dc.x), sqr(dc.y)));
 #pragma unroll
-                for (int s = 0; s < NYQ_SITES; s++)
-                    if ((sites >> s) & 1u) {
-                        cfa[s] += v;
-                        sh[s] += h2;
-                        sv[s] += v2;
-                        qh[s] += dh;
-                        qv[s] += dv;
+                    for (int s = 0; s < NYQ_SITES; s++)
+                        if ((sites >> s) & 1u) {
+                            sn[s] = __fadd2_rn(sn[s], nb);
+                            sd[s] = __fadd2_rn(sd[s], sq);
+                        }
+#pragma unroll
+                    for (int j = 0; j < (NYQ_SITES + 1) / 2; j++) {
+                        const unsigned two = (sites >> (2 * j)) & 3u;
+                        if (two == 3u) sc[j] = __fadd2_rn(sc[j], make_float2(v, v));
+                        if (two == 1u) sc[j].x += v;
+                        if (two == 2u) sc[j].y += v;
                     }
+                }
+                l = r;
             }
         }
 #pragma unroll
         for (int s = 0; s < NYQ_SITES; s++) {
             if (!((voted >> s) & 1u)) continue;
-            const float sumh = cfa[s] - sh[s] * 0.5f, sumv = cfa[s] - sv[s] * 0.5f, area = (float)cnt[s] * 0.5f;
-            const float hvar = epssq + fabsf(area * qh[s] - sumh * sumh);
-            const float vvar = epssq + fabsf(area * qv[s] - sumv * sumv);
+            const float cfa = s & 1 ? sc[s >> 1].y : sc[s >> 1].x;
+            const float sumh = cfa - sn[s].x * 0.5f, sumv = cfa - sn[s].y * 0.5f, area = (float)cnt[s] * 0.5f;
+            const float hvar = epssq + fabsf(area * sd[s].x - sumh * sumh);
+            const float vvar = epssq + fabsf(area * sd[s].y - sumv * sumv);
             b.hvwt[((rr + 2 * s) * TS + cc) >> 1] = hvar / (vvar + hvar);
         }
     }
@@ -991,56 +1038,69 @@ __device__ void st_green_rb(const P& p, const Geo& g, const Bufs& b) {
 // demosaic.rs:978-998.  dgrb2h/v of a voted site j are
 // (rgbgreen_j - mean of its horizontal / vertical green neighbours)^2 with
 // rgbgreen_j = mos_j + the colour difference st_green_rb forms at j, and
-// zero at the other sites.  New values are computed by all sites first and stored after a
-// barrier, so every site reads the pre-update dgrb0.
-
+// zero at the other sites.  Each is formed once, by its site's thread, and
+// kept where the site's weight and vcd were (hvwt, vcd_rb), which wait in
+// that thread's registers; after a barrier each voted site takes its 13 taps
+// from there, and after another puts the weight back beside the new dgrb0.
 template <class P>
 __device__ void st_nyquist_green(const P& p, const Geo& g, const Bufs& b, const NyqBox& box) {
     const float epssq = 1e-10f;
     const float q0 = 0.169917f, q1 = 0.108947f, q2 = 0.069855f, q3 = 0.0287182f;
     const float* m = b.mos;
-    auto d2 = [&](int j, float& h, float& v) {
-        if (!rbflag(b.nyq2w, j)) {
-            h = v = 0.0f;
-            return;
-        }
-        // j is voted: its colour difference as st_green_rb forms it (not
-        // stored there for voted sites)
-        const float wt = b.hvwt[j >> 1];
-        const float gr = m[j] + (wt * b.vcd_rb[j >> 1] + (1.0f - wt) * b.hcd_rb[j >> 1]);
-        h = sqr(gr - (m[j - 1] + m[j + 1]) * 0.5f);
-        v = sqr(gr - (m[j - V1] + m[j + V1]) * 0.5f);
-    };
-    float nd[RB_PER_THREAD];
+    float wt[RB_PER_THREAD], nd[RB_PER_THREAD];  // nd: vcd, then the new dgrb0
     const int n = (box.r1 - box.r0) * TSH;
+    // slot s's site: column and flat index, when it is a voted one
+    auto site = [&](int s, int& cc, int& i) {
+        const int k = (int)threadIdx.x + s * NTHREADS;
+        if (k >= n) return false;
+        const int rr = box.r0 + (k >> 6);
+        cc = box.c0 + (p.cfa.at(g.top + rr, g.left + 2) & 1) + 2 * (k & (TSH - 1));
+        i = rr * TS + cc;
+        return cc < box.c1 && rbflag(b.nyq2w, i);
+    };
 #pragma unroll
     for (int s = 0; s < RB_PER_THREAD; s++) {
-        const int k = (int)threadIdx.x + s * NTHREADS;
-        nd[s] = 0.0f;
-        if (k >= n) continue;
-        const int rr = box.r0 + (k >> 6);
-        const int cc = box.c0 + (p.cfa.at(g.top + rr, g.left + 2) & 1) + 2 * (k & (TSH - 1));
-        const int i = rr * TS + cc;
-        if (cc >= box.c1 || !rbflag(b.nyq2w, i)) continue;
-        float h[13], v[13];
-        const int off[13] = {0, -M1, -P1, P1, M1, -V2, -2, 2, V2, -M2, -P2, P2, M2};
-#pragma unroll
-        for (int t = 0; t < 13; t++) d2(i + off[t], h[t], v[t]);
-        const float gvarh = epssq + (q0 * h[0] + q1 * (h[1] + h[2] + h[3] + h[4]) + q2 * (h[5] + h[6] + h[7] + h[8]) +
-                                     q3 * (h[9] + h[10] + h[11] + h[12]));
-        const float gvarv = epssq + (q0 * v[0] + q1 * (v[1] + v[2] + v[3] + v[4]) + q2 * (v[5] + v[6] + v[7] + v[8]) +
-                                     q3 * (v[9] + v[10] + v[11] + v[12]));
-        nd[s] = (b.hcd_rb[i >> 1] * gvarv + b.vcd_rb[i >> 1] * gvarh) / (gvarv + gvarh);
+        int cc, i;
+        wt[s] = nd[s] = 0.0f;
+        if (!site(s, cc, i)) continue;
+        wt[s] = b.hvwt[i >> 1];
+        nd[s] = b.vcd_rb[i >> 1];
+        const float gr = m[i] + (wt[s] * nd[s] + (1.0f - wt[s]) * b.hcd_rb[i >> 1]);
+        b.hvwt[i >> 1] = sqr(gr - (m[i - 1] + m[i + 1]) * 0.5f);
+        b.vcd_rb[i >> 1] = sqr(gr - (m[i - V1] + m[i + V1]) * 0.5f);
     }
     __syncthreads();
 #pragma unroll
     for (int s = 0; s < RB_PER_THREAD; s++) {
-        const int k = (int)threadIdx.x + s * NTHREADS;
-        if (k >= n) continue;
-        const int rr = box.r0 + (k >> 6);
-        const int cc = box.c0 + (p.cfa.at(g.top + rr, g.left + 2) & 1) + 2 * (k & (TSH - 1));
-        const int i = rr * TS + cc;
-        if (cc < box.c1 && rbflag(b.nyq2w, i)) b.dgrb0[i >> 1] = nd[s];
+        int cc, i;
+        if (!site(s, cc, i)) continue;
+        const unsigned long long* f = b.nyq2w + (i >> 7);
+        // flags of the pairs about the column: three of the even rows, two of the odd ones
+        const int ke = (cc >> 1) - 1, ko = (cc - 1) >> 1;
+        const unsigned f0 = (unsigned)(f[-2] >> ke), f1 = (unsigned)(f[-1] >> ko), f2 = (unsigned)(f[0] >> ke),
+                       f3 = (unsigned)(f[1] >> ko), f4 = (unsigned)(f[2] >> ke);
+        auto d2 = [&](int o, unsigned flag) {  // (dgrb2h, dgrb2v) of the site at i + o
+            const int h = (i + o) >> 1;
+            return flag ? make_float2(b.hvwt[h], b.vcd_rb[h]) : make_float2(0.0f, 0.0f);
+        };
+        auto four = [&](float2 x, float2 y, float2 z, float2 w) {
+            return __fadd2_rn(__fadd2_rn(__fadd2_rn(x, y), z), w);
+        };
+        const float2 t0 = d2(0, f2 & 2u);
+        const float2 t1 = four(d2(-M1, f1 & 1u), d2(-P1, f1 & 2u), d2(P1, f3 & 1u), d2(M1, f3 & 2u));
+        const float2 t2 = four(d2(-V2, f0 & 2u), d2(-2, f2 & 1u), d2(2, f2 & 4u), d2(V2, f4 & 2u));
+        const float2 t3 = four(d2(-M2, f0 & 1u), d2(-P2, f0 & 4u), d2(P2, f4 & 1u), d2(M2, f4 & 4u));
+        const float gvarh = epssq + (q0 * t0.x + q1 * t1.x + q2 * t2.x + q3 * t3.x);
+        const float gvarv = epssq + (q0 * t0.y + q1 * t1.y + q2 * t2.y + q3 * t3.y);
+        nd[s] = (b.hcd_rb[i >> 1] * gvarv + nd[s] * gvarh) / (gvarv + gvarh);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int s = 0; s < RB_PER_THREAD; s++) {
+        int cc, i;
+        if (!site(s, cc, i)) continue;
+        b.dgrb0[i >> 1] = nd[s];
+        b.hvwt[i >> 1] = wt[s];
     }
 }
 
