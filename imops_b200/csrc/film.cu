@@ -356,13 +356,13 @@ __global__ void dir_apply_kernel(float* __restrict__ planes, const float* __rest
 // an SM.  Tiles are 128 wide and TH high, their runs a whole number of
 // rounds of the 512 threads where that fits two blocks an SM: 39 rows for up
 // to three layers (96 KB), 24 for six (113 KB).  Six layers in one block mix
-// 13.25 draws a pixel, two blocks of three 25.  Images of fewer tiles than two an
-// SM take tiles of 18 rows, so that the few blocks finish sooner (1.1 MP: 36
-// us against 44).  24 MP: three layers 0.44 ms (0.57 with f32 sums of draws
-// converted one by one), six layers 0.61 ms (2.55 one layer a launch).
+// 13.25 draws a pixel, two blocks of three 25; with fewer than two tiles of
+// 39 rows an SM the layers go three at a time, in the tile height that fills
+// the SMs best (grain_rows).  24 MP: three layers 0.44 ms (0.57 with f32 sums
+// of draws converted one by one), six layers 0.61 ms (2.55 one layer a launch).
 constexpr int GR_TW = 128, GR_MAXR = 16, GR_RUN = 4;
 constexpr int GR_THREADS = 512, GR_GROUPS = GR_THREADS / GR_TW;
-constexpr int GR_TH = 39, GR_TH6 = 24, GR_TH_SMALL = 18;
+constexpr int GR_TH = 39, GR_TH6 = 24;
 static_assert(GR_TW == 128, "the blur loops index tile columns with & 127");
 // output rows a thread, and rows of the row-blurred buffer: the last group's
 // window reaches past the tile's halo where TH is not a multiple of the groups
@@ -543,15 +543,39 @@ __global__ void __launch_bounds__(1024) sum_partials_kernel(const double* __rest
     if (threadIdx.x == 0) sums[blockIdx.x] = red[0];
 }
 
-// Fewer tiles of full height than two an SM: the low tiles.
-static bool grain_small(int W, int H) {
-    return (size_t)((W + GR_TW - 1) / GR_TW) * ((H + GR_TH - 1) / GR_TH) < (size_t)sm_count() * 2;
+static size_t grain_tiles(int W, int H, int th) {
+    return (size_t)((W + GR_TW - 1) / GR_TW) * ((H + th - 1) / th);
+}
+
+// Fewer tiles of full height than two an SM: no six layers to a block.
+static bool grain_small(int W, int H) { return grain_tiles(W, H, GR_TH) < (size_t)sm_count() * 2; }
+
+// Tile height of the blocks of up to three layers.  A block alone on its SM
+// takes 4.9 + 0.38 TH us, two at once 1.7 times that, and of more each takes
+// 0.65 of it after a run-in (fitted to 13 sizes from 32x32 to 24 MP at seven
+// heights): the height of the least of that.  39 from about 2 MP on; below,
+// 9 against 39 rows: 324x216 8.3 us against 19.3; 640x480, 18 rows: 11.7
+// against 19.9; 1200x800, 28 rows: 27.0 against 33.3; 1296x864, 34 rows: 31.6
+// against 34.0.
+static int grain_rows(int W, int H) {
+    const int heights[] = {GR_TH, 34, 28, 18, 9};
+    int best = GR_TH;
+    double least = 0.0;
+    for (int th : heights) {
+        const double per_sm = (double)grain_tiles(W, H, th) / sm_count();
+        const double cost = (4.9 + 0.38 * th) * (per_sm <= 1.0 ? 1.0 : per_sm <= 2.0 ? 1.7 : 0.6 + 0.65 * per_sm);
+        if (th == GR_TH || cost < least) {
+            least = cost;
+            best = th;
+        }
+    }
+    return best;
 }
 
 // Doubles of scratch that grain_fields needs for its block sums.
 size_t grain_partials(int W, int H, int layers) {
-    const int th = grain_small(W, H) ? GR_TH_SMALL : (layers >= 6 ? GR_TH6 : GR_TH);
-    return (size_t)((W + GR_TW - 1) / GR_TW) * ((H + th - 1) / th) * layers;
+    const int th = grain_rows(W, H);
+    return grain_tiles(W, H, layers >= 6 && !grain_small(W, H) && GR_TH6 < th ? GR_TH6 : th) * layers;
 }
 
 template <int LAYERS, int TH>
@@ -569,6 +593,18 @@ static int grain_launch(float* noise, int W, int H, uint64_t seed, int layer0, c
     return IMOPS_OK;
 }
 
+template <int LAYERS>
+static int grain_launch_rows(int th, float* noise, int W, int H, uint64_t seed, int layer0, const Taps& tp,
+                             double* partial, double* sums, cudaStream_t s) {
+    switch (th) {
+        case 9: return grain_launch<LAYERS, 9>(noise, W, H, seed, layer0, tp, partial, sums, s);
+        case 18: return grain_launch<LAYERS, 18>(noise, W, H, seed, layer0, tp, partial, sums, s);
+        case 28: return grain_launch<LAYERS, 28>(noise, W, H, seed, layer0, tp, partial, sums, s);
+        case 34: return grain_launch<LAYERS, 34>(noise, W, H, seed, layer0, tp, partial, sums, s);
+        default: return grain_launch<LAYERS, GR_TH>(noise, W, H, seed, layer0, tp, partial, sums, s);
+    }
+}
+
 // Blurred grain fields of RNG layers layer0 .. layer0+layers-1 (planes
 // noise[z * n]) and their sums of squares sums[z].  partial: scratch of
 // grain_partials(W, H, layers) doubles.
@@ -577,6 +613,7 @@ int grain_fields(float* noise, int W, int H, uint64_t seed, int layer0, int laye
     if (tp.R > GR_MAXR) return fail(IMOPS_ERR_UNSUPPORTED_SIZE, "film: grain blur radius above 16 px");
     const size_t n = (size_t)W * H;
     const bool small = grain_small(W, H);
+    const int th = grain_rows(W, H);
     for (int z = 0; z < layers;) {
         int rc, take;
         float* nz = noise + z * n;
@@ -586,14 +623,13 @@ int grain_fields(float* noise, int W, int H, uint64_t seed, int layer0, int laye
             rc = grain_launch<6, GR_TH6>(nz, W, H, seed, l0, tp, partial, sums + z, s);
         } else if (left >= 3) {
             take = 3;
-            rc = small ? grain_launch<3, GR_TH_SMALL>(nz, W, H, seed, l0, tp, partial, sums + z, s)
-                       : grain_launch<3, GR_TH>(nz, W, H, seed, l0, tp, partial, sums + z, s);
+            rc = grain_launch_rows<3>(th, nz, W, H, seed, l0, tp, partial, sums + z, s);
         } else if (left == 2) {
             take = 2;
-            rc = grain_launch<2, GR_TH>(nz, W, H, seed, l0, tp, partial, sums + z, s);
+            rc = grain_launch_rows<2>(th, nz, W, H, seed, l0, tp, partial, sums + z, s);
         } else {
             take = 1;
-            rc = grain_launch<1, GR_TH>(nz, W, H, seed, l0, tp, partial, sums + z, s);
+            rc = grain_launch_rows<1>(th, nz, W, H, seed, l0, tp, partial, sums + z, s);
         }
         if (rc) return rc;
         z += take;
@@ -953,23 +989,30 @@ struct Base81 {
     float2 tap2[2 * HAL_R + 2];
 };
 
-// One thread per 16 consecutive rows of a column: the halation column pass
+// One thread per OUT consecutive rows of a column: the halation column pass
 // (register sliding window, tap pairs as parameter-bank operands, ascending
 // tap order as in blur_cols), then per pixel the exposure of the three layers
 // from its RGB, the logistic curves, grain and the 81-bin scan with its
 // tables as parameter-bank operands; the result replaces the pixel's RGB
 // (each pixel is read, a step ahead, and written by the same thread).  Four
 // blocks an SM (64 registers a thread): the scan is bound by the MUFU, and
-// 32 warps keep more of its exponentials in flight than 24.
+// 32 warps keep more of its exponentials in flight than 24.  Sixteen rows a
+// thread; four where the blocks of sixteen would be fewer than three an SM,
+// which leaves SMs short of warps and the busiest with twice the mean work:
+// 640x480 29.6 -> 19.6 us, 1200x800 45.3 -> 37.8, 1536x1024 (2.6 blocks an SM)
+// 58.9 -> 55.4, but 2048x1365 (4.8) 87.2 -> 90.6 and 6048x4024 626 -> 725 (the
+// window's run-in, 128 rows for 32 instead of 128).
+constexpr int SCAN_OUT_SMALL = 4;
+template <int OUT>
 __global__ void __launch_bounds__(R64_COL_TW * R64_COL_GROUPS, 4) scan81_fused_kernel(
     const float* __restrict__ hr, const float* __restrict__ noise, const double* __restrict__ sumsq, int W, int H,
     const __grid_constant__ Base81 c, float* __restrict__ rgb) {
     static_assert(HAL_R == R64, "the fused scan's column pass is the radius-64 window");
-    static_assert(R64_COL_OUT % 2 == 0, "column outputs go in pairs");
-    __shared__ float s[(R64_COL_TH + 2 * HAL_R) * R64_COL_TW];
-    const int x0 = blockIdx.x * R64_COL_TW, y0 = blockIdx.y * R64_COL_TH;
+    static_assert(OUT % 2 == 0, "column outputs go in pairs");
+    __shared__ float s[((R64_COL_GROUPS * OUT) + 2 * HAL_R) * R64_COL_TW];
+    const int x0 = blockIdx.x * R64_COL_TW, y0 = blockIdx.y * (R64_COL_GROUPS * OUT);
     const int tx = threadIdx.x, ty = threadIdx.y, x = x0 + tx;
-    if (x < W) stage_col_window<R64_COL_TH>(s, hr, W, H, x, y0, tx, ty);
+    if (x < W) stage_col_window<(R64_COL_GROUPS * OUT)>(s, hr, W, H, x, y0, tx, ty);
     __syncthreads();
     if (x >= W) return;
     const size_t n = (size_t)W * H;
@@ -979,18 +1022,18 @@ __global__ void __launch_bounds__(R64_COL_TW * R64_COL_GROUPS, 4) scan81_fused_k
             double var = sumsq[e] / (double)n;
             norm[e] = var > 1e-12 ? (float)(1.0 / sqrt(var)) : 1.0f;
         }
-    const int rb = ty * R64_COL_OUT;
+    const int rb = ty * OUT;
     // bs[q] = (output row 2q, output row 2q+1); at window row m the pair takes
     // taps m-2q and m-2q-1
-    float2 bs[R64_COL_OUT / 2];
+    float2 bs[OUT / 2];
 #pragma unroll
-    for (int q = 0; q < R64_COL_OUT / 2; q++) bs[q] = make_float2(0.0f, 0.0f);
+    for (int q = 0; q < OUT / 2; q++) bs[q] = make_float2(0.0f, 0.0f);
 #pragma unroll
-    for (int m = 0; m < R64_COL_OUT + 2 * HAL_R; m++) {
+    for (int m = 0; m < OUT + 2 * HAL_R; m++) {
         const float v = s[(rb + m) * R64_COL_TW + tx];
         const float2 vv = make_float2(v, v);
 #pragma unroll
-        for (int q = 0; q < R64_COL_OUT / 2; q++) {
+        for (int q = 0; q < OUT / 2; q++) {
             const int k = m - 2 * q;
             if (k >= 0 && k <= 2 * HAL_R + 1) bs[q] = __ffma2_rn(vv, c.tap2[k], bs[q]);
         }
@@ -999,7 +1042,7 @@ __global__ void __launch_bounds__(R64_COL_TW * R64_COL_GROUPS, 4) scan81_fused_k
     // fetched once for both, and the next step's RGB and noise are loaded
     // while this step is scanned, so the global-load latency hides behind
     // the 81-bin loop.  Each pixel's arithmetic is unchanged.
-    static_assert(R64_COL_OUT % 2 == 0, "pixels go in pairs");
+    static_assert(OUT % 2 == 0, "pixels go in pairs");
     const bool grain = c.B.grain_sigma > 0.0f;
     float na[2][3], nz[2][3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
     auto fetch = [&](int jj) {  // rows jj, jj+1 (clamped to the image)
@@ -1015,7 +1058,7 @@ __global__ void __launch_bounds__(R64_COL_TW * R64_COL_GROUPS, 4) scan81_fused_k
     };
     fetch(0);
 #pragma unroll 1
-    for (int j = 0; j < R64_COL_OUT; j += 2) {
+    for (int j = 0; j < OUT; j += 2) {
         const int y = y0 + rb + j;
         if (y >= H) break;
         float ca[2][3], cz[2][3];
@@ -1029,10 +1072,10 @@ __global__ void __launch_bounds__(R64_COL_TW * R64_COL_GROUPS, 4) scan81_fused_k
                 cz[u][e] = nz[u][e];
             }
         }
-        if (j + 2 < R64_COL_OUT && y + 2 < H) fetch(j + 2);
+        if (j + 2 < OUT && y + 2 < H) fetch(j + 2);
         float bsum[2] = {bs[0].x, bs[0].y};
 #pragma unroll
-        for (int q = 0; q < R64_COL_OUT / 2; q++)
+        for (int q = 0; q < OUT / 2; q++)
             if (2 * q == j) {
                 bsum[0] = bs[q].x;
                 bsum[1] = bs[q].y;
@@ -1973,7 +2016,12 @@ int baseline_forward_in(float* rgb, int W, int H, const ImopsBaselineFilm& P, co
                        "cudaFuncSetAttribute(tensor-core scan)");
         scan81_tc_kernel<<<cg, cb, tc::SMEM_REQ, s>>>(hr, noise, sums, W, H, tp, rgb);
     } else {
-        scan81_fused_kernel<<<cg, cb, 0, s>>>(hr, noise, sums, W, H, hp, rgb);
+        if ((long)cg.x * cg.y < 3L * sm_count()) {
+            cg.y = (H + R64_COL_GROUPS * SCAN_OUT_SMALL - 1) / (R64_COL_GROUPS * SCAN_OUT_SMALL);
+            scan81_fused_kernel<SCAN_OUT_SMALL><<<cg, cb, 0, s>>>(hr, noise, sums, W, H, hp, rgb);
+        } else {
+            scan81_fused_kernel<R64_COL_OUT><<<cg, cb, 0, s>>>(hr, noise, sums, W, H, hp, rgb);
+        }
     }
     note_launch();
     IMOPS_CUDA_TRY(cudaGetLastError(), "baseline film kernels");

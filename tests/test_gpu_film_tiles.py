@@ -78,11 +78,14 @@ def _noise_rows(seed, layer, y0, y1, W):
     return acc - 6.0
 
 
-@pytest.mark.parametrize("stock,H,W", [(2, 1500, 2100), (4, 1500, 2100), (1, 1500, 2100), (1, 300, 517), (6, 300, 517)])
+@pytest.mark.parametrize("stock,H,W", [(2, 1500, 2100), (4, 1500, 2100), (1, 1500, 2100), (1, 300, 517), (6, 300, 517),
+                                       (0, 216, 324), (1, 216, 324), (1, 480, 640), (6, 480, 640), (0, 800, 1200),
+                                       (1, 800, 1200), (6, 864, 1296), (1, 864, 1296), (1, 683, 1024)])
 def test_grain_fields_match_the_generator(gpu, stock, H, W):
     """The grain added to flat planes, against the generator in 64 bits, over
     rows that cross tile edges, for one block of six layers (2), six and one
-    (4), three (1), the low tiles of small images, and two layers (6).  Up to
+    (4), three (1), two layers (6) and one (0), and every height of the tiles
+    that smaller images take.  Up to
     the layer's amplitude the added densities are the blurred noise.  Error: two
     f32 roundings of an output below 0.5 (6e-8 each), and 1e-5 of the
     grain for the rounding of its blur and scale."""
@@ -120,4 +123,17 @@ def test_capture_over_twelve_decades_matches_oracle(oracle_lib, gpu, stock, outp
     ref = oracle_lib.film_process(x, stock=stock, seed=3, output=output, grain=False, precision="f32")
     out = im.film_process(torch.from_numpy(x).to(gpu), stock=stock, seed=3, output=output, grain=False).cpu().numpy()
     assert np.isfinite(out).all()
+    assert np.abs(out - ref).max() < TOL
+
+
+@pytest.mark.parametrize("H,W", [(1, 1), (5, 33), (31, 65), (33, 64), (97, 1200), (800, 1200), (1024, 1536), (1100, 1536)])
+def test_preset_scan_matches_oracle_on_both_sides_of_its_block_rule(oracle_lib, gpu, H, W):
+    """The 81-band preset with four rows a thread (few blocks) and sixteen."""
+    import torch
+
+    import imops_b200 as im
+    x = (np.random.default_rng(H + W).random((H, W, 3)) ** 2).astype(np.float32)
+    ref = oracle_lib.film_baseline(x, oracle_lib.baseline_params(grain_on=1, seed=9), precision="f64")
+    out = im.film_process(torch.from_numpy(x).to(gpu), stock=im.STOCK_BASELINE81,
+                          baseline=im.baseline_film_defaults(grain_on=1, seed=9)).cpu().numpy()
     assert np.abs(out - ref).max() < TOL
