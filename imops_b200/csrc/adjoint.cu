@@ -555,29 +555,63 @@ __global__ void __launch_bounds__(CD_THREADS, 2) cols_dual_t_kernel(const float*
     }
 }
 
-// The transposes' end terms of the two radius-64 column blurs of g (rows within
-// 64 of an end): G's added to t3 and, as the products are linear, both to the
-// inner products, in partial[block].  A block has 32 columns, the warps of its
-// CE_SPLIT blocks the rows.
-constexpr int CE_SPLIT = 4;
+// The transposes' end terms (film::transpose_end) of the two radius-64 column
+// blurs of g: G's added to t3 and, as the products are linear, both to the
+// inner products, in partial[block].  A block has 32 columns of an end; a warp
+// takes eight of the 64 distances, each sample once for both blurs and for its
+// own row's term and the end row's sum.  Bound by latency: every load is in
+// flight at once.  2.8 MP: 3.5 us (24 MP: 5.6), where a thread a row, the end rows' 64
+// samples one thread's, took 11.4 us (16.4).  With H <= 129 rows the ends share rows and one
+// block takes both, one after the other.
 __global__ void __launch_bounds__(BLK) cols_ends_kernel(const float* __restrict__ g, int W, int H,
                                                         const __grid_constant__ DualTaps tp,
                                                         const float* __restrict__ t1, const float* __restrict__ t2,
                                                         float* __restrict__ t3, double* __restrict__ partial) {
     using film::R64;
-    const int x = blockIdx.x * 32 + (threadIdx.x & 31);
+    constexpr int WARPS = BLK / 32, PER = R64 / WARPS;
+    static_assert(WARPS * PER == R64, "the warps share the distances evenly");
+    __shared__ float2 red[WARPS][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, x = blockIdx.x * 32 + lane;
     float acc[1] = {0.0f};
-    if (x < W)
-        for (int r = blockIdx.y * (BLK / 32) + (threadIdx.x >> 5); r < 2 * R64 + 2; r += CE_SPLIT * (BLK / 32)) {
-            const int y = r <= R64 ? r : H - 1 - (r - R64 - 1);
-            if (r > R64 && y <= R64) continue;  // the first end's row adds both ends' terms
-            auto line = [&](int i) { return __ldg(g + (size_t)i * W + x); };
-            const float ea = film::transpose_end(y, H, R64, 0.0f, line, [&](int k) { return tp.t[k]; });
-            const float ed = film::transpose_end(y, H, R64, 0.0f, line, [&](int k) { return tp.d[k]; });
-            const size_t p = (size_t)y * W + x;
-            t3[p] += ea;
-            acc[0] = fmaf(ea, t2[p], fmaf(ed, t1[p], acc[0]));
+    for (int end = blockIdx.y; end < 2; end += gridDim.y) {
+        const int y0 = end ? H - 1 : 0, dir = end ? -W : W;
+        const size_t p0 = (size_t)y0 * W + x;
+        float sa = 0.0f, sd = 0.0f;
+        if (x < W) {
+            const float ge = __ldg(g + p0);
+            float v[PER], u1[PER], u2[PER], u3[PER];
+#pragma unroll
+            for (int i = 0; i < PER; i++) {
+                const ptrdiff_t p = (ptrdiff_t)p0 + (ptrdiff_t)(1 + w * PER + i) * dir;
+                v[i] = __ldg(g + p);
+                u1[i] = __ldg(t1 + p);
+                u2[i] = __ldg(t2 + p);
+                u3[i] = t3[p];
+            }
+#pragma unroll
+            for (int i = 0; i < PER; i++) {
+                const int k = 1 + w * PER + i;
+                const float ta = tp.t[R64 - k], td = tp.d[R64 - k], ea = ta * ge, ed = td * ge;
+                sa = fmaf(ta, v[i], sa);
+                sd = fmaf(td, v[i], sd);
+                t3[(ptrdiff_t)p0 + (ptrdiff_t)k * dir] = u3[i] + ea;
+                acc[0] = fmaf(ea, u2[i], fmaf(ed, u1[i], acc[0]));
+            }
         }
+        red[w][lane] = make_float2(sa, sd);
+        __syncthreads();
+        if (w == 0 && x < W) {
+            sa = sd = 0.0f;
+#pragma unroll
+            for (int i = 0; i < WARPS; i++) {
+                sa += red[i][lane].x;
+                sd += red[i][lane].y;
+            }
+            t3[p0] -= sa;
+            acc[0] -= fmaf(sa, t2[p0], sd * t1[p0]);
+        }
+        __syncthreads();
+    }
     block_partials(acc, partial);
 }
 
@@ -797,7 +831,7 @@ int prepare(const float* x, int W, int H, const ImopsFilmGradParams* P, const Im
     b->chunks = film::stream_chunks(W, H, sm_count());
     b->cols_grid = dim3((W + film::R64_COL_TW - 1) / film::R64_COL_TW,
                         (H + b->chunks * film::SC_SLAB - 1) / (b->chunks * film::SC_SLAB));
-    const size_t ns = std::max((size_t)b->cols_grid.x * (b->cols_grid.y + CE_SPLIT), (size_t)b->nb);
+    const size_t ns = std::max((size_t)b->cols_grid.x * (b->cols_grid.y + 2), (size_t)b->nb);
     const size_t nh = std::max((size_t)b->rows_grid.x * b->rows_grid.y, (size_t)b->nb);
     const size_t bytes = (backward ? 5 : 3) * (n * 4 + 256) + (b->nb1 * NP1 + nh * NPH + ns) * 8 + 8192;
     void* ws = nullptr;
@@ -845,8 +879,9 @@ int backward_halation(Bufs& b, const float* x, int W, int H, int* nbh, int* nbs,
     if (b.R == film::R64) {
         cols_dual_t_kernel<<<b.cols_grid, CD_THREADS, 0, s>>>(b.gB, W, H, b.chunks, dual_taps(b), b.t1, b.t2, b.t3, b.ps);
         const int nb = (int)(b.cols_grid.x * b.cols_grid.y);
-        cols_ends_kernel<<<dim3(b.cols_grid.x, CE_SPLIT), BLK, 0, s>>>(b.gB, W, H, dual_taps(b), b.t1, b.t2, b.t3, b.ps + nb);
-        *nbs = nb + (int)b.cols_grid.x * CE_SPLIT;
+        const int ends = H > 2 * film::R64 + 1 ? 2 : 1;
+        cols_ends_kernel<<<dim3(b.cols_grid.x, ends), BLK, 0, s>>>(b.gB, W, H, dual_taps(b), b.t1, b.t2, b.t3, b.ps + nb);
+        *nbs = nb + (int)b.cols_grid.x * ends;
         rows_t_color_kernel<<<b.rows_grid, film::R64_ROW_THREADS, 0, s>>>(b.t3, x, W, H, film::pair_taps(b.tp), b.src,
                                                                           b.ph);
         *nbh = (int)(b.rows_grid.x * b.rows_grid.y);
