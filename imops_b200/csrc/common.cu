@@ -207,7 +207,7 @@ int download(void* dst, const void* src, size_t bytes, cudaStream_t s, const cha
     IMOPS_CUDA_TRY(cudaGetDevice(&dev), "cudaGetDevice");
     Ring* ring = nullptr;
     cudaPointerAttributes to{}, from{};
-    if (bytes > 2 * DOWNLOAD_CHUNK && cudaPointerGetAttributes(&to, dst) == cudaSuccess &&
+    if (bytes > DOWNLOAD_LEAST && cudaPointerGetAttributes(&to, dst) == cudaSuccess &&
         to.type == cudaMemoryTypeUnregistered && cudaPointerGetAttributes(&from, src) == cudaSuccess &&
         from.type == cudaMemoryTypeDevice && from.device == dev)
         ring = take_ring(dev);

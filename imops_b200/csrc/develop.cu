@@ -1,5 +1,6 @@
-// develop.cu -- the fused forward of the path: demosaic (scaling fused into
-// its tile load, WB / exposure / camera CST fused into its output stage),
+// develop.cu -- the fused forward of the path: demosaic (WB / exposure /
+// camera CST fused into its output stage; the 3x3 mean of a Bayer or X-Trans
+// frame scales the u16 samples as it loads them, AMaZE takes a scaled mosaic),
 // then the film simulation.  Same results as the stage entry points run in
 // the reference's module order (pipeline.rs:4-13).
 #include <mutex>

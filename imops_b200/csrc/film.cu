@@ -1,13 +1,15 @@
 // film.cu -- spectral film simulation kernels and imops_film_process.
 //
 // Reference model (film::process, pichromatic/src/film/mod.rs:77-129) as a
-// chain of planar kernels:
-//   expose (rank-3 spectral collapse) -> local scatter -> support bounce ->
-//   capture LUT -> reduce -> DIR -> adjacency -> grain -> 16-bin scan ->
-//   [invert].
-// Baseline preset (81 bins): expose + halation source -> halation row pass
-// -> grain noise -> one fused kernel doing the halation column pass, the
-// logistic curves, grain and the 81-bin scan.
+// chain of planar kernels, in brackets what one kernel does:
+//   [expose (rank-3 spectral collapse) -> local scatter] -> blur of the
+//   support's plane -> [bounce -> capture LUT -> reduce] -> [DIR blur and
+//   inhibition] -> grain fields -> [adjacency -> grain -> 16-bin scan ->
+//   invert].
+// Blurs too wide for the tiles (film_tiles.cuh) run as passes of their own.
+// Baseline preset (81 bins): halation row pass (its source formed from the
+// RGB) beside the grain fields -> one fused kernel doing the exposure, the
+// halation column pass, the logistic curves, grain and the 81-bin scan.
 //
 // Layout: per-layer planes (row-major f32), so every pass is a coalesced
 // stream; RGB stays interleaved as in Image.rgb_data.

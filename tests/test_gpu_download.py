@@ -17,7 +17,8 @@ def _image(h, w, seed):
 
 
 @pytest.mark.parametrize("h,w", [(100, 100), (1, 2 * CHUNK // 12), (1, 2 * CHUNK // 12 + 1), (3, CHUNK // 12 + 5),
-                                 (512, 2048), (1365, 2049), (2011, 3001)])
+                                 (512, 2048), (1, 8 * CHUNK // 12), (1, 8 * CHUNK // 12 + 1), (3, 3 * CHUNK // 12 + 5),
+                                 (1365, 2049), (2011, 3001)])
 def test_round_trip(gpu, h, w):
     import imops_b200 as im
     from imops_b200.pipeline import Image
@@ -37,7 +38,7 @@ def test_threads_and_pinned(gpu):
 
     import imops_b200 as im
     from imops_b200.pipeline import Image
-    xs = [_image(700 + 3 * k, 2000 + k, seed=k) for k in range(6)]  # more at once than there are rings
+    xs = [_image(1400 + 3 * k, 2000 + k, seed=k) for k in range(6)]  # more at once than there are rings
     imgs = [Image.from_rgb(x, im.CS_ACESCG) for x in xs]
     bad = []
 
