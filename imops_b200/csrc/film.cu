@@ -948,8 +948,14 @@ __global__ void __launch_bounds__(EX_THREADS, 2) expose_scatter_kernel(const flo
     }
 }
 
-// mean RGB of a small buffer in f64 (invert.rs:111-125), one block
-__global__ void mean_rgb_kernel(const float* __restrict__ rgb, int n, float* __restrict__ out) {
+__global__ void fill_kernel(float* __restrict__ p, int n, float v) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) p[i] = v;
+}
+
+// mean RGB of a small buffer in f64 (invert.rs:111-125) into out[0..2], dmin into out[3..5]; one block
+__global__ void mean_rgb_kernel(const float* __restrict__ rgb, int n, float dmin0, float dmin1, float dmin2,
+                                float* __restrict__ out) {
     __shared__ double s[3][256];
     double a[3] = {0, 0, 0};
     for (int p = threadIdx.x; p < n; p += blockDim.x)
@@ -962,7 +968,12 @@ __global__ void mean_rgb_kernel(const float* __restrict__ rgb, int n, float* __r
         __syncthreads();
     }
     if (threadIdx.x == 0)
+    {
         for (int c = 0; c < 3; c++) out[c] = (float)(s[c][0] / (double)n);
+        out[3] = dmin0;
+        out[4] = dmin1;
+        out[5] = dmin2;
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -1817,9 +1828,10 @@ int print_scan(float* dens, const float* mask, const float* noise, const double*
 }
 
 // The reference model's kernels on rgb in place, inverted with the reference
-// points mid_dmin unless that is NULL.
+// points mid_dmin unless that is NULL; those are waited for on `ready` where
+// another stream forms them.
 int run_reference(float* rgb, int W, int H, const Stock& st, uint64_t seed, int grain, const float* mid_dmin, Arena& A,
-                  const float* lut, cudaStream_t s) {
+                  const float* lut, cudaStream_t s, cudaEvent_t ready = nullptr) {
     const int E = st.ref.E;
     const size_t n = (size_t)W * H;
     float* planes = A.take<float>(E * n);
@@ -1837,6 +1849,7 @@ int run_reference(float* rgb, int W, int H, const Stock& st, uint64_t seed, int 
     // the other set of planes is free after develop: it takes the grain fields
     float* noise = grain ? (dens == planes ? inh : planes) : nullptr;
     if (grain && (rc = stage_grain_fields(W, H, st.ref, seed, noise, partial, sums, s))) return rc;
+    if (ready) IMOPS_CUDA_TRY(cudaStreamWaitEvent(s, ready, 0), "cudaStreamWaitEvent(mid grey)");
     if ((rc = print_scan(dens, mask, noise, sums, mid_dmin, W, H, st, tmp, rgb, s))) return rc;
     IMOPS_CUDA_TRY(cudaGetLastError(), "film kernels");
     return IMOPS_OK;
@@ -1849,15 +1862,83 @@ int run_reference(float* rgb, int W, int H, const Stock& st, uint64_t seed, int 
 int mid_gray_negative(const Stock& st, int grain, Arena& A, const float* lut, float* mid_dmin, cudaStream_t s) {
     const size_t nm = 32 * 32;
     float g = relative_to_absolute_y(0.185f, st.ref.box_iso);
-    std::vector<float> patch(nm * 3, g);
     float* dpatch = A.take<float>(nm * 3);
-    IMOPS_CUDA_TRY(cudaMemcpyAsync(dpatch, patch.data(), nm * 12, cudaMemcpyHostToDevice, s), "copy patch");
+    fill_kernel<<<12, 256, 0, s>>>(dpatch, (int)nm * 3, g);
+    note_launch();
     int rc;
     if ((rc = run_reference(dpatch, 32, 32, st, 0, grain, nullptr, A, lut, s))) return rc;
-    mean_rgb_kernel<<<1, 256, 0, s>>>(dpatch, (int)nm, mid_dmin);
+    mean_rgb_kernel<<<1, 256, 0, s>>>(dpatch, (int)nm, st.ref.dmin_norm[0], st.ref.dmin_norm[1], st.ref.dmin_norm[2],
+                                      mid_dmin);
     note_launch();
-    IMOPS_CUDA_TRY(cudaMemcpyAsync(mid_dmin + 3, st.ref.dmin_norm, 12, cudaMemcpyHostToDevice, s), "copy dmin");
+    IMOPS_CUDA_TRY(cudaGetLastError(), "film mid-grey patch");
     return IMOPS_OK;
+}
+
+// A second stream per device for work that does not depend on the image (the
+// preset's grain fields, a positive's mid-grey patch), forked from and joined
+// back to the caller's stream with events: it then runs beside the kernels
+// before its result is needed.
+struct SideStream {
+    bool init = false;
+    cudaStream_t side = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
+};
+std::mutex g_side_mu;
+SideStream g_side[64];
+
+// the current device's side stream, created on first use; call with g_side_mu held
+int side_stream(SideStream** out) {
+    int dev = 0;
+    IMOPS_CUDA_TRY(cudaGetDevice(&dev), "cudaGetDevice");
+    if (dev < 0 || dev >= 64) return fail(IMOPS_ERR_INVALID_ARGUMENT, "film: device index above 63");
+    SideStream& d = g_side[dev];
+    if (!d.init) {
+        cudaStream_t st = nullptr;
+        cudaEvent_t f = nullptr, j = nullptr;
+        cudaError_t e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&f, cudaEventDisableTiming);
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&j, cudaEventDisableTiming);
+        if (e != cudaSuccess) {
+            if (st) cudaStreamDestroy(st);
+            if (f) cudaEventDestroy(f);
+            if (j) cudaEventDestroy(j);
+            return cuda_status(e, "film side stream");
+        }
+        d.side = st;
+        d.fork = f;
+        d.join = j;
+        d.init = true;
+    }
+    *out = &d;
+    return IMOPS_OK;
+}
+
+// run_reference with the mid-grey patch on the side stream: its dozen small
+// kernels (60 us) run beside the frame's, up to the print.  The events are
+// this call's own, so calls on other threads may queue theirs in between; the
+// stream waits for the patch on every way out, as its scratch is the stream's.
+int run_positive(float* rgb, int W, int H, const Stock& st, const ImopsFilmParams& P, Arena& A, const float* lut,
+                 float* mid_dmin, cudaStream_t s) {
+    SideStream* ss = nullptr;
+    int rc;
+    {
+        std::lock_guard<std::mutex> lock(g_side_mu);
+        if ((rc = side_stream(&ss))) return rc;
+    }
+    cudaEvent_t fork = nullptr, join = nullptr;
+    cudaError_t e = cudaEventCreateWithFlags(&fork, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&join, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventRecord(fork, s);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(ss->side, fork, 0);
+    if (e == cudaSuccess) {
+        rc = mid_gray_negative(st, P.grain, A, lut, mid_dmin, ss->side);
+        e = cudaEventRecord(join, ss->side);
+        if (!rc && e == cudaSuccess) rc = run_reference(rgb, W, H, st, P.seed, P.grain, mid_dmin, A, lut, s, join);
+        if (rc && e == cudaSuccess) cudaStreamWaitEvent(s, join, 0);
+    }
+    if (fork) cudaEventDestroy(fork);  // released once the work recorded in it is done
+    if (join) cudaEventDestroy(join);
+    return rc ? rc : cuda_status(e, "film mid-grey events");
 }
 
 int process_reference(float* rgb, int W, int H, const ImopsFilmParams& P, cudaStream_t s) {
@@ -1875,8 +1956,8 @@ int process_reference(float* rgb, int W, int H, const ImopsFilmParams& P, cudaSt
     float* mid_dmin = A.take<float>(8);
     if ((rc = launch_capture_lut(st.ref, lut, s))) return rc;
     bool positive = P.output == IMOPS_FILM_POSITIVE_LINEAR && !st.ref.any_reversal;
-    if (positive && (rc = mid_gray_negative(st, P.grain, A, lut, mid_dmin, s))) return rc;
-    return run_reference(rgb, W, H, st, P.seed, P.grain, positive ? mid_dmin : nullptr, A, lut, s);
+    if (positive) return run_positive(rgb, W, H, st, P, A, lut, mid_dmin, s);
+    return run_reference(rgb, W, H, st, P.seed, P.grain, nullptr, A, lut, s);
 }
 
 // One sub-stage call: the stock (reference model only) and an arena of `extra` bytes in the film workspace.
@@ -1940,44 +2021,6 @@ int baseline_forward_impl(float* rgb, int W, int H, const ImopsBaselineFilm* Pp,
 // The baseline preset's kernels with the working set at `scratch` (256-byte
 // aligned, baseline_scratch_bytes(W, H) long).  Every byte the kernels read
 // there is written earlier in the same call.
-// A second stream per device for work that does not depend on the image
-// (the grain fields), forked from and joined back to the caller's stream with
-// events: the grain then runs beside the halation row pass.
-struct SideStream {
-    bool init = false;
-    cudaStream_t side = nullptr;
-    cudaEvent_t fork = nullptr, join = nullptr;
-};
-std::mutex g_side_mu;
-SideStream g_side[64];
-
-// the current device's side stream, created on first use; call with g_side_mu held
-int side_stream(SideStream** out) {
-    int dev = 0;
-    IMOPS_CUDA_TRY(cudaGetDevice(&dev), "cudaGetDevice");
-    if (dev < 0 || dev >= 64) return fail(IMOPS_ERR_INVALID_ARGUMENT, "film: device index above 63");
-    SideStream& d = g_side[dev];
-    if (!d.init) {
-        cudaStream_t st = nullptr;
-        cudaEvent_t f = nullptr, j = nullptr;
-        cudaError_t e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
-        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&f, cudaEventDisableTiming);
-        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&j, cudaEventDisableTiming);
-        if (e != cudaSuccess) {
-            if (st) cudaStreamDestroy(st);
-            if (f) cudaEventDestroy(f);
-            if (j) cudaEventDestroy(j);
-            return cuda_status(e, "film side stream");
-        }
-        d.side = st;
-        d.fork = f;
-        d.join = j;
-        d.init = true;
-    }
-    *out = &d;
-    return IMOPS_OK;
-}
-
 int baseline_forward_in(float* rgb, int W, int H, const ImopsBaselineFilm& P, const Stock& st, void* scratch,
                         cudaStream_t s) {
     int rc;

@@ -137,3 +137,35 @@ def test_preset_scan_matches_oracle_on_both_sides_of_its_block_rule(oracle_lib, 
     out = im.film_process(torch.from_numpy(x).to(gpu), stock=im.STOCK_BASELINE81,
                           baseline=im.baseline_film_defaults(grain_on=1, seed=9)).cpu().numpy()
     assert np.abs(out - ref).max() < TOL
+
+
+def test_positives_from_threads_and_streams(gpu):
+    """A positive's mid-grey patch runs on a stream of the device's own, shared
+    by all callers: frames of other sizes and stocks from four threads, each
+    on its stream, give what each gives alone."""
+    import threading
+
+    import torch
+
+    import imops_b200 as im
+    work = [(1, 40, 61), (3, 300, 517), (6, 33, 129), (2, 64, 2050)]
+    xs = [torch.from_numpy(_scene(h, w, seed=h)).to(gpu) for _, h, w in work]
+    alone = [im.film_process(x.clone(), stock=st, seed=2, output=1, grain=True) for x, (st, _, _) in zip(xs, work)]
+    torch.cuda.synchronize()
+    bad = []
+
+    def run(k):
+        s = torch.cuda.Stream(gpu)
+        with torch.cuda.stream(s):
+            for _ in range(8):
+                out = im.film_process(xs[k].clone(), stock=work[k][0], seed=2, output=1, grain=True)
+                s.synchronize()
+                if not torch.equal(out, alone[k]):
+                    bad.append(k)
+
+    ts = [threading.Thread(target=run, args=(k,)) for k in range(len(work))]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert not bad
