@@ -169,3 +169,17 @@ def test_positives_from_threads_and_streams(gpu):
     for t in ts:
         t.join()
     assert not bad
+
+
+@pytest.mark.parametrize("stock,H,W", [(1, 300, 680), (1, 300, 690), (0, 760, 808), (0, 760, 809), (2, 300, 343)])
+def test_grain_beside_the_frame_matches_the_sub_stages(gpu, stock, H, W):
+    """Negatives just below and above the size from which the grain fields run
+    on the side stream, against the sub-stages, which never do; repeated, as
+    each call's planes are the last one's."""
+    import torch
+
+    import imops_b200 as im
+    x = torch.from_numpy(_scene(H, W, seed=stock + W)).to(gpu)
+    ref = im.FilmStages(stock=stock, seed=5, output=0, grain=True).run(x.clone())
+    for _ in range(4):
+        assert torch.equal(im.film_process(x.clone(), stock=stock, seed=5, output=0, grain=True), ref)
