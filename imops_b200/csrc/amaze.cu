@@ -222,22 +222,13 @@ __device__ void fill(const P& p, const Geo& g, float* mos) {
                   [&](int rr, int cc) { return get_in(p, H - rr - 2, 32 - cc); });
 }
 
-// Loop helpers: every site of rows [r0,r1) x cols [c0,c1).  Threads map to
-// (row group, column) directly: a tile row has at most 128 sites, so no
-// integer division is needed.
-template <class F>
-__device__ __forceinline__ void for_rect(int r0, int r1, int c0, int c1, F f) {
-    const int cc = c0 + (int)(threadIdx.x & (TS - 1));
-    if (cc >= c1) return;
-    for (int rr = r0 + (int)(threadIdx.x / TS); rr < r1; rr += NTHREADS / TS) f(rr, cc);
-}
-
-// The same sites, and the R/B sites of those rows (first R/B column = c0 +
-// parity of the row; c0 even), dense over the block's threads: thread t takes sites t,
-// t + NTHREADS, ... in row-major order, so no lane idles at a row's end (the
-// inner stages' rows are 96-112 sites of 128, or 50-56 R/B sites of 64); the
-// row and column advance without a division.  Bayer rows alternate the
-// parity of their R/B columns.
+// Loop helpers: every site of rows [r0,r1) x cols [c0,c1), or the R/B sites
+// of those rows (first R/B column = c0 + parity of the row; c0 even), dense
+// over the block's threads: thread t takes sites t, t + NTHREADS, ... in
+// row-major order, so no lane idles at a row's end (the inner stages' rows
+// are 96-112 sites of 128, or 50-56 R/B sites of 64); the row and column
+// advance without a division.  Bayer rows alternate the parity of their R/B
+// columns.
 template <class F>
 __device__ __forceinline__ void for_rect_dense(int r0, int r1, int c0, int c1, F f) {
     const int w = c1 - c0;

@@ -58,16 +58,13 @@ __device__ __forceinline__ float layer_exposure(const ExposeSpec& X, const float
     return dot3(X.A[0][e], w[0], X.A[1][e], w[1], X.A[2][e], w[2]);
 }
 
-// rgb (interleaved) -> E planes of absorbed band-mean fluence, optional
-// halation source plane max(0, R - threshold).
-__global__ void expose_kernel(const float* __restrict__ rgb, size_t n, ExposeSpec X, float* __restrict__ planes,
-                              float* __restrict__ hal) {
+// rgb (interleaved) -> E planes of absorbed band-mean fluence.
+__global__ void expose_kernel(const float* __restrict__ rgb, size_t n, ExposeSpec X, float* __restrict__ planes) {
     for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < n; p += (size_t)gridDim.x * blockDim.x) {
         float r = rgb[3 * p], g = rgb[3 * p + 1], b = rgb[3 * p + 2];
         float w[3];
         basis_weights(X, r, g, b, w);
         for (int e = 0; e < X.E; e++) planes[e * n + p] = layer_exposure(X, w, e);
-        if (X.hal_src) hal[p] = fmaxf(0.0f, r - X.hal_threshold);
     }
 }
 
@@ -1571,7 +1568,7 @@ size_t ref_workspace_bytes(int W, int H, int E) {
 //     absorption.rs:24-108)
 int stage_expose(const float* rgb, int W, int H, const Stock& st, float* planes, cudaStream_t s) {
     const size_t n = (size_t)W * H;
-    expose_kernel<<<grid_for(n), 256, 0, s>>>(rgb, n, st.expose, planes, nullptr);
+    expose_kernel<<<grid_for(n), 256, 0, s>>>(rgb, n, st.expose, planes);
     note_launch();
     return IMOPS_OK;
 }

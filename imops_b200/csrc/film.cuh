@@ -25,7 +25,7 @@ struct ExposeSpec {
     int E;
     float minv[9];
     float A[3][MAXE];
-    int hal_src;        // baseline preset: also emit max(0, R - hal_threshold)
+    int hal_src;        // baseline preset: halation of max(0, R - hal_threshold)
     float hal_threshold;
 };
 
