@@ -35,3 +35,21 @@ def test_result_does_not_depend_on_place(gpu, n, offset):
         assert torch.equal(view, ref[:n])
         # nothing outside the image is touched
         assert bool((buf[:offset] == -7.0).all()) and bool((buf[offset + 3 * n:] == -7.0).all())
+
+
+@pytest.mark.parametrize("space", [0, 1, 2, 3, 4])
+@pytest.mark.parametrize("n", [1, 129, 5000])
+def test_lch_equals_its_three_ops(gpu, space, n):
+    """Into Oklch, scaled, and back in one kernel: the bits of the three calls."""
+    import torch
+
+    import imops_b200 as im
+    x = torch.from_numpy(np.random.default_rng(n).uniform(-0.2, 2.0, (n, 3)).astype(np.float32)).to(gpu)
+    one, three = x.clone(), x.clone()
+    im.lch(one, space, 1.1, 0.9, 1.05)
+    if space != im.CS_OKLCH:
+        im.cst(three, space, im.CS_OKLCH)
+    im.lch(three, im.CS_OKLCH, 1.1, 0.9, 1.05)
+    if space != im.CS_OKLCH:
+        im.cst(three, im.CS_OKLCH, space)
+    assert torch.equal(one, three)
