@@ -116,22 +116,31 @@ int StreamCache::get(cudaStream_t s, size_t bytes, void** out) {
     if (fault_injected("alloc")) return fail(IMOPS_ERR_OUT_OF_MEMORY, std::string("injected allocation failure (") + what_ + ")");
     int dev = 0;
     IMOPS_CUDA_TRY(cudaGetDevice(&dev), "cudaGetDevice");
-    const std::string m = std::string("cudaMallocAsync(") + what_ + ")";
+    // a request without room leaves nothing behind: the stream's next one
+    // allocates anew, and the runtime's last error is not for others to find
+    auto allocate = [&](void** p) {
+        const cudaError_t e = cudaMallocAsync(p, bytes, s);
+        if (e != cudaSuccess) cudaGetLastError();
+        return cuda_status(e, (std::string("cudaMallocAsync(") + what_ + ")").c_str());
+    };
     std::lock_guard<std::mutex> lock(mu_);
     for (auto& e : v_)
         if (e.dev == dev && e.s == s) {
             if (e.bytes < bytes) {
-                IMOPS_CUDA_TRY(cudaFreeAsync(e.p, s), "cudaFreeAsync");
+                if (e.p) IMOPS_CUDA_TRY(cudaFreeAsync(e.p, s), "cudaFreeAsync");
                 e.p = nullptr;
                 e.bytes = 0;
-                IMOPS_CUDA_TRY(cudaMallocAsync(&e.p, bytes, s), m.c_str());
+                if (int rc = allocate(&e.p)) {
+                    e.p = nullptr;
+                    return rc;
+                }
                 e.bytes = bytes;
             }
             *out = e.p;
             return IMOPS_OK;
         }
     void* p = nullptr;
-    IMOPS_CUDA_TRY(cudaMallocAsync(&p, bytes, s), m.c_str());
+    if (int rc = allocate(&p)) return rc;
     v_.push_back({dev, s, p, bytes});
     *out = p;
     return IMOPS_OK;

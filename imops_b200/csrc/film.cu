@@ -1972,7 +1972,6 @@ int process_reference(float* rgb, int W, int H, const ImopsFilmParams& P, cudaSt
     void* ws = nullptr;
     rc = workspace(s, bytes + more, &ws);
     if (rc && more) {  // no room for planes of the grain's own
-        cudaGetLastError();
         clear_error();
         grain_beside = false;
         rc = workspace(s, bytes, &ws);

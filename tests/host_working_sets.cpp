@@ -1,0 +1,42 @@
+// The working sets' cache (StreamCache) on the fake runtime: a request that
+// finds no room for a larger buffer fails and leaves nothing behind: the next
+// ones work, and no later check finds its error.
+#include "fake_cuda.hpp"
+
+#include <cstdio>
+
+#include "common.cuh"
+
+extern "C" {
+cudaError_t cudaPointerGetAttributes(cudaPointerAttributes*, const void*) { return cudaErrorNotSupported; }
+cudaError_t cudaHostAlloc(void**, size_t, unsigned) { return cudaErrorNotSupported; }
+cudaError_t cudaFreeHost(void*) { return cudaErrorNotSupported; }
+cudaError_t cudaEventCreateWithFlags(cudaEvent_t*, unsigned) { return cudaErrorNotSupported; }
+cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaErrorNotSupported; }
+cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaErrorNotSupported; }
+cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaErrorNotSupported; }
+cudaError_t cudaMemcpyAsync(void*, const void*, size_t, cudaMemcpyKind, cudaStream_t) { return cudaErrorNotSupported; }
+}
+
+#define EXPECT(x) \
+    if (!(x)) return std::printf("line %d: %s\n", __LINE__, #x), 1
+
+int main() {
+    imops::StreamCache cache("test");
+    const cudaStream_t s = reinterpret_cast<cudaStream_t>(0x10);
+    void* p = nullptr;
+    fake::room = 1000;
+    EXPECT(cache.get(s, 100, &p) == IMOPS_OK && p);
+    EXPECT(cache.get(s, 2000, &p) == IMOPS_ERR_OUT_OF_MEMORY);  // the larger form of a call
+    EXPECT(cudaGetLastError() == cudaSuccess);
+    EXPECT(cache.get(s, 800, &p) == IMOPS_OK && p);             // and its form with less
+    EXPECT(cache.get(s, 100, &p) == IMOPS_OK && p);
+    EXPECT(fake::room == 200 && fake::null_frees == 0);
+    EXPECT(cache.get(s, 2000, &p) == IMOPS_ERR_OUT_OF_MEMORY);
+    EXPECT(cache.get(s, 3000, &p) == IMOPS_ERR_OUT_OF_MEMORY);  // twice in a row
+    cache.release_device(0);
+    EXPECT(fake::room == 1000 && fake::null_frees == 0);
+    EXPECT(cache.get(s, 500, &p) == IMOPS_OK && p);
+    std::puts("ok");
+    return 0;
+}

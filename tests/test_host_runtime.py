@@ -1,0 +1,25 @@
+"""The library's host logic around the CUDA runtime (common.cu), compiled
+against a fake runtime on host memory, so that failures and devices that no
+test machine has can be played through without a GPU."""
+import os
+import subprocess
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+ROOT = os.path.dirname(HERE)
+
+
+def _run(tmp_path, name):
+    exe = tmp_path / name
+    src = os.path.join(ROOT, "imops_b200", "csrc")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-pthread", "-I", HERE, "-I", src, "-I", os.path.join(ROOT, "include"),
+                    "-I", "/usr/local/cuda/include", "-x", "c++", os.path.join(HERE, name + ".cpp"),
+                    os.path.join(src, "common.cu"), "-o", str(exe)], check=True, timeout=300)
+    r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=60)
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
+@pytest.mark.parametrize("name", ["host_working_sets"])
+def test_host(tmp_path, name):
+    _run(tmp_path, name)
