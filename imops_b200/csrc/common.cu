@@ -158,6 +158,74 @@ void StreamCache::release_device(int dev) {
     }
 }
 
+// ---- side streams ----------------------------------------------------------------
+
+namespace {
+
+struct SideEntry {
+    int dev;
+    cudaStream_t s;
+    SideStream ss;
+};
+std::mutex g_sides_mu;
+std::vector<SideEntry> g_sides;
+
+void destroy_side(SideStream& ss) {
+    if (ss.side) cudaStreamDestroy(ss.side);
+    if (ss.forked) cudaEventDestroy(ss.forked);
+    if (ss.joined) cudaEventDestroy(ss.joined);
+}
+
+}  // namespace
+
+int side_stream(cudaStream_t s, SideStream* out) {
+    int dev = 0;
+    IMOPS_CUDA_TRY(cudaGetDevice(&dev), "cudaGetDevice");
+    std::lock_guard<std::mutex> lock(g_sides_mu);
+    int held = 0;
+    for (const SideEntry& e : g_sides) {
+        if (e.dev != dev) continue;
+        if (e.s == s) {
+            *out = e.ss;
+            return IMOPS_OK;
+        }
+        held++;
+    }
+    SideStream ss;
+    if (held >= SIDE_STREAMS) {
+        ss.side = s;
+        *out = ss;
+        return IMOPS_OK;
+    }
+    cudaError_t e = cudaStreamCreateWithFlags(&ss.side, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ss.forked, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ss.joined, cudaEventDisableTiming);
+    if (e != cudaSuccess) {
+        destroy_side(ss);
+        return cuda_status(e, "side stream");
+    }
+    g_sides.push_back({dev, s, ss});
+    *out = ss;
+    return IMOPS_OK;
+}
+
+int SideStream::fork(cudaStream_t s) const {
+    if (side == s) return IMOPS_OK;
+    IMOPS_CUDA_TRY(cudaEventRecord(forked, s), "cudaEventRecord(side fork)");
+    IMOPS_CUDA_TRY(cudaStreamWaitEvent(side, forked, 0), "cudaStreamWaitEvent(side fork)");
+    return IMOPS_OK;
+}
+
+int SideStream::record(cudaStream_t s) const {
+    if (side != s) IMOPS_CUDA_TRY(cudaEventRecord(joined, side), "cudaEventRecord(side join)");
+    return IMOPS_OK;
+}
+
+int SideStream::wait(cudaStream_t s) const {
+    if (side != s) IMOPS_CUDA_TRY(cudaStreamWaitEvent(s, joined, 0), "cudaStreamWaitEvent(side join)");
+    return IMOPS_OK;
+}
+
 // ---- downloads -----------------------------------------------------------------
 
 namespace {
@@ -276,6 +344,17 @@ int release_working_sets(int dev) {
         std::lock_guard<std::mutex> lock(g_rings_mu);
         for (Ring& r : g_rings)
             if (r.dev == dev && !r.busy) free_ring(r);
+    }
+    {
+        std::lock_guard<std::mutex> lock(g_sides_mu);
+        for (size_t k = 0; k < g_sides.size();) {
+            if (g_sides[k].dev == dev) {
+                destroy_side(g_sides[k].ss);
+                g_sides.erase(g_sides.begin() + k);
+            } else {
+                k++;
+            }
+        }
     }
     std::lock_guard<std::mutex> lock(g_caches_mu);
     for (StreamCache* c : caches()) c->release_device(dev);

@@ -118,6 +118,27 @@ class StreamCache {
     std::vector<E> v_;
 };
 
+// A second stream for the work of a call on stream s that its other kernels do
+// not need yet, ordered by a fork and a join.  Every caller's stream has its
+// own: one that all callers shared would run their side work in the order of
+// the calls, so that a film waited for whatever another caller's stream had
+// queued before its own film, and a capture of one into a graph drew the
+// others in.  Kept per (device, stream), as the working sets are, for at most
+// SIDE_STREAMS streams a device (for more, `side` is s itself, and a call's
+// kernels run one after the other), and destroyed with them.
+struct SideStream {
+    cudaStream_t side = nullptr;
+    cudaEvent_t forked = nullptr, joined = nullptr;
+    // What follows on `side` comes after what s holds so far.
+    int fork(cudaStream_t s) const;
+    // What follows on s comes after what `side` holds so far: record marks the
+    // place, wait (at any later point of s) orders s behind it.
+    int record(cudaStream_t s) const;
+    int wait(cudaStream_t s) const;
+};
+constexpr int SIDE_STREAMS = 128;
+int side_stream(cudaStream_t s, SideStream* out);
+
 // Copies `bytes` from device memory to a host buffer after the work queued on
 // s, and waits for it.  Large copies into pageable memory go through a ring of
 // pinned chunks: each of a few threads waits for its chunk, copies it out (and

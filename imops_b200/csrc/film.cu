@@ -15,7 +15,6 @@
 // stream; RGB stays interleaved as in Image.rgb_data.
 #include <cmath>
 #include <cstring>
-#include <mutex>
 #include <type_traits>
 #include <utility>
 #include <vector>
@@ -1825,10 +1824,10 @@ int print_scan(float* dens, const float* mask, const float* noise, const double*
 }
 
 // The reference model's kernels on rgb in place, inverted with the reference
-// points mid_dmin unless that is NULL; those are waited for on `ready` where
-// another stream forms them.
+// points mid_dmin unless that is NULL; those, and the grain fields where they
+// are given, are waited for on `beside` where that stream forms them.
 int run_reference(float* rgb, int W, int H, const Stock& st, uint64_t seed, int grain, const float* mid_dmin, Arena& A,
-                  const float* lut, cudaStream_t s, cudaEvent_t ready = nullptr, float* fields = nullptr,
+                  const float* lut, cudaStream_t s, const SideStream* beside = nullptr, float* fields = nullptr,
                   double* field_sums = nullptr) {
     const int E = st.ref.E;
     const size_t n = (size_t)W * H;
@@ -1847,7 +1846,7 @@ int run_reference(float* rgb, int W, int H, const Stock& st, uint64_t seed, int 
     // the other set of planes is free after develop: it takes the grain fields
     float* noise = fields ? fields : grain ? (dens == planes ? inh : planes) : nullptr;
     if (grain && !fields && (rc = stage_grain_fields(W, H, st.ref, seed, noise, partial, sums, s))) return rc;
-    if (ready) IMOPS_CUDA_TRY(cudaStreamWaitEvent(s, ready, 0), "cudaStreamWaitEvent(mid grey)");
+    if (beside && (rc = beside->wait(s))) return rc;
     if ((rc = print_scan(dens, mask, noise, sums, mid_dmin, W, H, st, tmp, rgb, s))) return rc;
     IMOPS_CUDA_TRY(cudaGetLastError(), "film kernels");
     return IMOPS_OK;
@@ -1872,82 +1871,31 @@ int mid_gray_negative(const Stock& st, int grain, Arena& A, const float* lut, fl
     return IMOPS_OK;
 }
 
-// A second stream per device for work that does not depend on the image (the
-// preset's grain fields, a positive's mid-grey patch), forked from and joined
-// back to the caller's stream with events: it then runs beside the kernels
-// before its result is needed.
-struct SideStream {
-    bool init = false;
-    cudaStream_t side = nullptr;
-    cudaEvent_t fork = nullptr, join = nullptr;
-};
-std::mutex g_side_mu;
-SideStream g_side[64];
-
-// the current device's side stream, created on first use; call with g_side_mu held
-int side_stream(SideStream** out) {
-    int dev = 0;
-    IMOPS_CUDA_TRY(cudaGetDevice(&dev), "cudaGetDevice");
-    if (dev < 0 || dev >= 64) return fail(IMOPS_ERR_INVALID_ARGUMENT, "film: device index above 63");
-    SideStream& d = g_side[dev];
-    if (!d.init) {
-        cudaStream_t st = nullptr;
-        cudaEvent_t f = nullptr, j = nullptr;
-        cudaError_t e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
-        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&f, cudaEventDisableTiming);
-        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&j, cudaEventDisableTiming);
-        if (e != cudaSuccess) {
-            if (st) cudaStreamDestroy(st);
-            if (f) cudaEventDestroy(f);
-            if (j) cudaEventDestroy(j);
-            return cuda_status(e, "film side stream");
-        }
-        d.side = st;
-        d.fork = f;
-        d.join = j;
-        d.init = true;
-    }
-    *out = &d;
-    return IMOPS_OK;
-}
-
-// run_reference with the work that does not depend on the image on the side
-// stream, up to the print: a positive's mid-grey patch, whose dozen small
-// kernels take 60 us, or the grain fields (grain_beside: into planes of their
-// own).  Not both: the grain before the patch delays the print (640x480, six
-// layers: 142 -> 177 us), and after it is late itself.  The events are this call's own, so calls on other threads may queue theirs in between; the
-// stream waits for the patch on every way out, as its scratch is the stream's.
+// run_reference with the work that does not depend on the image on the
+// caller's side stream, up to the print: a positive's mid-grey patch, whose
+// dozen small kernels take 60 us, or the grain fields (grain_beside: into
+// planes of their own).  Not both: the grain before the patch delays the print
+// (640x480, six layers: 142 -> 177 us), and after it is late itself.  The
+// stream waits for the side stream on every way out, as its scratch is the
+// stream's.
 int run_beside(float* rgb, int W, int H, const Stock& st, const ImopsFilmParams& P, Arena& A, const float* lut,
                float* mid_dmin, bool grain_beside, cudaStream_t s) {
-    SideStream* ss = nullptr;
-    int rc = IMOPS_OK;
-    {
-        std::lock_guard<std::mutex> lock(g_side_mu);
-        if ((rc = side_stream(&ss))) return rc;
+    SideStream ss;
+    int rc = side_stream(s, &ss);
+    if (rc || (rc = ss.fork(s))) return rc;
+    float* fields = nullptr;
+    double* sums = nullptr;
+    if (grain_beside) {
+        fields = A.take<float>(st.ref.E * (size_t)W * H);
+        double* partial = A.take<double>(grain_partials(W, H, st.ref.E));
+        sums = A.take<double>(MAXE);
+        rc = stage_grain_fields(W, H, st.ref, P.seed, fields, partial, sums, ss.side);
     }
-    cudaEvent_t fork = nullptr, join = nullptr;
-    cudaError_t e = cudaEventCreateWithFlags(&fork, cudaEventDisableTiming);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&join, cudaEventDisableTiming);
-    if (e == cudaSuccess) e = cudaEventRecord(fork, s);
-    if (e == cudaSuccess) e = cudaStreamWaitEvent(ss->side, fork, 0);
-    if (e == cudaSuccess) {
-        float* fields = nullptr;
-        double* sums = nullptr;
-        if (grain_beside) {
-            fields = A.take<float>(st.ref.E * (size_t)W * H);
-            double* partial = A.take<double>(grain_partials(W, H, st.ref.E));
-            sums = A.take<double>(MAXE);
-            rc = stage_grain_fields(W, H, st.ref, P.seed, fields, partial, sums, ss->side);
-        }
-        if (!rc && mid_dmin) rc = mid_gray_negative(st, P.grain, A, lut, mid_dmin, ss->side);
-        e = cudaEventRecord(join, ss->side);
-        if (!rc && e == cudaSuccess)
-            rc = run_reference(rgb, W, H, st, P.seed, P.grain, mid_dmin, A, lut, s, join, fields, sums);
-        if (rc && e == cudaSuccess) cudaStreamWaitEvent(s, join, 0);
-    }
-    if (fork) cudaEventDestroy(fork);  // released once the work recorded in it is done
-    if (join) cudaEventDestroy(join);
-    return rc ? rc : cuda_status(e, "film side events");
+    if (!rc && mid_dmin) rc = mid_gray_negative(st, P.grain, A, lut, mid_dmin, ss.side);
+    const int joined = ss.record(s);
+    if (!rc && !joined) rc = run_reference(rgb, W, H, st, P.seed, P.grain, mid_dmin, A, lut, s, &ss, fields, sums);
+    if (rc && !joined) ss.wait(s);
+    return rc ? rc : joined;
 }
 
 // The layer values (layers x pixels) at which the grain runs beside the other
@@ -2062,19 +2010,19 @@ int baseline_forward_in(float* rgb, int W, int H, const ImopsBaselineFilm& P, co
     build_base81(st, &hp);
     if (P.grain_on && P.grain_sigma != 0.0f) {
         // grain fields on the side stream while the halation row pass runs on
-        // s; the scan waits for both.  The lock keeps one call's
-        // record / wait pairs of the shared events together.
+        // s; the scan waits for both
         Taps tp;
         if ((rc = taps_for(fmaxf(P.grain_blur, 1.0f), &tp))) return rc;
-        std::lock_guard<std::mutex> lock(g_side_mu);
-        SideStream* ss = nullptr;
-        if ((rc = side_stream(&ss))) return rc;
-        IMOPS_CUDA_TRY(cudaEventRecord(ss->fork, s), "cudaEventRecord(film fork)");
-        IMOPS_CUDA_TRY(cudaStreamWaitEvent(ss->side, ss->fork, 0), "cudaStreamWaitEvent(film fork)");
-        if ((rc = grain_fields(noise, W, H, P.seed, 0, 3, tp, gpart, sums, ss->side))) return rc;
-        IMOPS_CUDA_TRY(cudaEventRecord(ss->join, ss->side), "cudaEventRecord(film join)");
-        if ((rc = blur_rows_halation(rgb, st.expose.hal_threshold, hr, W, H, st.hal_taps, s))) return rc;
-        IMOPS_CUDA_TRY(cudaStreamWaitEvent(s, ss->join, 0), "cudaStreamWaitEvent(film join)");
+        SideStream ss;
+        if ((rc = side_stream(s, &ss)) || (rc = ss.fork(s))) return rc;
+        rc = grain_fields(noise, W, H, P.seed, 0, 3, tp, gpart, sums, ss.side);
+        const int joined = ss.record(s);
+        if (!rc && !joined) rc = blur_rows_halation(rgb, st.expose.hal_threshold, hr, W, H, st.hal_taps, s);
+        if (!joined) {
+            const int waited = ss.wait(s);
+            if (!rc) rc = waited;
+        }
+        if (rc || (rc = joined)) return rc;
     } else {
         if ((rc = blur_rows_halation(rgb, st.expose.hal_threshold, hr, W, H, st.hal_taps, s))) return rc;
     }

@@ -20,6 +20,6 @@ def _run(tmp_path, name):
     assert r.returncode == 0, r.stdout + r.stderr
 
 
-@pytest.mark.parametrize("name", ["host_working_sets"])
+@pytest.mark.parametrize("name", ["host_working_sets", "host_side_streams"])
 def test_host(tmp_path, name):
     _run(tmp_path, name)
