@@ -215,16 +215,32 @@ __device__ __forceinline__ float lut_sample(const float2* lut, float phi) {
     return fmaf(t, c.y, c.x);
 }
 
-// f^g for f in [0, 1], g > 0, to about an ulp: the product g log2 f is split
-// into its nearest integer and a remainder rounded once, and 2^remainder is a
-// polynomial of degree 6 fitted here for least relative error on
-// [-1/2, 1/2] (2e-9).  (The hardware exponential's 2 ulp near f = 1, where a
-// positive print's highlights lie, were the largest error of the reduction.)
+// f^g for f in [0, 1], g > 0, to about an ulp (1.4e-7 at g = 2.9): with
+// f = 2^k (1 + t), 1 + t in [0.71, 1.41), the product g log2 f is g k +
+// g log2(1 + t).  Its nearest integer n leaves g k by one fused operation, and
+// log2(1 + t), at most 1/2, is good to 4e-8 as t (log2 e + t Q(t)), Q a
+// polynomial of degree 7 fitted here for least error; a logarithm of f itself
+// rounds at 5e-7 for f = 1e-4, an error of 10 ulp.  2^remainder is a polynomial of degree 6
+// fitted here for least relative error on [-1/2, 1/2] (2e-9).  (The hardware
+// exponential's 2 ulp near f = 1, where a positive print's highlights lie, were
+// the largest error of the reduction.)  0 and subnormals, and results below
+// 2^-125, are 0.
 __device__ __forceinline__ float pow_unit(float f, float g) {
-    const float l = log2f(f);
-    const float n = rintf(g * l);
-    if (!(n > -126.0f)) return f != f ? f : 0.0f;
-    const float r = fmaf(g, l, -n);
+    const uint32_t up = __float_as_uint(f) - 0x3F3504F3u;  // from the bits of sqrt(1/2)
+    const float k = (float)((int)up >> 23);
+    const float t = __uint_as_float((up & 0x007FFFFFu) + 0x3F3504F3u) - 1.0f;
+    float p = 0.12592235207557678f;
+    p = fmaf(p, t, -0.20859862864017487f);
+    p = fmaf(p, t, 0.21626605093479156f);
+    p = fmaf(p, t, -0.23876483738422394f);
+    p = fmaf(p, t, 0.2878434956073761f);
+    p = fmaf(p, t, -0.36071109771728516f);
+    p = fmaf(p, t, 0.48091256618499756f);
+    p = fmaf(p, t, -0.7213472723960876f);
+    const float lm = fmaf(t, 1.44269502f, p * (t * t));
+    const float n = rintf(fmaf(g, lm, g * k));
+    if (f < 1.17549435e-38f || n <= -126.0f) return 0.0f;
+    const float r = fmaf(g, lm, fmaf(g, k, -n));
     float q = 0.0001535336923552677f;
     q = fmaf(q, r, 0.0013398876180872321f);
     q = fmaf(q, r, 0.00961843691766262f);
