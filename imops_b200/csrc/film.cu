@@ -1950,14 +1950,17 @@ int process_reference(float* rgb, int W, int H, const ImopsFilmParams& P, cudaSt
     return run_reference(rgb, W, H, st, P.seed, P.grain, nullptr, A, lut, s);
 }
 
-// One sub-stage call: the stock (reference model only) and an arena of `extra` bytes in the film workspace.
+// One sub-stage call: the stock (reference model only) and, once its layers are
+// known, an arena in the film workspace.
 struct StageCtx {
     Stock st;
     Arena A;
     float* lut;  // the capture LUT's place (launch_capture_lut fills it)
 };
 
-int stage_ctx(const ImopsFilmParams* P, int W, int H, size_t extra, cudaStream_t s, StageCtx* c) {
+// extra(E): bytes of the arena besides the LUT for a stock of E layers.
+template <class Extra>
+int stage_ctx(const ImopsFilmParams* P, int W, int H, Extra extra, cudaStream_t s, StageCtx* c) {
     if (!P) return fail(IMOPS_ERR_INVALID_ARGUMENT, "film stage: NULL params");
     if (W <= 0 || H <= 0) return fail(IMOPS_ERR_INVALID_DIMENSIONS, "invalid image dimensions");
     float pitch = 0;
@@ -1966,11 +1969,13 @@ int stage_ctx(const ImopsFilmParams* P, int W, int H, size_t extra, cudaStream_t
     if (c->st.model != MODEL_REFERENCE)
         return fail(IMOPS_ERR_INVALID_STOCK, "film stages: the baseline preset runs only whole (imops_film_process)");
     void* ws = nullptr;
-    if ((rc = workspace(s, MAXE * LUTN * sizeof(float) + extra + 4096, &ws))) return rc;
+    const size_t bytes = MAXE * LUTN * sizeof(float) + (size_t)extra(c->st.ref.E) + 4096;
+    if ((rc = workspace(s, bytes, &ws))) return rc;
     c->A = Arena{static_cast<char*>(ws), 0};
     c->lut = c->A.take<float>(MAXE * LUTN);
     return IMOPS_OK;
 }
+size_t no_extra(int) { return 0; }
 
 }  // namespace film
 }  // namespace imops
@@ -2091,7 +2096,7 @@ extern "C" int imops_film_expose(const float* rgb, int w, int h, const ImopsFilm
     clear_error();
     cudaStream_t s = as_stream(stream);
     film::StageCtx c;
-    int rc = film::stage_ctx(params, w, h, 0, s, &c);
+    int rc = film::stage_ctx(params, w, h, film::no_extra, s, &c);
     if (rc) return rc;
     if (!rgb || !planes) return fail(IMOPS_ERR_INVALID_ARGUMENT, "film_expose: NULL buffer");
     if ((rc = film::stage_expose(rgb, w, h, c.st, planes, s))) return rc;
@@ -2105,7 +2110,7 @@ extern "C" int imops_film_halation(float* planes, int w, int h, const ImopsFilmP
     cudaStream_t s = as_stream(stream);
     const size_t n = (size_t)(w > 0 ? w : 0) * (h > 0 ? h : 0);
     film::StageCtx c;
-    int rc = film::stage_ctx(params, w, h, 2 * n * 4 + 512, s, &c);
+    int rc = film::stage_ctx(params, w, h, [=](int) { return 2 * n * 4 + 512; }, s, &c);
     if (rc) return rc;
     if (!planes) return fail(IMOPS_ERR_INVALID_ARGUMENT, "film_halation: NULL buffer");
     float* tmp = c.A.take<float>(n);
@@ -2127,7 +2132,7 @@ extern "C" int imops_film_develop(float* planes, float* mask, int w, int h, cons
     cudaStream_t s = as_stream(stream);
     const size_t n = (size_t)(w > 0 ? w : 0) * (h > 0 ? h : 0);
     film::StageCtx c;
-    int rc = film::stage_ctx(params, w, h, (size_t)(film::MAXE + 1) * n * 4 + 512, s, &c);
+    int rc = film::stage_ctx(params, w, h, [=](int E) { return (E + 1) * n * 4 + 512; }, s, &c);
     if (rc) return rc;
     if (!planes || !mask) return fail(IMOPS_ERR_INVALID_ARGUMENT, "film_develop: NULL buffer");
     float* inh = c.A.take<float>((size_t)c.st.ref.E * n);
@@ -2142,14 +2147,14 @@ extern "C" int imops_film_grain(float* planes, int w, int h, const ImopsFilmPara
     clear_error();
     cudaStream_t s = as_stream(stream);
     const size_t n = (size_t)(w > 0 ? w : 0) * (h > 0 ? h : 0);
-    const size_t np = w > 0 && h > 0 ? film::grain_partials(w, h, film::MAXE) : 0;
     film::StageCtx c;
-    int rc = film::stage_ctx(params, w, h, film::MAXE * n * 4 + np * 8 + film::MAXE * 8 + 768, s, &c);
+    int rc = film::stage_ctx(
+        params, w, h, [=](int E) { return E * n * 4 + film::grain_partials(w, h, E) * 8 + film::MAXE * 8 + 768; }, s, &c);
     if (rc) return rc;
     if (!planes) return fail(IMOPS_ERR_INVALID_ARGUMENT, "film_grain: NULL buffer");
     if (!params->grain) return IMOPS_OK;
     float* noise = c.A.take<float>(c.st.ref.E * n);
-    double* partial = c.A.take<double>(np);
+    double* partial = c.A.take<double>(film::grain_partials(w, h, c.st.ref.E));
     double* sums = c.A.take<double>(film::MAXE);
     if ((rc = film::stage_grain(planes, w, h, c.st, params->seed, noise, partial, sums, s))) return rc;
     IMOPS_CUDA_TRY(cudaGetLastError(), "film_grain");
@@ -2161,7 +2166,7 @@ extern "C" int imops_film_scan(const float* planes, const float* mask, int w, in
     clear_error();
     cudaStream_t s = as_stream(stream);
     film::StageCtx c;
-    int rc = film::stage_ctx(params, w, h, 0, s, &c);
+    int rc = film::stage_ctx(params, w, h, film::no_extra, s, &c);
     if (rc) return rc;
     if (!planes || !mask || !rgb) return fail(IMOPS_ERR_INVALID_ARGUMENT, "film_scan: NULL buffer");
     if ((rc = film::stage_scan(planes, mask, false, w, h, c.st.scan16, rgb, s))) return rc;
@@ -2175,7 +2180,8 @@ extern "C" int imops_film_invert(float* rgb, int w, int h, const ImopsFilmParams
     // the mid-grey patch's path and its reference points come from the same arena
     const size_t nm = 32 * 32;
     film::StageCtx c;
-    int rc = film::stage_ctx(params, w, h, film::ref_workspace_bytes(32, 32, film::MAXE) + nm * 12 + 1024, s, &c);
+    int rc = film::stage_ctx(
+        params, w, h, [=](int E) { return film::ref_workspace_bytes(32, 32, E) + nm * 12 + 1024; }, s, &c);
     if (rc) return rc;
     if (!rgb) return fail(IMOPS_ERR_INVALID_ARGUMENT, "film_invert: NULL buffer");
     if (!(params->output == IMOPS_FILM_POSITIVE_LINEAR && !c.st.ref.any_reversal)) return IMOPS_OK;

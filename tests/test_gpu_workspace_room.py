@@ -66,3 +66,33 @@ for output in (1, 0, 1):
         assert e.code == 5, e
     check(film(small), ref_small)
 """)
+
+
+@pytest.mark.parametrize("stock,layers", [(0, 1), (6, 2), (1, 3), (2, 6), (4, 7)])
+@pytest.mark.parametrize("stage,planes", [("grain", 0), ("develop", 1)])
+def test_stages_take_a_plane_a_layer(gpu, stock, layers, stage, planes):
+    """The working set of a stage: a plane for each of the stock's layers, and
+    one more for the blurs of develop (the block sums and tables are below
+    1 MiB here)."""
+    import torch
+    from cuda.bindings import driver as d
+
+    import imops_b200 as im
+    H, W = 1024, 2048
+    st = im.FilmStages(stock=stock, seed=3, grain=True)
+    v = torch.full((layers, H, W), 0.25, device=gpu)
+    torch.cuda.synchronize()
+    im.release_working_sets()
+    err, pool = d.cuDeviceGetMemPool(0)
+    assert err == 0
+
+    def used():
+        torch.cuda.synchronize()
+        err, n = d.cuMemPoolGetAttribute(pool, d.CUmemPool_attribute.CU_MEMPOOL_ATTR_USED_MEM_CURRENT)
+        assert err == 0
+        return int(n)
+
+    before = used()
+    getattr(st, stage)(v)
+    assert used() - before <= (layers + planes) * H * W * 4 + (1 << 20)
+    im.release_working_sets()
