@@ -1738,8 +1738,9 @@ int stage_develop(float* planes, float* mask, bool sum, const float* deep, int W
             if ((rc = launch_dir(in, out, W, H, tp, R, s))) return rc;
             planes = out;
         } else {
-            // a blur wider than the tiles' halo: 35 mm images above 12000 pixels, which only the
-            // sub-stage takes (their wide bounce is above 64 px)
+            // a blur wider than the tiles' halo: 35 mm Ektar100 images of 13715 to 13963 pixels
+            // width, and wider or other ones in the sub-stage alone (a whole image's wide bounce
+            // is then above 64 px)
             for (int i = 0; i < E; i++)
                 if ((rc = blur(planes + i * n, tmp, W, H, tp, EpiStore{inh + i * n}, s))) return rc;
             DirAny any;
@@ -1806,8 +1807,8 @@ int launch_print(const float* dens, const float* mask, const float* noise, const
 
 // Adjacency, grain (noise not NULL), scan and inversion (mid_dmin not NULL)
 // of the densities in one pass.  The radius classes are the stocks' at 35 mm
-// up to about 25 and 50 MP; wider blurs (only where the bounce is refused)
-// run as launches of their own.
+// up to about 25 and 50 MP; wider adjacency blurs (the stock without a wide
+// bounce, BwStub, above 19200 pixels width) run as launches of their own.
 int print_scan(float* dens, const float* mask, const float* noise, const double* sums, const float* mid_dmin, int W,
                int H, const Stock& st, float* tmp, float* rgb, cudaStream_t s) {
     const RefSpec& R = st.ref;
