@@ -28,13 +28,17 @@ using canon::XTransCanon;
 // (the window clamped at the image edges), the centre's own colour keeping
 // the centre sample.  Cfa: CfaFixed<2, 2> / CfaFixed<6, 6> for Bayer and
 // X-Trans, CfaDev for other periods; coordinates here are never negative.
-// in(y, x): the mosaic.
+// in(y, x): the mosaic; in.load(in.window(row, col), a, b): sample (a, b) of the
+// 3x3 window about (row, col), from one address for the window (24 MP by the
+// per-pixel kernel: other 6x6 CFAs 247 us, 268 with an address a sample; other
+// 2x2 ones 169, 191).
 template <class In, class Cfa>
 __device__ __forceinline__ void mean_px(const In& in, int W, int H, const Cfa& cfa, int row, int col, float* o) {
     const int centre = cfa.at(row, col);
     if (row >= 1 && row + 1 < H && col >= 1 && col + 1 < W) {
         // interior: the whole 3x3 window, unrolled and branch-free; each
         // colour's sum takes its sites in row-major order (predicated adds)
+        const float* p = in.window(row, col);
         float s0 = 0.0f, s1 = 0.0f, s2 = 0.0f, n0 = 0.0f, n1 = 0.0f, n2 = 0.0f;
 #pragma unroll
         for (int a = 0; a < 3; a++)
@@ -42,7 +46,7 @@ __device__ __forceinline__ void mean_px(const In& in, int W, int H, const Cfa& c
             for (int b = 0; b < 3; b++) {
                 if (a == 1 && b == 1) continue;
                 const int k = cfa.at(row + a - 1, col + b - 1);
-                const float v = in(row + a - 1, col + b - 1);
+                const float v = in.load(p, a, b);
                 s0 = k == 0 ? s0 + v : s0;
                 n0 = k == 0 ? n0 + 1.0f : n0;
                 s1 = k == 1 ? s1 + v : s1;
@@ -89,6 +93,10 @@ struct SrcF32 {
     int W;
     using Raw = float;
     __device__ __forceinline__ float operator()(int y, int x) const { return __ldg(p + (size_t)y * W + x); }
+    __device__ __forceinline__ const float* window(int row, int col) const {
+        return p + (size_t)(row - 1) * W + (col - 1);
+    }
+    __device__ __forceinline__ float load(const float* q, int a, int b) const { return __ldg(q + (size_t)a * W + b); }
 };
 
 // The mean alone.
@@ -165,6 +173,15 @@ __device__ __forceinline__ void run_phase(int rp, const float (&v)[3][RUN + 2], 
         else run_phase<P, RP + 1>(rp, v, o);
     }
 }
+
+// The rows a block has staged, from row y0 and column x0 of the mosaic on.
+struct SrcStaged {
+    const float (*s)[IN_STRIDE];
+    int y0, x0;
+    __device__ __forceinline__ float operator()(int y, int x) const { return s[y - y0][x - x0]; }
+    __device__ __forceinline__ const float* window(int row, int col) const { return &s[row - 1 - y0][col - 1 - x0]; }
+    __device__ __forceinline__ float load(const float* q, int a, int b) const { return q[a * IN_STRIDE + b]; }
+};
 
 // What the aligned kernel stages: an f32 mosaic as it is, or a u16 sensor
 // frame's crop scaled as color::scale_u16_kernel does, (v - black) / (white -
@@ -300,7 +317,7 @@ __global__ void __launch_bounds__(32 * MEAN_WARPS, std::is_same<Stage, StageF32>
             const int x = x0 + j;
             if (x >= 0 && x < W) {
                 float q[3];
-                mean_px([&](int yy, int xx) { return sin_[yy - y0 + 1][xx - xw + 1]; }, W, H, cfa, y, x, q);
+                mean_px(SrcStaged{sin_, y0 - 1, xw - 1}, W, H, cfa, y, x, q);
                 o[3 * j] = q[0];
                 o[3 * j + 1] = q[1];
                 o[3 * j + 2] = q[2];
