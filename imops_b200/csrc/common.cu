@@ -230,52 +230,67 @@ int SideStream::wait(cudaStream_t s) const {
 
 namespace {
 
+// Pinned chunks, of use to every device; the table is guarded, its memory is
+// made and used by the call that holds the ring.
 struct Ring {
-    int dev = -1;
     bool busy = false;
     void* slot[DOWNLOAD_SLOTS] = {};
-    cudaEvent_t filled[DOWNLOAD_SLOTS] = {};
 };
 std::mutex g_rings_mu;
 Ring g_rings[DOWNLOAD_RINGS];
 
-void free_ring(Ring& r) {
-    for (int i = 0; i < DOWNLOAD_SLOTS; i++) {
-        if (r.slot[i]) cudaFreeHost(r.slot[i]);
-        if (r.filled[i]) cudaEventDestroy(r.filled[i]);
+void free_slots(Ring& r) {
+    for (void*& p : r.slot) {
+        if (p) cudaFreeHost(p);
+        p = nullptr;
     }
-    r = Ring{};
-}
-
-// A free ring of the device, made if there is room for one; nullptr otherwise
-// (the caller then copies directly).
-Ring* take_ring(int dev) {
-    std::lock_guard<std::mutex> lock(g_rings_mu);
-    Ring* empty = nullptr;
-    for (Ring& r : g_rings) {
-        if (r.dev == dev && !r.busy) {
-            r.busy = true;
-            return &r;
-        }
-        if (r.dev < 0 && !empty) empty = &r;
-    }
-    if (!empty) return nullptr;
-    empty->dev = dev;
-    for (int i = 0; i < DOWNLOAD_SLOTS; i++)
-        if (cudaHostAlloc(&empty->slot[i], DOWNLOAD_CHUNK, cudaHostAllocDefault) != cudaSuccess ||
-            cudaEventCreateWithFlags(&empty->filled[i], cudaEventDisableTiming) != cudaSuccess) {
-            cudaGetLastError();  // not this call's failure: it has another way
-            free_ring(*empty);
-            return nullptr;
-        }
-    empty->busy = true;
-    return empty;
 }
 
 void give_back(Ring* r) {
     std::lock_guard<std::mutex> lock(g_rings_mu);
     r->busy = false;
 }
+
+// A ring that no call holds, rather one that has its memory; nullptr when all
+// are held or there is no memory for one (the caller then copies directly).
+Ring* take_ring() {
+    Ring* ring = nullptr;
+    {
+        std::lock_guard<std::mutex> lock(g_rings_mu);
+        for (Ring& r : g_rings)
+            if (!r.busy && (!ring || (r.slot[0] && !ring->slot[0]))) ring = &r;
+        if (!ring) return nullptr;
+        ring->busy = true;
+    }
+    if (ring->slot[0]) return ring;
+    for (void*& p : ring->slot)
+        if (cudaHostAlloc(&p, DOWNLOAD_CHUNK, cudaHostAllocPortable) != cudaSuccess) {
+            cudaGetLastError();  // not this call's failure: it has another way
+            p = nullptr;
+            free_slots(*ring);
+            give_back(ring);
+            return nullptr;
+        }
+    return ring;
+}
+
+// One call's events of the current device, one a slot.
+struct SlotEvents {
+    cudaEvent_t e[DOWNLOAD_SLOTS] = {};
+    bool make() {
+        for (cudaEvent_t& v : e)
+            if (cudaEventCreateWithFlags(&v, cudaEventDisableTiming) != cudaSuccess) {
+                cudaGetLastError();
+                v = nullptr;
+                return false;
+            }
+        return true;
+    }
+    ~SlotEvents() {
+        for (cudaEvent_t v : e)
+            if (v) cudaEventDestroy(v);
+    }
+};
 
 }  // namespace
 
@@ -287,7 +302,12 @@ int download(void* dst, const void* src, size_t bytes, cudaStream_t s, const cha
     if (bytes > DOWNLOAD_LEAST && cudaPointerGetAttributes(&to, dst) == cudaSuccess &&
         to.type == cudaMemoryTypeUnregistered && cudaPointerGetAttributes(&from, src) == cudaSuccess &&
         from.type == cudaMemoryTypeDevice && from.device == dev)
-        ring = take_ring(dev);
+        ring = take_ring();
+    SlotEvents filled;
+    if (ring && !filled.make()) {
+        give_back(ring);
+        ring = nullptr;
+    }
     if (!ring) {
         IMOPS_CUDA_TRY(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s), what);
         IMOPS_CUDA_TRY(cudaStreamSynchronize(s), "cudaStreamSynchronize");
@@ -300,13 +320,13 @@ int download(void* dst, const void* src, size_t bytes, cudaStream_t s, const cha
     auto queue = [&](int i, size_t c) {
         cudaError_t e = cudaMemcpyAsync(ring->slot[i], static_cast<const char*>(src) + c * DOWNLOAD_CHUNK, size_of(c),
                                         cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess) e = cudaEventRecord(ring->filled[i], s);
+        if (e == cudaSuccess) e = cudaEventRecord(filled.e[i], s);
         return e;
     };
     auto drain = [&](int i) {
         cudaError_t e = cudaSetDevice(dev);  // a helper's; the caller's current device already
         for (size_t c = i; c < chunks && e == cudaSuccess && failed.load() == (int)cudaSuccess; c += DOWNLOAD_SLOTS) {
-            if ((e = cudaEventSynchronize(ring->filled[i])) != cudaSuccess) break;
+            if ((e = cudaEventSynchronize(filled.e[i])) != cudaSuccess) break;
             std::memcpy(static_cast<char*>(dst) + c * DOWNLOAD_CHUNK, ring->slot[i], size_of(c));
             if (c + DOWNLOAD_SLOTS < chunks) e = queue(i, c + DOWNLOAD_SLOTS);
         }
@@ -343,7 +363,7 @@ int release_working_sets(int dev) {
     {
         std::lock_guard<std::mutex> lock(g_rings_mu);
         for (Ring& r : g_rings)
-            if (r.dev == dev && !r.busy) free_ring(r);
+            if (!r.busy) free_slots(r);
     }
     {
         std::lock_guard<std::mutex> lock(g_sides_mu);

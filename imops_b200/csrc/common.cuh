@@ -149,9 +149,9 @@ int side_stream(cudaStream_t s, SideStream* out);
 // malloc starts to hand out fresh pages each time.  (A whole run with a 41 MB
 // image 10.3 -> 3.8 ms, with 28 MB 2.3 -> 2.2, but with 10 to 20 MB, a buffer
 // whose pages are there already, 1.00 -> 1.17 and 1.76 -> 1.85: the threads'
-// start is not won back.)  Rings are kept for the next call (at most
-// DOWNLOAD_RINGS, 16 MB each; a call that finds none free copies directly) and
-// freed by release_working_sets.
+// start is not won back.)  Rings are kept for the next call, on whichever
+// device (at most DOWNLOAD_RINGS, 16 MB each; a call that finds all of them in
+// use copies directly), and freed by release_working_sets.
 constexpr size_t DOWNLOAD_CHUNK = (size_t)4 << 20;
 constexpr size_t DOWNLOAD_LEAST = 8 * DOWNLOAD_CHUNK;
 constexpr int DOWNLOAD_SLOTS = 4, DOWNLOAD_RINGS = 4;

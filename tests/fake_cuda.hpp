@@ -24,6 +24,7 @@ inline size_t room = (size_t)-1;                     // device bytes left for cu
 inline std::atomic<int> null_frees{0}, streams{0}, events{0}, pinned{0};  // the last three: alive
 inline void (*on_copy)(void* dst, size_t bytes) = nullptr;
 inline void (*on_event_wait)() = nullptr;
+inline void (*on_host_alloc)() = nullptr;
 inline std::mutex mu;
 struct Block {
     size_t bytes;
@@ -93,6 +94,7 @@ cudaError_t cudaEventSynchronize(cudaEvent_t) {
 }
 
 cudaError_t cudaHostAlloc(void** p, size_t bytes, unsigned) {
+    if (fake::on_host_alloc) fake::on_host_alloc();
     return fake::pinned++, *p = std::malloc(bytes), cudaSuccess;
 }
 cudaError_t cudaFreeHost(void* p) { return fake::pinned--, std::free(p), cudaSuccess; }
