@@ -6,7 +6,6 @@
 #include <cstring>
 #include <atomic>
 #include <mutex>
-#include <system_error>
 #include <thread>
 
 namespace imops {
@@ -344,8 +343,8 @@ int download(void* dst, const void* src, size_t bytes, cudaStream_t s, const cha
     int started = 1;  // slot 0 is this thread's
     try {
         for (; started < queued; started++) helpers[started] = std::thread(drain, started);
-    } catch (const std::system_error&) {
-        // no more threads: this one drains the rest
+    } catch (...) {
+        // no thread (std::system_error) or no memory for one: this one drains the rest
     }
     if (queued > 0) drain(0);
     for (int i = started; i < queued; i++) drain(i);

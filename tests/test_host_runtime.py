@@ -25,6 +25,6 @@ def test_host(tmp_path, name):
     _run(tmp_path, name)
 
 
-@pytest.mark.parametrize("case", ["other_device", "slow_pinned_memory"])
+@pytest.mark.parametrize("case", ["other_device", "slow_pinned_memory", "no_threads"])
 def test_download(tmp_path, case):
     _run(tmp_path, "host_download", case)
