@@ -709,12 +709,10 @@ __device__ __forceinline__ void scan16_px(const Scan16<E>& c, const float (&D)[E
     for (int k = 0; k < 3; k++) o[k] = __fadd_rn(acc[k].x, acc[k].y);
 }
 
-// A thread a pixel: 16 exponentials and 8 (E + 4) packed FMAs against
-// 4 (E + 4) bytes a layer plane, mask sum and RGB.  SUM: `mask` is the one
-// plane of the layers' mask sum; otherwise E planes, summed here in the same
-// order.  24 MP, six layers: 0.22 ms (2.14 with run-time layer loops over
-// tables in shared memory).
-template <int E, bool SUM>
+// The scan as a step of its own, from a plane of image and one of mask densities
+// a layer; a whole image is scanned by print_kernel.  A thread a pixel: 16
+// exponentials and 8 (E + 4) packed FMAs against 8 E + 12 bytes.
+template <int E>
 __global__ void __launch_bounds__(256) scan16_kernel(const float* __restrict__ img, const float* __restrict__ mask,
                                                      size_t n, const __grid_constant__ Scan16<E> c,
                                                      float* __restrict__ rgb) {
@@ -722,12 +720,8 @@ __global__ void __launch_bounds__(256) scan16_kernel(const float* __restrict__ i
         float D[E], M = 0.0f, o[3];
 #pragma unroll
         for (int e = 0; e < E; e++) D[e] = __ldg(img + e * n + p);
-        if (SUM) {
-            M = __ldg(mask + p);
-        } else {
 #pragma unroll
-            for (int e = 0; e < E; e++) M = __fadd_rn(M, __ldg(mask + e * n + p));
-        }
+        for (int e = 0; e < E; e++) M = __fadd_rn(M, __ldg(mask + e * n + p));
         scan16_px<E>(c, D, M, o);
         rgb[3 * p] = o[0];
         rgb[3 * p + 1] = o[1];
@@ -1781,13 +1775,11 @@ int stage_grain(float* planes, int W, int H, const Stock& st, uint64_t seed, flo
 
 //   scan: densities -> ACEScg RGB of the scanned negative (scan/mod.rs:24-30,
 //     densitometry.rs:13-73)
-int stage_scan(const float* planes, const float* mask, bool sum, int W, int H, const ScanSpec16& S, float* rgb,
-               cudaStream_t s) {
+int stage_scan(const float* planes, const float* mask, int W, int H, const ScanSpec16& S, float* rgb, cudaStream_t s) {
     const size_t n = (size_t)W * H;
     return with_layers(S.E, [&](auto e) {
         constexpr int E = decltype(e)::value;
-        if (sum) scan16_kernel<E, true><<<grid_for(n), 256, 0, s>>>(planes, mask, n, scan16_pairs<E>(S), rgb);
-        else scan16_kernel<E, false><<<grid_for(n), 256, 0, s>>>(planes, mask, n, scan16_pairs<E>(S), rgb);
+        scan16_kernel<E><<<grid_for(n), 256, 0, s>>>(planes, mask, n, scan16_pairs<E>(S), rgb);
         note_launch();
         return IMOPS_OK;
     });
@@ -2170,7 +2162,7 @@ extern "C" int imops_film_scan(const float* planes, const float* mask, int w, in
     int rc = film::stage_ctx(params, w, h, film::no_extra, s, &c);
     if (rc) return rc;
     if (!planes || !mask || !rgb) return fail(IMOPS_ERR_INVALID_ARGUMENT, "film_scan: NULL buffer");
-    if ((rc = film::stage_scan(planes, mask, false, w, h, c.st.scan16, rgb, s))) return rc;
+    if ((rc = film::stage_scan(planes, mask, w, h, c.st.scan16, rgb, s))) return rc;
     IMOPS_CUDA_TRY(cudaGetLastError(), "film_scan");
     return IMOPS_OK;
 }
