@@ -186,7 +186,7 @@ __global__ void __launch_bounds__(BLK) pixel_forward_kernel(const float* __restr
 // tables a pixel: warps that read them at different places evict one another's
 // constants, so one block of 20 warps an SM steps through the pixels together
 // (24 MP, the barrier kept: 1.26 ms; two blocks of 8 warps 1.30, four of 4
-// 1.43).  Bound by the FMA pipe (0.97 ms with the curves).  One bin an FMA,
+// 1.43).  Bound by the FMA pipe (0.97 ms with the curves; busy 0.76 of the time).  One bin an FMA,
 // bound by issue: 1.42 ms.  18 multiply-adds from the six forward tables alone
 // (1.9 KB): 1.30 ms.
 constexpr int NP1 = 20;
@@ -396,7 +396,9 @@ struct CamSource {
     }
 };
 
-// t1 = rows_G(h), t2 = rows_dG(h); four outputs of a row a thread.
+// t1 = rows_G(h), t2 = rows_dG(h); four outputs of a row a thread.  Bound by
+// instruction issue (0.72 of its rate, the FMA pipe at 0.53): 24 MP 264 us for
+// both, one pass by packed pairs from the same source 148.
 __global__ void __launch_bounds__(film::R64_ROW_THREADS) rows_dual_kernel(const CamSource in, float* __restrict__ t1,
                                                                           float* __restrict__ t2, int W,
                                                                           const __grid_constant__ DualTaps tp) {
@@ -453,11 +455,13 @@ __global__ void __launch_bounds__(film::R64_ROW_THREADS) rows_dual_kernel(const 
 }
 
 // t3 = cols_G(g), and the block's part of <t3, t2> + <cols_dG(g), t1> into
-// partial[block]; cols_ends_kernel makes both the transposes.  A block walks a 32-column strip over a ring of three
-// 128-row slabs as blur_cols_r64_stream_kernel does; a thread forms eight
-// outputs of a chunk from two windows that slide towards each other.  24 MP: 0.26
-// ms, where the three column passes of G(gB) and dB/dsigma took 0.53.  (The end
-// terms in this kernel's epilogue cost registers: 0.32-0.45 ms.)
+// partial[block]; cols_ends_kernel makes both the transposes.  A block walks a
+// 32-column strip over a ring of three 128-row slabs as
+// blur_cols_r64_stream_kernel does; a thread forms eight outputs of a chunk from
+// two windows that slide towards each other.  Bound by instruction issue (0.76
+// of its rate, the FMA pipe at 0.55).  24 MP: 0.26 ms, where the three column
+// passes of G(gB) and dB/dsigma took 0.53.  (The end terms in this kernel's
+// epilogue cost registers: 0.32-0.45 ms.)
 constexpr int CD_OUT = 8, CD_GROUPS = film::SC_SLAB / CD_OUT, CD_PER = film::SC_SLAB / CD_GROUPS;
 constexpr int CD_THREADS = film::R64_COL_TW * CD_GROUPS;
 
@@ -566,9 +570,9 @@ __global__ void __launch_bounds__(CD_THREADS, 2) cols_dual_t_kernel(const float*
 // inner products, in partial[block].  A block has 32 columns of an end; a warp
 // takes eight of the 64 distances, each sample once for both blurs and for its
 // own row's term and the end row's sum.  Bound by latency: every load is in
-// flight at once.  2.8 MP: 3.5 us (24 MP: 5.6), where a thread a row, the end rows' 64
-// samples one thread's, took 11.4 us (16.4).  With H <= 129 rows the ends share rows and one
-// block takes both, one after the other.
+// flight at once.  2.8 MP: 3.5 us (24 MP: 5.6), where a thread a row, the end
+// rows' 64 samples one thread's, took 11.4 us (16.4).  With H <= 129 rows the
+// ends share rows and one block takes both, one after the other.
 __global__ void __launch_bounds__(BLK) cols_ends_kernel(const float* __restrict__ g, int W, int H,
                                                         const __grid_constant__ DualTaps tp,
                                                         const float* __restrict__ t1, const float* __restrict__ t2,
@@ -883,10 +887,12 @@ int backward_halation(Bufs& b, const float* x, int W, int H, int* nbh, int* nbs,
     const size_t n = (size_t)W * H;
     int rc;
     if (b.R == film::R64) {
-        cols_dual_t_kernel<<<b.cols_grid, CD_THREADS, 0, s>>>(b.gB, W, H, b.chunks, dual_taps(b), b.t1, b.t2, b.t3, b.ps);
+        cols_dual_t_kernel<<<b.cols_grid, CD_THREADS, 0, s>>>(b.gB, W, H, b.chunks, dual_taps(b), b.t1, b.t2, b.t3,
+                                                              b.ps);
         const int nb = (int)(b.cols_grid.x * b.cols_grid.y);
         const int ends = H > 2 * film::R64 + 1 ? 2 : 1;
-        cols_ends_kernel<<<dim3(b.cols_grid.x, ends), BLK, 0, s>>>(b.gB, W, H, dual_taps(b), b.t1, b.t2, b.t3, b.ps + nb);
+        cols_ends_kernel<<<dim3(b.cols_grid.x, ends), BLK, 0, s>>>(b.gB, W, H, dual_taps(b), b.t1, b.t2, b.t3,
+                                                                   b.ps + nb);
         *nbs = nb + (int)b.cols_grid.x * ends;
         rows_t_color_kernel<<<b.rows_grid, film::R64_ROW_THREADS, 0, s>>>(b.t3, x, W, H, film::pair_taps(b.tp), b.src,
                                                                           b.ph);
@@ -940,8 +946,8 @@ extern "C" int imops_param_backward(const float* cam_rgb, const float* g_out, co
     int rc = adj::prepare(cam_rgb, w, h, params, fixed, true, s, &b);
     if (rc) return rc;
     const size_t n = (size_t)w * h;
-    adj::pixel_backward_kernel<<<b.nb1, adj::PB_THREADS, 0, s>>>(cam_rgb, b.B, g_out, target, loss_scale, n, b.c, b.bt, b.gB,
-                                                                 b.p1);
+    adj::pixel_backward_kernel<<<b.nb1, adj::PB_THREADS, 0, s>>>(cam_rgb, b.B, g_out, target, loss_scale, n, b.c, b.bt,
+                                                                 b.gB, b.p1);
     note_launch();
     int nbh = 0, nbs = 0;
     if ((rc = adj::backward_halation(b, cam_rgb, w, h, &nbh, &nbs, s))) return rc;

@@ -51,8 +51,9 @@ __device__ __forceinline__ int reflect(int i, int n) {
 // sums its taps in ascending order.
 constexpr int ROW_OUT = 4, ROW_THREADS = 256, ROW_TILE = ROW_OUT * ROW_THREADS;
 
-static __global__ void __launch_bounds__(ROW_THREADS) blur_rows_kernel(const float* __restrict__ in, float* __restrict__ out,
-                                                                int W, int H, const __grid_constant__ Taps tp) {
+static __global__ void __launch_bounds__(ROW_THREADS)
+    blur_rows_kernel(const float* __restrict__ in, float* __restrict__ out, int W, int H,
+                     const __grid_constant__ Taps tp) {
     __shared__ __align__(16) float s[ROW_TILE + 2 * MAXR + ROW_OUT];
     const int y = blockIdx.y, x0 = blockIdx.x * ROW_TILE, R2 = 2 * tp.R;
     const float* row = in + (size_t)y * W;

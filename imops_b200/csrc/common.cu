@@ -112,7 +112,8 @@ StreamCache::StreamCache(const char* what) : what_(what) {
 // image, does not stall frames in flight on other streams.  Work on other
 // streams that uses the buffer is ordered after s with events.
 int StreamCache::get(cudaStream_t s, size_t bytes, void** out) {
-    if (fault_injected("alloc")) return fail(IMOPS_ERR_OUT_OF_MEMORY, std::string("injected allocation failure (") + what_ + ")");
+    if (fault_injected("alloc"))
+        return fail(IMOPS_ERR_OUT_OF_MEMORY, std::string("injected allocation failure (") + what_ + ")");
     int dev = 0;
     IMOPS_CUDA_TRY(cudaGetDevice(&dev), "cudaGetDevice");
     // a request without room leaves nothing behind: the stream's next one

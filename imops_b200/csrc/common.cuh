@@ -94,9 +94,10 @@ void note_launch(int n = 1);
 bool fault_injected(const char* site);
 
 // A device buffer per (device, stream), grown on demand: the working sets of
-// the film, adjoint, X-Trans and fused-develop paths.  Growing waits for the
-// stream, frees the old buffer and allocates the new one.  Every cache
-// registers itself, so imops_release_working_sets can free them all.
+// the film, adjoint, X-Trans and fused-develop paths.  Growing frees
+// the old buffer and allocates the new one in the stream's order; a request
+// without room fails and leaves the stream without one.  Every cache registers
+// itself, so imops_release_working_sets can free them all.
 class StreamCache {
    public:
     explicit StreamCache(const char* what);

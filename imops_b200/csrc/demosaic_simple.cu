@@ -3,13 +3,14 @@
 // (Fast / SuperFast / SuperSuperFast, demosaic.rs:189-356).
 //
 // The mean reads a mosaic (4 B a pixel, or 2 B of the sensor frame, scaled
-// while it is staged) and writes 12 B.  Every Bayer CFA is a shift of RGGB and every X-Trans sensor's CFA a shift of one 6x6 pattern, so
-// for those the kernel aligns each thread's run of pixels with the pattern:
-// the colour of every site in a run's window is then a compile-time constant
-// (per row phase, and a warp handles one row), the per-colour sums are plain
-// adds and the counts constants.  Other CFAs take the per-pixel kernel.  Both
-// sum each colour's sites in row-major order and divide once, as the
-// reference's f32 code does; built with --fmad=false.
+// while it is staged) and writes 12 B.  Every Bayer CFA is a shift of RGGB and
+// every X-Trans sensor's CFA a shift of one 6x6 pattern, so for those the
+// kernel aligns each thread's run of pixels with the pattern: the colour of
+// every site in a run's window is then a compile-time constant (per row phase,
+// and a warp handles one row), the per-colour sums are plain adds and the
+// counts constants.  Other CFAs take the per-pixel kernel.  Both sum each
+// colour's sites in row-major order and divide once, as the reference's f32
+// code does; built with --fmad=false.
 #include <type_traits>
 
 #include "cfa_canon.cuh"

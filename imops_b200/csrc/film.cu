@@ -283,7 +283,8 @@ __global__ void __launch_bounds__(8 * LUTN) capture_lut_kernel(const __grid_cons
 // Image-dye densities over the fluences in place, and the mask densities
 // (SUM: `mask` is one plane, their sum in layer order; otherwise E planes);
 // BOUNCE: the support bounce `deep` is added to the fluences first.  Bound by
-// the issue of the interpolation and the power of each layer and pixel.  24 MP, six layers, with the bounce: 0.55 ms against 1.86
+// instruction issue (0.84 of its rate): the interpolation and the power of each
+// layer and pixel.  24 MP, six layers, with the bounce: 0.55 ms against 1.86
 // (reduction and bounce epilogue apart, a binary search and powf a value).
 template <int E, bool SUM, bool BOUNCE>
 __global__ void __launch_bounds__(256) lut_reduce_kernel(float* __restrict__ planes, float* __restrict__ mask,
@@ -366,8 +367,8 @@ __global__ void dir_apply_kernel(float* __restrict__ planes, const float* __rest
 // one conversion to f32, where twelve f32 additions rounded at 2^-22 each.  The
 // mixer's last xor-shift by 31 reaches only bit 32 of a draw, so it is left out.
 //
-// Bound by the integer ALU (11 of the 17 instructions of a draw) at 32 warps
-// an SM.  Tiles are 128 wide and TH high, their runs a whole number of
+// Bound by the integer ALU (11 of the 17 instructions of a draw; its pipe at 0.66
+// of its rate, issue at 0.75) at 32 warps an SM.  Tiles are 128 wide and TH high, their runs a whole number of
 // rounds of the 512 threads where that fits two blocks an SM: 39 rows for up
 // to three layers (96 KB), 24 for six (113 KB).  Six layers in one block mix
 // 13.25 draws a pixel, two blocks of three 25; with fewer than two tiles of
@@ -802,10 +803,10 @@ __global__ void invert_kernel(float* __restrict__ rgb, size_t n, const float* __
 // in with cp.async while the layer before is blurred (adjacency), its grain
 // is added, and its densities stay in shared memory (a thread's own four
 // pixels); when all layers are through, the thread scans its pixels and
-// inverts them.  RC: the blur radius class (taps beyond the radius are zero:
+// inverts them.  Bound by instruction issue (0.78 of its rate; six layers).  RC: the blur radius class (taps beyond the radius are zero:
 // densities are finite, so they add nothing), 0 where the densities are
 // final.  Same arithmetic as the steps one by one.  24 MP, six layers, grain:
-// 0.71 ms against 2.1 (12 blur launches, 6 of the grain, the scan).
+// 0.73 ms against 2.1 (12 blur launches, 6 of the grain, the scan).
 constexpr int PR_THREADS = 512, PR_ROWS = ft_rpt(PR_THREADS);
 template <int E>
 struct Print {
@@ -900,8 +901,10 @@ __global__ void __launch_bounds__(PR_THREADS, 2) print_kernel(const float* __res
 
 // Exposure of the layers and their local scatter on a 64 x 32 tile: the basis
 // weights of the tile and its halo once, then each layer formed from them,
-// blurred and mixed, so the layers reach memory once, scattered.  24 MP, six
-// layers, radius 2: 0.56 ms against 1.5 (an exposure pass and 12 blur launches).
+// blurred and mixed, so the layers reach memory once, scattered.  Bound by
+// instruction issue (0.68 of its rate) and the barriers between its passes.
+// 24 MP, six layers, radius 2: 0.56 ms against 1.5 (an exposure pass and 12 blur
+// launches).
 constexpr int EX_THREADS = 512, EX_ROWS = ft_rpt(EX_THREADS), EX_MAXR = 8;
 __host__ __device__ constexpr int expose_smem_floats(int R) { return 5 * ft_tile_floats(R) + ft_row_floats(R); }
 
@@ -1610,7 +1613,8 @@ int expose_scatter(const float* rgb, int W, int H, const Stock& st, float* plane
     IMOPS_CUDA_TRY(cudaFuncSetAttribute(expose_scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                    "cudaFuncSetAttribute(exposure)");
     const dim3 g((W + FT_W - 1) / FT_W, (H + FT_H - 1) / FT_H);
-    expose_scatter_kernel<<<g, EX_THREADS, smem, s>>>(rgb, W, H, st.expose, tp, 1.0f - R.local_mix, R.local_mix, planes);
+    expose_scatter_kernel<<<g, EX_THREADS, smem, s>>>(rgb, W, H, st.expose, tp, 1.0f - R.local_mix, R.local_mix,
+                                                      planes);
     note_launch();
     return IMOPS_OK;
 }
@@ -2112,7 +2116,8 @@ extern "C" int imops_film_halation(float* planes, int w, int h, const ImopsFilmP
     if ((rc = film::stage_scatter(planes, w, h, c.st.ref, tmp, s))) return rc;
     if ((rc = film::stage_bounce(planes, w, h, c.st.ref, tmp, bounce, &deep, s))) return rc;
     if (deep) {
-        film::bounce_kernel<<<film::grid_for(n), 256, 0, s>>>(planes, deep, n, c.st.ref.E, film::bounce_gains(c.st.ref));
+        film::bounce_kernel<<<film::grid_for(n), 256, 0, s>>>(planes, deep, n, c.st.ref.E,
+                                                              film::bounce_gains(c.st.ref));
         note_launch();
     }
     IMOPS_CUDA_TRY(cudaGetLastError(), "film_halation");
@@ -2142,7 +2147,8 @@ extern "C" int imops_film_grain(float* planes, int w, int h, const ImopsFilmPara
     const size_t n = (size_t)(w > 0 ? w : 0) * (h > 0 ? h : 0);
     film::StageCtx c;
     int rc = film::stage_ctx(
-        params, w, h, [=](int E) { return E * n * 4 + film::grain_partials(w, h, E) * 8 + film::MAXE * 8 + 768; }, s, &c);
+        params, w, h, [=](int E) { return E * n * 4 + film::grain_partials(w, h, E) * 8 + film::MAXE * 8 + 768; }, s,
+        &c);
     if (rc) return rc;
     if (!planes) return fail(IMOPS_ERR_INVALID_ARGUMENT, "film_grain: NULL buffer");
     if (!params->grain) return IMOPS_OK;

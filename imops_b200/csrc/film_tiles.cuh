@@ -153,7 +153,7 @@ __device__ __forceinline__ void ft_blur(const float* s, float* rows, int tx, int
 // in registers as the layers go by, so a layer's blur is never stored.  Bound
 // by instruction issue (0.66 of the issue rate at two blocks an SM: the
 // accumulators take 48 of 128 registers).  24 MP, six layers, radius 9:
-// 0.65 ms against 2.8 ms as twelve blur launches and a mixing pass (0.90 with
+// 0.66 ms against 2.8 ms as twelve blur launches and a mixing pass (0.90 with
 // the halo copied sample by sample in index order).
 template <int E>
 struct DirMix {
@@ -163,9 +163,9 @@ struct DirMix {
 constexpr int DIR_THREADS = 256, DIR_ROWS = ft_rpt(DIR_THREADS);
 
 template <int E>
-__global__ void __launch_bounds__(DIR_THREADS, E <= 3 ? 3 : 2) dir_kernel(const float* __restrict__ in, float* __restrict__ out,
-                                                            int W, int H, const __grid_constant__ Taps tp,
-                                                            const __grid_constant__ DirMix<E> mix) {
+__global__ void __launch_bounds__(DIR_THREADS, E <= 3 ? 3 : 2)
+    dir_kernel(const float* __restrict__ in, float* __restrict__ out, int W, int H, const __grid_constant__ Taps tp,
+               const __grid_constant__ DirMix<E> mix) {
     extern __shared__ __align__(16) float ftsm[];
     const int R = tp.R, tile = ft_tile_floats(R);
     float* rows = ftsm + 2 * tile;

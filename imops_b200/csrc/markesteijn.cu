@@ -121,8 +121,9 @@ __device__ void mean3(const Img& im, int r, int c, float* o) {
 // ordered from the inside out).  Every value is the specification's f32
 // arithmetic in its order (a sum's leading 0 + x aside).
 //
-// Bound by instruction issue (0.61 of its rate; a third of the instructions
-// are CIELab's cube roots) and shared-memory latency between the barriers.
+// Bound by instruction issue (0.61 of its rate; CIELab's 15 cube roots an output,
+// of about 30 operations each, are a quarter of it) and by shared-memory latency
+// between the barriers.
 // 24 MP: 2.07 ms against 4.52 (the general tiles below: 5260 instructions an
 // output, here 1930).  512 threads: 2.07 ms, 384 2.14, 448 2.12, 576 2.13, 672
 // 2.23; list entries read from memory in every stage instead of held in

@@ -5,6 +5,8 @@
   python -m imops_b200.profile_cases fwdbwd --width 6048 --height 4024
   python -m imops_b200.profile_cases display --width 6048 --height 4024
   python -m imops_b200.profile_cases xtrans --width 6032 --height 4032
+  python -m imops_b200.profile_cases xtrans_develop --width 6032 --height 4032
+  python -m imops_b200.profile_cases stock --width 6048 --height 4024 [--stock 2] [--positive]
 
 Each case builds a seeded synthetic input, runs the stage once and
 synchronises, so `ncu -k regex:<kernel> -c 1` captures exactly one launch.
@@ -18,11 +20,14 @@ import numpy as np
 
 def main() -> None:
     ap = argparse.ArgumentParser()
-    ap.add_argument("case", choices=["amaze", "film81", "develop", "fwdbwd", "display", "xtrans"])
+    ap.add_argument("case", choices=["amaze", "film81", "develop", "fwdbwd", "display", "xtrans", "xtrans_develop",
+                                     "stock"])
     ap.add_argument("--width", type=int, default=4096)
     ap.add_argument("--height", type=int, default=3072)
     ap.add_argument("--scan", choices=["fp32", "bf16_tc"], default="fp32",
                     help="the 81-bin scan's contractions: CUDA cores (FP32) or tensor cores (BF16 hi/lo)")
+    ap.add_argument("--stock", type=int, default=2, help="the stock case's film (2: Portra400, six layers)")
+    ap.add_argument("--positive", action="store_true", help="the stock case's output: an inverted print")
     a = ap.parse_args()
 
     import torch
@@ -39,6 +44,26 @@ def main() -> None:
         out = im.demosaic_markesteijn3(m, synthetic.XTRANS)
         torch.cuda.synchronize()
         print(f"{a.case} {W}x{H} ok, mean {float(mean.mean()):.6f} {float(out.mean()):.6f}")
+        return
+    if a.case == "xtrans_develop":
+        # u16 frame to ACEScg: the 3x3 mean that scales as it stages its rows
+        raw = torch.from_numpy(synthetic.mosaic_u16(H, W, seed=5, pattern=synthetic.XTRANS).view(np.int16)).cuda()
+        p = im.DevelopParams()
+        p.demosaic, p.cfa, p.clip_pt, p.target = im.DEMOSAIC_MARKESTEIJN, synthetic.XTRANS.encode(), 1.0, im.CS_ACESCG
+        for i in range(4):
+            p.wb[i] = synthetic.WB[i]
+        for i in range(9):
+            p.calib_d65[i] = synthetic.CALIB_D65[i]
+        out = im.develop_u16(raw, (0, 0, W, H), synthetic.BLACK, synthetic.WHITE, p)
+        torch.cuda.synchronize()
+        print(f"{a.case} {W}x{H} ok, mean {float(out.mean()):.6f}")
+        return
+    if a.case == "stock":
+        # a reference stock with grain on a scene-linear frame at its box speed
+        x = torch.from_numpy((synthetic.scene(H, W, seed=5) * 800.0).astype(np.float32)).cuda()
+        out = im.film_process(x, stock=a.stock, seed=3, output=int(a.positive), grain=True)
+        torch.cuda.synchronize()
+        print(f"{a.case} {a.stock} {W}x{H} ok, mean {float(out.mean()):.6f}")
         return
     raw = torch.from_numpy(synthetic.mosaic_u16(H, W, seed=5).view(np.int16)).cuda()
     if a.case == "fwdbwd":

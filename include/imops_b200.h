@@ -71,10 +71,11 @@ const char *imops_version(void);
 
 /* Frees the working sets the stage entry points cache per (device, stream)
  * on the current device (film, adjoint, the scaled mosaics of the u16
- * develop paths), after waiting for the device, and the pinned chunks of
- * downloads into pageable memory; the next call allocates again.  No counterpart in the reference (its buffers are Rust Vecs freed
- * with each module).  Call it when no work of this library is in flight on
- * the device from another thread. */
+ * develop paths) and the film calls' side streams, after waiting for the
+ * device, and the pinned chunks of downloads into pageable memory; the next
+ * call allocates again.  No counterpart in the reference (its buffers are
+ * Rust Vecs freed with each module).  Call it when no work of this library is
+ * in flight on the device from another thread. */
 int imops_release_working_sets(void);
 
 /* ---- decode-side normalisation ------------------------------------------
